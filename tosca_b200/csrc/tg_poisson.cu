@@ -14,17 +14,20 @@
 // use preconditioned CG on the reduced system (the pinned unknown stays zero);
 // others use right-preconditioned BiCGStab.
 //
-// Preconditioner: the geometric multigrid V-cycle of tg_mg.cu on the 7-point
-// part of the operator, applied in the grounded form z = P M P^T r (P shifts
+// Preconditioner: on a mesh of planes the direct solve of tg_fdm.cu, elsewhere
+// the geometric multigrid V-cycle of tg_mg.cu on the 7-point part of the
+// operator; both are applied in the grounded form z = P M P^T r (P shifts
 // so that z at the pinned cell is zero), which is the inverse structure of the
 // pinned operator. In the mixed-precision mode the multigrid stores and
-// computes in FP32; residuals, inner products and the solution stay FP64.
+// computes in FP32; the direct solve, residuals, inner products and the
+// solution stay FP64.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "tg_internal.cuh"
+#include "tg_fdm.cuh"
 #include "tg_mg.cuh"
 
 namespace tg {
@@ -39,7 +42,8 @@ struct PoissonCtx {
     double *xprev, *xprev2;      // the two previous steps' solutions (extrapolated initial guess)
     double *part;                // reduction partials (4 per block)
     int nblocks;
-    MG *mg;                      // multigrid preconditioner (host object)
+    MG *mg;                      // multigrid preconditioner (host object), where fdm does not apply
+    Fdm *fdm;                    // direct solve on a mesh of planes, else null
 };
 
 namespace {
@@ -216,17 +220,20 @@ __device__ __forceinline__ void dot_store(double (&v)[3], double *part)
     block_reduce<RB>(v, RedSum{}, RedSum{}, RedMax{});
     if (threadIdx.x == 0) { part[3 * blockIdx.x] = v[0]; part[3 * blockIdx.x + 1] = v[1]; part[3 * blockIdx.x + 2] = v[2]; }
 }
-__global__ void __launch_bounds__(RB) k_dot_partial(int64_t n, const double *a, const double *b, const double *w, double *part)
+// sh: constant subtracted from b (the preconditioned residual is used up to
+// its value at the pinned cell), or null
+__global__ void __launch_bounds__(RB) k_dot_partial(int64_t n, const double *a, const double *b, const double *sh, const double *w, double *part)
 {
     double v[3] = {0.0, 0.0, 0.0};
+    const double b0 = sh ? sh[0] : 0.0;
     const int64_t n2 = n >> 1;
     TG_PAIRS(t, n2) {
         const double2 av = v2(a)[t], bv = v2(b)[t];
         const double2 wv = w ? v2(w)[t] : double2{0.0, 0.0};
-        dot_acc(av.x, bv.x, wv.x, v);
-        dot_acc(av.y, bv.y, wv.y, v);
+        dot_acc(av.x, bv.x - b0, wv.x, v);
+        dot_acc(av.y, bv.y - b0, wv.y, v);
     }
-    if (odd_tail(n)) dot_acc(a[n - 1], b[n - 1], w ? w[n - 1] : 0.0, v);
+    if (odd_tail(n)) dot_acc(a[n - 1], b[n - 1] - b0, w ? w[n - 1] : 0.0, v);
     dot_store(v, part);
 }
 // final: out[0..2] = totals
@@ -250,6 +257,10 @@ __global__ void k_copy(int64_t n, const double *a, double *b)
     const int64_t n2 = n >> 1;
     TG_PAIRS(t, n2) v2(b)[t] = v2(a)[t];
     if (odd_tail(n)) b[n - 1] = a[n - 1];
+}
+__global__ void k_fill(int64_t n, double *a, double v)
+{
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) a[t] = v;
 }
 __global__ void k_zero_at(double *z, int pin) { z[pin] = 0.0; }
 // initial guess of the step's solve from the last three solutions (the
@@ -300,14 +311,6 @@ __global__ void __launch_bounds__(RB, 4) k_cg_update_rr(int64_t n, const double 
         dot_acc(rv, rv, w ? w[n - 1] : 0.0, v);
     }
     dot_store(v, part);
-}
-// CG: beta = rz_new / rz_old ; p = z + beta p
-__global__ void k_cg_dir(int64_t n, const double *rznew, const double *rzold, const double *z, double *p)
-{
-    const double beta = rznew[0] / rzold[0];
-    const int64_t n2 = n >> 1;
-    TG_PAIRS(t, n2) { const double2 zv = v2(z)[t], pv = v2(p)[t]; v2(p)[t] = double2{zv.x + beta * pv.x, zv.y + beta * pv.y}; }
-    if (odd_tail(n)) p[n - 1] = z[n - 1] + beta * p[n - 1];
 }
 __global__ void k_scalar_copy(const double *a, double *b, int n) { for (int t = 0; t < n; t++) b[t] = a[t]; }
 
@@ -374,18 +377,20 @@ __global__ void k_cg_finish(double *sc, int base)
     if (!isfinite(rn)) sc[base + ST_NAN] = 1.0;
     else if (sc[52] == 0.0) sc[base + ST_NOCONV] += 1.0;
 }
-// p = z on the first pass through the loop body, else p = z + (rz_new / rz_old) p
-__global__ void k_cg_dir_loop(int64_t n, const double *sc, const double *z, double *p)
+// CG direction: p = z - z[0] on the first pass through the loop (sc[51]), else
+// p = z - z[0] + (rz_new / rz_old) p
+__global__ void k_cg_dir(int64_t n, const double *sc, const double *z, double *p)
 {
     const bool first = sc[51] != 0.0;
-    const double beta = first ? 0.0 : sc[6] / sc[14];
+    const double beta = first ? 0.0 : sc[6] / sc[14], z0 = z[0];
     const int64_t n2 = n >> 1;
     TG_PAIRS(t, n2) {
         const double2 zv = v2(z)[t];
-        if (first) v2(p)[t] = zv;
-        else { const double2 pv = v2(p)[t]; v2(p)[t] = double2{zv.x + beta * pv.x, zv.y + beta * pv.y}; }
+        double2 o{zv.x - z0, zv.y - z0};
+        if (!first) { const double2 pv = v2(p)[t]; o = double2{o.x + beta * pv.x, o.y + beta * pv.y}; }
+        v2(p)[t] = o;
     }
-    if (odd_tail(n)) p[n - 1] = first ? z[n - 1] : z[n - 1] + beta * p[n - 1];
+    if (odd_tail(n)) p[n - 1] = first ? z[n - 1] - z0 : z[n - 1] - z0 + beta * p[n - 1];
 }
 
 inline dim3 cgrid(int nx, int ny, int nz) { return grid3(nx, ny, nz); }
@@ -401,18 +406,20 @@ static void apply_op(tg_ctx *C, const double *x, double *y)
     else TG_PROF(C, "pois_apply19", k_apply19<<<cgrid(P.nx, P.ny, P.nz), block3(), 0, C->stream>>>(P, x, y));
 }
 
-// totals of (a.b, sum a, max|a w|) into out[0..2] (device)
-static void dot3v(tg_ctx *C, const double *a, const double *b, const double *w, double *out)
+// totals of (a.b, sum a, max|a w|) into out[0..2] (device); sh: see k_dot_partial
+static void dot3v(tg_ctx *C, const double *a, const double *b, const double *w, double *out, const double *sh = nullptr)
 {
     PoissonCtx &P = *C->pois;
-    TG_PROF(C, "pois_dot", k_dot_partial<<<P.nblocks, RB, 0, C->stream>>>(P.n, a, b, w, P.part));
+    TG_PROF(C, "pois_dot", k_dot_partial<<<P.nblocks, RB, 0, C->stream>>>(P.n, a, b, sh, w, P.part));
     k_dot_final<<<1, RB, 0, C->stream>>>(P.part, P.nblocks, out);
 }
 
-// z = P M P^T r (grounded multigrid); needs sum(r) at d_sum
+// z = P M P^T r up to a constant (z[0], which the multigrid returns as zero);
+// needs sum(r) at d_sum
 static void precondition(tg_ctx *C, const double *r, double *z, const double *d_sum)
 {
-    mg_apply(C, C->pois->mg, r, d_sum, z);
+    if (C->pois->fdm) fdm_apply(C, C->pois->fdm, r, d_sum, z);
+    else mg_apply(C, C->pois->mg, r, d_sum, z);
 }
 
 // SetRHS (peqn.c:1942-2063) into the compact vector, negated (L = -A)
@@ -462,14 +469,16 @@ void poisson_setup(tg_ctx *C)
     P->part = dallocd(C, 3 * (size_t)P->nblocks);
     k_gather_g<<<cgrid(P->nx, P->ny, P->nz), block3(), 0, C->stream>>>(g, C->m, *P);
 
-    P->mg = mg_create(C, C->cfg.precision == TG_PREC_MIXED, P->gE1, P->gN2, P->gT3,
-                      P->nx, P->ny, P->nz, P->pi, P->pj, P->pk);
+    P->fdm = P->ortho ? fdm_create(C, P->gE1, P->gN2, P->gT3, P->nx, P->ny, P->nz, P->pi, P->pj, P->pk) : nullptr;
+    P->mg = P->fdm ? nullptr : mg_create(C, C->cfg.precision == TG_PREC_MIXED, P->gE1, P->gN2, P->gT3,
+                                         P->nx, P->ny, P->nz, P->pi, P->pj, P->pk);
     TG_CUDA(cudaGetLastError());
 }
 
 void poisson_destroy(tg_ctx *C)
 {
     if (C->pois && C->pois->mg) mg_destroy(C->pois->mg);
+    if (C->pois && C->pois->fdm) fdm_destroy(C->pois->fdm);
     delete C->pois;   // device buffers are owned by the context allocation list
     C->pois = nullptr;
 }
@@ -513,8 +522,10 @@ static int krylov_solve(tg_ctx *C, tg_stats *st, double rtol, double divtol, int
     if (P.ortho) {
         // preconditioned CG on the reduced SPD system (r[pin] = 0, x[pin] = 0)
         precondition(C, P.r, P.z, sc + 4);
-        dot3v(C, P.r, P.z, nullptr, sc + 6);                 // rz at sc[6]
-        TG_PROF(C, "pois_copy", k_copy<<<vblocks(n), RB, 0, s>>>(n, P.z, P.p));
+        dot3v(C, P.r, P.z, nullptr, sc + 6, P.z);            // rz at sc[6]
+        k_fill<<<1, 32, 0, s>>>(1, sc + 51, 1.0);
+        TG_PROF(C, "pois_cg_dir", k_cg_dir<<<vblocks(n), RB, 0, s>>>(n, sc, P.z, P.p));
+        k_fill<<<1, 32, 0, s>>>(1, sc + 51, 0.0);
         while (!converged() && it < maxit) {
             apply_op(C, P.p, P.q);
             k_zero_at<<<1, 1, 0, s>>>(P.q, P.pin);
@@ -528,8 +539,8 @@ static int krylov_solve(tg_ctx *C, tg_stats *st, double rtol, double divtol, int
             if (converged()) { ok = true; break; }
             precondition(C, P.r, P.z, sc + 4);
             k_scalar_copy<<<1, 1, 0, s>>>(sc + 6, sc + 14, 1);   // rz_old
-            dot3v(C, P.r, P.z, nullptr, sc + 6);                 // rz_new
-            TG_PROF(C, "pois_cg_dir", k_cg_dir<<<vblocks(n), RB, 0, s>>>(n, sc + 6, sc + 14, P.z, P.p));
+            dot3v(C, P.r, P.z, nullptr, sc + 6, P.z);            // rz_new
+            TG_PROF(C, "pois_cg_dir", k_cg_dir<<<vblocks(n), RB, 0, s>>>(n, sc, P.z, P.p));
         }
     } else {
         // right-preconditioned BiCGStab on the full pinned system
@@ -666,10 +677,6 @@ static cudaGraphConditionalHandle capture_handle(tg_ctx *C)
     return h;
 }
 
-__global__ void k_fill(int64_t n, double *a, double v)
-{
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) a[t] = v;
-}
 // BiCGStab restarts from the true residual every 50 iterations, and after a
 // true residual that missed the stopping test (sc[53] set); clears sc[53]
 __global__ void k_bicg_restart_flag(double *sc, cudaGraphConditionalHandle h)
@@ -716,8 +723,8 @@ static void krylov_capture(tg_ctx *C, double rtol, double divtol, int maxit, int
             cudaStream_t a = C->stream;
             precondition(C, P.r, P.z, sc + 4);
             k_scalar_copy<<<1, 1, 0, a>>>(sc + 6, sc + 14, 1);           // rz_old
-            dot3v(C, P.r, P.z, nullptr, sc + 6);                          // rz
-            k_cg_dir_loop<<<vb, RB, 0, a>>>(n, sc, P.z, P.p);
+            dot3v(C, P.r, P.z, nullptr, sc + 6, P.z);                     // rz
+            k_cg_dir<<<vb, RB, 0, a>>>(n, sc, P.z, P.p);
             apply_op(C, P.p, P.q);
             k_zero_at<<<1, 1, 0, a>>>(P.q, P.pin);
             dot3v(C, P.p, P.q, nullptr, sc + 9);                          // pq
