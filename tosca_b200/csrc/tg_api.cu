@@ -408,7 +408,7 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
         for (const V3f<double> &v : {M.csi, M.icsi, M.jcsi, M.kcsi}) along(v, 1);
         for (const V3f<double> &v : {M.eta, M.ieta, M.jeta, M.keta}) along(v, 2);
         for (const V3f<double> &v : {M.zet, M.izet, M.jzet, M.kzet}) along(v, 0);
-        C->axis_aligned = ax;
+        C->axis_aligned = ax && tensor_setup(C);
         graph_destroy(C);          // the captured step refers to the old solver buffers
         C->graph_failed = false;
         farm_destroy(C);           // turbine stencils refer to the old cell centres
@@ -453,7 +453,13 @@ tg_status tg_set_field(tg_ctx *C, int32_t w, const double *host, int32_t halo)
         TG_CUDA(cudaStreamSynchronize(C->stream));
         if (w == TG_F_RHS) C->clear_rhs = true;
         if (w == TG_F_DP) C->clear_dp = true;
-        if ((w >= TG_F_CSI && w <= TG_F_KZET) || (w >= TG_F_AJ && w <= TG_F_KAJ)) C->met32_stale = true;
+        if ((w >= TG_F_CSI && w <= TG_F_KZET) || (w >= TG_F_AJ && w <= TG_F_KAJ)) {
+            C->met32_stale = true;
+            if (C->axis_aligned) {         // the caller's metrics need not be those of a mesh of planes
+                C->axis_aligned = false;
+                graph_destroy(C);
+            }
+        }
         return TG_OK;
     });
 }

@@ -73,6 +73,15 @@ struct FaceMet {
     T *flt2;      // Smagorinsky filter width squared, ((1/aj)^(1/3))^2 (les.c:2204-2514)
 };
 
+// cell sizes and face distances of a mesh of planes, their reciprocals, and the
+// factors q of the Smagorinsky width squared, (dx dy dz)^(2/3) = qx qy qz
+// (tg_tensor.cu); x by k, y by i, z by j, device arrays
+struct Tensor {
+    const double *dx, *dy, *dz, *dxf, *dyf, *dzf;
+    const double *rdx, *rdy, *rdz, *rdxf, *rdyf, *rdzf;
+    const double *qx, *qy, *qz;
+};
+
 // FormU work planes at storage precision T: face fluxes per direction and
 // their cell divergence
 template <class T>
@@ -183,8 +192,11 @@ struct tg_ctx {
     bool orthogonal = true;              // all cross metric-tensor terms vanish
     // csi || y, eta || z, zet || x at every point of every cell and face
     // metric up to round-off (the reference's i -> y, j -> z, k -> x axes on
-    // a mesh of planes): FormU reads only those components
+    // a mesh of planes), and every metric a product of the spacings in ts: the
+    // stage kernels of tg_tensor.cu run
     bool axis_aligned = false;
+    tg::Tensor ts{};
+    double *ts_mem = nullptr;            // storage of ts
     bool ufilt_set = false;
     bool surf_set = false;               // thetaWallFunction -3 surfaceTheta seeded
     double *series_t = nullptr, *series_v = nullptr;   // thetaWallFunction -4 surface temperature series
@@ -333,6 +345,18 @@ void prof_flush(tg_ctx *C);
 constexpr int BX = 32, BY = 4, BZ = 2;
 inline dim3 grid3(int ni, int nj, int nk) { return dim3((ni + BX - 1) / BX, (nj + BY - 1) / BY, (nk + BZ - 1) / BZ); }
 inline dim3 block3() { return dim3(BX, BY, BZ); }
+
+// stage kernels on a mesh of planes (tg_tensor.cu)
+struct RkArgs;
+bool tensor_setup(tg_ctx *C);
+void contra_to_cart_tensor(tg_ctx *C, const char *name);
+void smagorinsky_tensor(tg_ctx *C);
+void grad_p_tensor(tg_ctx *C);
+void form_fp_tensor(tg_ctx *C, int mode);      // FormU passes 1 and 2, central convection
+void stage_fp_tensor(tg_ctx *C);               // an explicit stage's fp from Ucont
+void stage_tail_tensor(tg_ctx *C);             // boundary planes after the last such stage
+void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk);
+void project_tensor(tg_ctx *C);
 
 // stage entry points (tg_step.cu)
 void metrics_from_nodes(tg_ctx *C, const double *d_nodes);

@@ -7,6 +7,7 @@
 
 #include "tg_internal.cuh"
 #include "tg_mo.cuh"
+#include "tg_rk.cuh"
 
 namespace tg {
 namespace {
@@ -28,22 +29,9 @@ __device__ __forceinline__ R3<To> cvta(R3<From> a) { return R3<To>{(To)a.x, (To)
 // mode), A the arithmetic type; Ucont and Ucat stay FP64.
 // ------------------------------------------------------------------------
 template <class A, class MS>
-__device__ __forceinline__ void contra_cell(const Grid &g, const FaceMet<MS> &m, const State &s, int c, bool ax)
+__device__ __forceinline__ void contra_cell(const Grid &g, const FaceMet<MS> &m, const State &s, int c)
 {
     using M = A;
-    if (ax) {
-        // axis-aligned mesh: [csi; eta; zet] = [0 cs 0; 0 0 et; ze 0 0], the
-        // same Cramer products without the vanishing ones
-        const M cs = (M)m.csi.y[c], et = (M)m.eta.z[c], ze = (M)m.zet.x[c];
-        const M q0 = (M)(0.5 * (s.ucont.x[c - 1] + s.ucont.x[c]));
-        const M q1 = (M)(0.5 * (s.ucont.y[c - g.mx] + s.ucont.y[c]));
-        const M q2 = (M)(0.5 * (s.ucont.z[c - g.mx * g.my] + s.ucont.z[c]));
-        const M det = cs * (et * ze);
-        s.ucat.x[c] = (double)((q2 * (cs * et)) / det);
-        s.ucat.y[c] = (double)((q0 * (et * ze)) / det);
-        s.ucat.z[c] = (double)((q1 * (cs * ze)) / det);
-        return;
-    }
     R3<M> sc = cvta<M>(ld3(m.csi, c)), e = cvta<M>(ld3(m.eta, c)), z = cvta<M>(ld3(m.zet, c));
     M m00 = sc.x, m01 = sc.y, m02 = sc.z, m10 = e.x, m11 = e.y, m12 = e.z, m20 = z.x, m21 = z.y, m22 = z.z;
     M q0 = (M)(0.5 * (s.ucont.x[c - 1] + s.ucont.x[c]));
@@ -57,17 +45,17 @@ __device__ __forceinline__ void contra_cell(const Grid &g, const FaceMet<MS> &m,
 }
 
 template <class A, class MS>
-__global__ void k_contra_to_cart(Grid g, FaceMet<MS> m, State s, bool ax)
+__global__ void k_contra_to_cart(Grid g, FaceMet<MS> m, State s)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
-    contra_cell<A>(g, m, s, g.lin(k, j, i), ax);
+    contra_cell<A>(g, m, s, g.lin(k, j, i));
 }
 
 // the same on the interior cells next to the boundary only: the cells whose
 // Cartesian velocity reaches the ghost cells through the periodic copies.
 // blockIdx.z selects the boundary plane.
-__global__ void k_contra_to_cart_shell(Grid g, FaceMet<double> m, State s, bool ax)
+__global__ void k_contra_to_cart_shell(Grid g, FaceMet<double> m, State s)
 {
     int patch = blockIdx.z;
     int dir = patch >> 1, right = patch & 1;
@@ -78,7 +66,7 @@ __global__ void k_contra_to_cart_shell(Grid g, FaceMet<double> m, State s, bool 
     if (dir == 0) { k = b; j = a; i = right ? g.mx - 2 : 1; }
     else if (dir == 1) { k = b; i = a; j = right ? g.my - 2 : 1; }
     else { j = b; i = a; k = right ? g.mz - 2 : 1; }
-    contra_cell<double>(g, m, s, g.lin(k, j, i), ax);
+    contra_cell<double>(g, m, s, g.lin(k, j, i));
 }
 
 // FP32 copies of the stencil metrics
@@ -272,7 +260,7 @@ __global__ void k_scalar_ghosts(Grid g, double *v, int dir)
 // Compute_du_dxyz (inline.h:3635-3663). Interior cells.
 // ------------------------------------------------------------------------
 template <class M>
-__global__ void k_smagorinsky(Grid g, FaceMet<M> m, State s, Params p, bool ax)
+__global__ void k_smagorinsky(Grid g, FaceMet<M> m, State s, Params p)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
@@ -293,23 +281,15 @@ __global__ void k_smagorinsky(Grid g, FaceMet<M> m, State s, Params p, bool ax)
     else                        dz = 0.5 * (U(k + 1, j, i) - U(k - 1, j, i));
     const R3<M> a = cvta<M>(dc), b = cvta<M>(de), d = cvta<M>(dz);
     const M h = M(0.5);
-    M du_dx, du_dy, du_dz, dv_dx, dv_dy, dv_dz, dw_dx, dw_dy, dw_dz;
-    if (ax) {
-        // axis-aligned mesh: csi = (0, cs, 0), eta = (0, 0, et), zet = (ze, 0, 0)
-        du_dx = (d.x * z.x) * ajc; du_dy = (a.x * sc.y) * ajc; du_dz = (b.x * e.z) * ajc;
-        dv_dx = (d.y * z.x) * ajc; dv_dy = (a.y * sc.y) * ajc; dv_dz = (b.y * e.z) * ajc;
-        dw_dx = (d.z * z.x) * ajc; dw_dy = (a.z * sc.y) * ajc; dw_dz = (b.z * e.z) * ajc;
-    } else {
-        du_dx = (a.x * sc.x + b.x * e.x + d.x * z.x) * ajc;
-        du_dy = (a.x * sc.y + b.x * e.y + d.x * z.y) * ajc;
-        du_dz = (a.x * sc.z + b.x * e.z + d.x * z.z) * ajc;
-        dv_dx = (a.y * sc.x + b.y * e.x + d.y * z.x) * ajc;
-        dv_dy = (a.y * sc.y + b.y * e.y + d.y * z.y) * ajc;
-        dv_dz = (a.y * sc.z + b.y * e.z + d.y * z.z) * ajc;
-        dw_dx = (a.z * sc.x + b.z * e.x + d.z * z.x) * ajc;
-        dw_dy = (a.z * sc.y + b.z * e.y + d.z * z.y) * ajc;
-        dw_dz = (a.z * sc.z + b.z * e.z + d.z * z.z) * ajc;
-    }
+    const M du_dx = (a.x * sc.x + b.x * e.x + d.x * z.x) * ajc;
+    const M du_dy = (a.x * sc.y + b.x * e.y + d.x * z.y) * ajc;
+    const M du_dz = (a.x * sc.z + b.x * e.z + d.x * z.z) * ajc;
+    const M dv_dx = (a.y * sc.x + b.y * e.x + d.y * z.x) * ajc;
+    const M dv_dy = (a.y * sc.y + b.y * e.y + d.y * z.y) * ajc;
+    const M dv_dz = (a.y * sc.z + b.y * e.z + d.y * z.z) * ajc;
+    const M dw_dx = (a.z * sc.x + b.z * e.x + d.z * z.x) * ajc;
+    const M dw_dy = (a.z * sc.y + b.z * e.y + d.z * z.y) * ajc;
+    const M dw_dz = (a.z * sc.z + b.z * e.z + d.z * z.z) * ajc;
     M S00 = h * (du_dx + du_dx), S01 = h * (du_dy + dv_dx), S02 = h * (du_dz + dw_dx);
     M S10 = h * (dv_dx + du_dy), S11 = h * (dv_dy + dv_dy), S12 = h * (dv_dz + dw_dy);
     M S20 = h * (dw_dx + du_dz), S21 = h * (dw_dy + dv_dz), S22 = h * (dw_dz + dw_dz);
@@ -454,7 +434,7 @@ __global__ void k_wall_stress(Grid g, Metrics m, State s, Params p, const double
 // (ueqn_solvers.c:1314-1324); the products are associated as (g z) (grad .
 // S) aj, the reference's g z (grad . S) aj up to rounding
 template <class M, bool GH = false>
-__global__ void k_grad_p(Grid g, FaceMet<M> m, State s, bool ax, const double *node_z = nullptr, double t_ref = 0.0)
+__global__ void k_grad_p(Grid g, FaceMet<M> m, State s, const double *node_z = nullptr, double t_ref = 0.0)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
@@ -464,22 +444,6 @@ __global__ void k_grad_p(Grid g, FaceMet<M> m, State s, bool ax, const double *n
         return GH ? (t_ref - v) / t_ref : v;
     };
     const int mx = g.mx, my = g.my, mz = g.mz;
-    if (ax && !GH) {
-        // axis-aligned mesh: the cross terms g12, g13, g21, g23, g31, g32 vanish
-        // the + neighbours lie inside the DMDA except across a periodic seam,
-        // where index m + 1 wraps to 1
-        const M ic = m.icsi.y[c], je = m.jeta.z[c], kz = m.kzet.x[c];
-        const double pc = s.p[c];
-        const double dpdc = ((i == mx - 2 && g.pi) ? s.p[g.lin(k, j, 1)] : s.p[c + 1]) - pc;
-        const double dpde = ((j == my - 2 && g.pj) ? s.p[g.lin(k, 1, i)] : s.p[c + mx]) - pc;
-        const double dpdz = ((k == mz - 2 && g.pk) ? s.p[g.lin(1, j, i)] : s.p[c + mx * my]) - pc;
-        M ox = ((M)dpdc * (ic * ic)) * m.iaj[c], oy = ((M)dpde * (je * je)) * m.jaj[c], oz = ((M)dpdz * (kz * kz)) * m.kaj[c];
-        if (!g.pi && i == mx - 2) ox = 0;
-        if (!g.pj && j == my - 2) oy = 0;
-        if (!g.pk && k == mz - 2) oz = 0;
-        s.dp.x[c] = (double)ox; s.dp.y[c] = (double)oy; s.dp.z[c] = (double)oz;
-        return;
-    }
     R3<M> ic = ld3(m.icsi, c), ie = ld3(m.ieta, c), iz = ld3(m.izet, c);
     R3<M> jc = ld3(m.jcsi, c), je = ld3(m.jeta, c), jz = ld3(m.jzet, c);
     R3<M> kc = ld3(m.kcsi, c), ke = ld3(m.keta, c), kz = ld3(m.kzet, c);
@@ -833,25 +797,6 @@ __global__ void k_cell_fp(Grid g, FluxWork<F> w)
     st3(w.fp, g.lin(k, j, i), cell_fp(g, w, k, j, i));
 }
 
-// Explicit time update of one face value u with right-hand side r (UeqnFE,
-// ueqn_solvers.c:1411-1442: U = r dt + U_o; UeqnRK4, ueqn_solvers.c:1446-1504,
-// stage st: Utmp = U_o + b_st dt r (st = 0) or Utmp + b_st dt r, U = U_o +
-// a_{st+1} dt r, after the last stage U = Utmp + b_3 dt r), in the order of
-// the reference's VecScale / VecAXPY / VecWAXPY calls.
-struct RkArgs {
-    double cb, ca;      // b_st dt (FE: dt), a_{st+1} dt
-    int first, last, fe;
-};
-__device__ __forceinline__ void rk_point(double *uc, double *ut, const double *uo, double r, const RkArgs &a)
-{
-    if (a.fe) { *uc = r * a.cb + *uo; return; }
-    if (a.last) { *uc = a.cb * r + *ut; return; }
-    const double o = *uo;
-    if (a.first) *ut = a.cb * r + o;
-    else *ut = *ut + a.cb * r;
-    *uc = a.ca * r + o;
-}
-
 // Pass 3 (ueqn_solvers.c:1008-1035): rhs_face += scale * aj_face *
 // central(S . fp) at the faces of interior cells, fp of the cell and of its
 // +i, +j, +k neighbours read from pass 2. The neighbour beyond the last
@@ -866,7 +811,7 @@ __device__ __forceinline__ void rk_point(double *uc, double *ut, const double *u
 // 1 the ExplicitRhsU value is stored in R; 2 it is not stored but masked at
 // the non-resolved faces and applied at once by the explicit time update
 // (rk_point, one RK4 stage or the FE step).
-template <class MR, class F, int kind, bool AX>
+template <class MR, class F, int kind>
 __global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State s, FluxWork<F> w, V3f<double> R, double scale, Params p, int ab2, RkArgs rk)
 {
     constexpr bool fused = kind >= 1;
@@ -876,15 +821,11 @@ __global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State 
     // the value of the three faces: stored, or masked and applied (kind 2)
     auto finish = [&](double ox, double oy, double oz) {
         if (kind == 2) {
-            // resetNonResolvedCellFaces (inline.h:1674-1835) on the + faces of
-            // the last interior cells of a non-periodic direction (kept for
-            // outflow and on a zeroGradient patch)
-            if (!g.pi && i == g.mx - 2 && !(p.bc[TG_IRIGHT] == TG_BC_ZERO_GRADIENT || s.ucont_o.x[c] > 0)) ox = 0.0;
-            if (!g.pj && j == g.my - 2 && !(p.bc[TG_JRIGHT] == TG_BC_ZERO_GRADIENT || s.ucont_o.y[c] > 0)) oy = 0.0;
-            if (!g.pk && k == g.mz - 2 && !(p.bc[TG_KRIGHT] == TG_BC_ZERO_GRADIENT || s.ucont_o.z[c] > 0)) oz = 0.0;
-            rk_point(s.ucont.x + c, s.utmp.x + c, s.ucont_o.x + c, ox, rk);
-            rk_point(s.ucont.y + c, s.utmp.y + c, s.ucont_o.y + c, oy, rk);
-            rk_point(s.ucont.z + c, s.utmp.z + c, s.ucont_o.z + c, oz, rk);
+            R3<double> o{ox, oy, oz};
+            mask_last_faces(g, s, p, k, j, i, c, o);
+            rk_point(s.ucont.x + c, s.utmp.x + c, s.ucont_o.x + c, o.x, rk);
+            rk_point(s.ucont.y + c, s.utmp.y + c, s.ucont_o.y + c, o.y, rk);
+            rk_point(s.ucont.z + c, s.utmp.z + c, s.ucont_o.z + c, o.z, rk);
         } else {
             R.x[c] = ox; R.y[c] = oy; R.z[c] = oz;
         }
@@ -913,32 +854,6 @@ __global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State 
     const M sc = (M)scale, h = M(0.5);
     M v1, v2;
     double ox, oy, oz;
-    if (AX) {
-        // axis-aligned mesh: S . fp is csi.y fp.y, eta.z fp.z, zet.x fp.x
-        const int pl = g.mx * g.my;
-        const int ie = i < g.mx - 2 ? c + 1 : (g.pi ? g.lin(k, j, 1) : c);
-        const int jn = j < g.my - 2 ? c + g.mx : (g.pj ? g.lin(k, 1, i) : c);
-        const int kt = k < g.mz - 2 ? c + pl : (g.pk ? g.lin(1, j, i) : c);
-        v1 = (M)m.csi.y[c] * (M)w.fp.y[c]; v2 = (M)m.csi.y[c + 1] * (M)w.fp.y[ie];
-        ox = base.x + (double)(sc * (M)m.iaj[c] * (h * (v1 + v2)));
-        v1 = (M)m.eta.z[c] * (M)w.fp.z[c]; v2 = (M)m.eta.z[c + g.mx] * (M)w.fp.z[jn];
-        oy = base.y + (double)(sc * (M)m.jaj[c] * (h * (v1 + v2)));
-        v1 = (M)m.zet.x[c] * (M)w.fp.x[c]; v2 = (M)m.zet.x[c + pl] * (M)w.fp.x[kt];
-        oz = base.z + (double)(sc * (M)m.kaj[c] * (h * (v1 + v2)));
-        if (fused && p.source) {
-            const V3f<double> &f = s.source;
-            ox += 1.0 * (0.5 * (f.y[c] + f.y[c + 1]) * (double)m.icsi.y[c]);
-            oy += 1.0 * (0.5 * (f.z[c] + f.z[c + g.mx]) * (double)m.jeta.z[c]);
-            oz += 1.0 * (0.5 * (f.x[c] + f.x[c + pl]) * (double)m.kzet.x[c]);
-        }
-        if (fused && p.mean_grad_p) {
-            ox += (double)((M)p.mgp[1] * (M)m.icsi.y[c]);
-            oy += (double)((M)p.mgp[2] * (M)m.jeta.z[c]);
-            oz += (double)((M)p.mgp[0] * (M)m.kzet.x[c]);
-        }
-        finish(ox, oy, oz);
-        return;
-    }
     const R3<M> fpc = FP(k, j, i);
     { R3<M> fb = i < g.mx - 2 ? FP(k, j, i + 1) : (g.pi ? FP(k, j, 1) : fpc);
       R3<M> a = MT(m.csi, c), b = MT(m.csi, c + 1);
@@ -1094,29 +1009,13 @@ __global__ void k_non_resolved(Grid g, State s, Params p, int dir)
 // metric tensor; faces 0 and m-2 skipped unless periodic.
 // ------------------------------------------------------------------------
 template <class M>
-__global__ void k_project(Grid g, FaceMet<M> m, State s, double dt, bool ax)
+__global__ void k_project(Grid g, FaceMet<M> m, State s, double dt)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z * blockDim.z + threadIdx.z;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
     const int mx = g.mx, my = g.my, mz = g.mz;
     int f = g.lin(k, j, i);
     auto F = [&](int kk, int jj, int ii) { return s.phi[g.id(kk, jj, ii)]; };
-    if (ax) {
-        // axis-aligned mesh: only the normal derivative of phi has a metric weight
-        if (j > 0 && k > 0 && ((i > 0 && i < mx - 2) || g.pi)) {
-            const double c1 = (double)m.icsi.y[f];
-            s.ucont.x[f] -= ((F(k, j, i + 1) - F(k, j, i)) * (c1 * c1) * (double)m.iaj[f]) * dt;
-        }
-        if (i > 0 && k > 0 && ((j > 0 && j < my - 2) || g.pj)) {
-            const double e2 = (double)m.jeta.z[f];
-            s.ucont.y[f] -= ((F(k, j + 1, i) - F(k, j, i)) * (e2 * e2) * (double)m.jaj[f]) * dt;
-        }
-        if (i > 0 && j > 0 && ((k > 0 && k < mz - 2) || g.pk)) {
-            const double z3 = (double)m.kzet.x[f];
-            s.ucont.z[f] -= ((F(k + 1, j, i) - F(k, j, i)) * (z3 * z3) * (double)m.kaj[f]) * dt;
-        }
-        return;
-    }
     if (j > 0 && k > 0 && ((i > 0 && i < mx - 2) || g.pi)) {
         double dpdc = F(k, j, i + 1) - F(k, j, i), dpde, dpdz;
         if (j == my - 2)      dpde = (F(k, j, i) + F(k, j, i + 1) - F(k, j - 1, i) - F(k, j - 1, i + 1)) * 0.5;
@@ -1240,17 +1139,19 @@ inline int nblk(int64_t n) { int64_t b = (n + 255) / 256; return (int)(b < 148 *
 // error of p against the FP64 oracle rose to 3.3e-6 in 5 steps (ABL 16x16x12)
 void contra_to_cart(tg_ctx *C)
 {
-    TG_PROF(C, "contra_to_cart_final", k_contra_to_cart<double, double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s, C->axis_aligned));
+    if (C->axis_aligned) { contra_to_cart_tensor(C, "contra_to_cart_final"); return; }
+    TG_PROF(C, "contra_to_cart_final", k_contra_to_cart<double, double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
 }
 
 // contravariantToCartesian inside the momentum stages, at the precision the
 // context's policy gives it
 void contra_to_cart_stage(tg_ctx *C)
 {
+    if (C->axis_aligned) { contra_to_cart_tensor(C, "contra_to_cart"); return; }
     const dim3 gr = gi(C->g);
-    if (C->pol.contra_a32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<float, float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s, C->axis_aligned));
-    else if (C->pol.contra_m32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<double, float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s, C->axis_aligned));
-    else TG_PROF(C, "contra_to_cart", k_contra_to_cart<double, double><<<gr, block3(), 0, C->stream>>>(C->g, C->fm64, C->s, C->axis_aligned));
+    if (C->pol.contra_a32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<float, float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
+    else if (C->pol.contra_m32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<double, float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
+    else TG_PROF(C, "contra_to_cart", k_contra_to_cart<double, double><<<gr, block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
 }
 
 // Precision of each momentum stage in the mixed mode. Every momentum stencil
@@ -1398,8 +1299,9 @@ void update_nut(tg_ctx *C)
     const Grid g = C->g;
     TG_CUDA(cudaMemsetAsync(C->s.nut, 0, sizeof(double) * g.size(), C->stream));
     refresh_met32(C);
-    if (C->pol.smag32) TG_PROF(C, "smagorinsky", k_smagorinsky<float><<<gi(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm, C->axis_aligned));
-    else TG_PROF(C, "smagorinsky", k_smagorinsky<double><<<gi(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm, C->axis_aligned));
+    if (C->axis_aligned) smagorinsky_tensor(C);
+    else if (C->pol.smag32) TG_PROF(C, "smagorinsky", k_smagorinsky<float><<<gi(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm));
+    else TG_PROF(C, "smagorinsky", k_smagorinsky<double><<<gi(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm));
     int na = std::max(g.mx, g.my) - 2, nb = std::max(g.my, g.mz) - 2;
     dim3 grid((na + 31) / 32, (nb + 7) / 8, 6);
     TG_PROF(C, "bc_nut", k_nut_bcs<<<grid, b2, 0, C->stream>>>(g, C->s, C->prm));
@@ -1429,14 +1331,15 @@ void grad_p(tg_ctx *C)
         C->clear_dp = false;
     }
     refresh_met32(C);
-    if (C->pol.gradp32) TG_PROF(C, "grad_p", k_grad_p<float><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm32, C->s, C->axis_aligned));
-    else TG_PROF(C, "grad_p", k_grad_p<double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s, C->axis_aligned));
+    if (C->axis_aligned) grad_p_tensor(C);
+    else if (C->pol.gradp32) TG_PROF(C, "grad_p", k_grad_p<float><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
+    else TG_PROF(C, "grad_p", k_grad_p<double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
 }
 
 void buoyancy(tg_ctx *C)
 {
     if (C->cfg.p_tilde)   // ghGradRhoK (teqn.c:278), FP64
-        TG_PROF(C, "gh_grad_rhok", (k_grad_p<double, true><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s, false, C->node_z, C->prm.t_ref)));
+        TG_PROF(C, "gh_grad_rhok", (k_grad_p<double, true><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s, C->node_z, C->prm.t_ref)));
     else
         k_buoyancy<<<ga(C->g), block3(), 0, C->stream>>>(C->g, C->m, C->s, C->prm);
 }
@@ -1458,6 +1361,7 @@ static void face_fluxes(tg_ctx *C, dim3 gr)
 static void form_u_faces(tg_ctx *C, int mode)
 {
     const Grid g = C->g;
+    if (C->axis_aligned && C->prm.div_scheme == TG_DIV_CENTRAL) { form_fp_tensor(C, mode); return; }
     refresh_met32(C);
     // one thread per interior cell (k_face_fluxes)
     const dim3 gr((g.mx - 2 + FBX - 1) / FBX, (g.my - 2 + FBY - 1) / FBY, (g.mz - 2 + FBZ - 1) / FBZ);
@@ -1470,23 +1374,17 @@ static void form_u_faces(tg_ctx *C, int mode)
     else TG_PROF(C, "formu_cell_fp", k_cell_fp<double><<<gi(g), block3(), 0, C->stream>>>(g, C->fw64));
 }
 
-template <int fused, bool AX>
-static void rhs_faces_t(tg_ctx *C, V3f<double> rhs, double scale, int ab2, RkArgs rk)
-{
-    const Grid g = C->g;
-    const dim3 gr = gi(g);
-    const auto &P = C->pol;
-    if (P.rhs32 && P.flux32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<float, float, fused, AX><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw32, rhs, scale, C->prm, ab2, rk));
-    else if (P.rhs32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<float, double, fused, AX><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw64, rhs, scale, C->prm, ab2, rk));
-    else if (P.flux32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<double, float, fused, AX><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw32, rhs, scale, C->prm, ab2, rk));
-    else TG_PROF(C, "formu_rhs_faces", k_rhs_faces<double, double, fused, AX><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw64, rhs, scale, C->prm, ab2, rk));
-}
-
 template <int fused>
 static void rhs_faces(tg_ctx *C, V3f<double> rhs, double scale, int ab2, RkArgs rk = RkArgs{})
 {
-    if (C->axis_aligned) rhs_faces_t<fused, true>(C, rhs, scale, ab2, rk);
-    else rhs_faces_t<fused, false>(C, rhs, scale, ab2, rk);
+    if (C->axis_aligned) { rhs_faces_tensor(C, fused, rhs, scale, ab2, rk); return; }
+    const Grid g = C->g;
+    const dim3 gr = gi(g);
+    const auto &P = C->pol;
+    if (P.rhs32 && P.flux32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<float, float, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw32, rhs, scale, C->prm, ab2, rk));
+    else if (P.rhs32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<float, double, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw64, rhs, scale, C->prm, ab2, rk));
+    else if (P.flux32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<double, float, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw32, rhs, scale, C->prm, ab2, rk));
+    else TG_PROF(C, "formu_rhs_faces", k_rhs_faces<double, double, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw64, rhs, scale, C->prm, ab2, rk));
 }
 
 void form_u(tg_ctx *C, V3f<double> rhs, double scale, int mode)
@@ -1502,22 +1400,25 @@ void form_u_again(tg_ctx *C, V3f<double> rhs, double scale)
     rhs_faces<0>(C, rhs, scale, 0);
 }
 
+// every point outside the interior faces keeps Rhs = -dP + b = 0: zero from
+// the allocation, rewritten here only after a caller wrote Rhs
+static void clear_rhs(tg_ctx *C)
+{
+    if (!C->clear_rhs) return;
+    TG_CUDA(cudaMemsetAsync(C->s.rhs.x, 0, 3 * sizeof(double) * C->g.size(), C->stream));
+    C->clear_rhs = false;
+}
+
 // ExplicitRhsU up to the face fluxes: resets, Cartesian velocity, FormU passes 1-2
 static void explicit_rhs_head(tg_ctx *C, int mode)
 {
-    const Grid g = C->g;
     reset_no_penetration(C);
     reset_face_periodic(C, C->s.ucont);
     contra_to_cart_stage(C);
     reset_cell_periodic(C, C->s.ucat);
     if (C->taping) tape_stage(C);
     form_u_faces(C, mode);
-    // every point outside the interior faces keeps Rhs = -dP + b = 0: zero from
-    // the allocation, rewritten here only after a caller wrote Rhs
-    if (C->clear_rhs) {
-        TG_CUDA(cudaMemsetAsync(C->s.rhs.x, 0, 3 * sizeof(double) * g.size(), C->stream));
-        C->clear_rhs = false;
-    }
+    clear_rhs(C);
 }
 
 void explicit_rhs(tg_ctx *C, int mode)
@@ -1532,10 +1433,18 @@ void explicit_rhs(tg_ctx *C, int mode)
 
 // ExplicitRhsU followed by one explicit update (an RK4 stage or the FE step)
 // without storing Rhs: the face assembly applies the update at the faces of
-// the interior cells, k_rk_shell at every other point (zero right-hand side)
-static void explicit_rhs_update(tg_ctx *C, RkArgs rk)
+// the interior cells, k_rk_shell at every other point (zero right-hand side).
+// from_ucont: the stage reads Ucont alone (k_stage_fp), which needs the other
+// points as they were at the start of the step, so they are left alone
+static void explicit_rhs_update(tg_ctx *C, RkArgs rk, bool from_ucont)
 {
     const Grid g = C->g;
+    if (from_ucont) {
+        stage_fp_tensor(C);
+        clear_rhs(C);
+        rhs_faces<2>(C, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0, rk);
+        return;
+    }
     explicit_rhs_head(C, 0);
     rhs_faces<2>(C, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0, rk);
     dim3 grid((std::max(g.mx, g.my) + 31) / 32, (std::max(g.my, g.mz) + 7) / 8, 6);
@@ -1603,6 +1512,10 @@ static int solve_u_impl(tg_ctx *C, bool cart_tail, tg_stats *st = nullptr)
     const int64_t G = C->g.size();
     const double dt = C->prm.dt;
     int rc = 0;
+    // inside a step (Ucont_o = Ucont at its start) on a mesh of planes the
+    // stages read Ucont alone; a taped step records the Ucat of every stage
+    const bool lean = !cart_tail && !C->taping && C->axis_aligned && C->prm.div_scheme == TG_DIV_CENTRAL &&
+                      (C->cfg.ddt_scheme == TG_DDT_FE || C->cfg.ddt_scheme == TG_DDT_RK4);
     if (C->cfg.ddt_scheme == TG_DDT_CN) {
         // UeqnSNES, ueqn_solvers.c:1087-1199
         rc = solve_u_cn(C, st);
@@ -1611,15 +1524,20 @@ static int solve_u_impl(tg_ctx *C, bool cart_tail, tg_stats *st = nullptr)
         rc = solve_u_imex(C);
     } else if (C->cfg.ddt_scheme == TG_DDT_FE) {
         // UeqnFE, ueqn_solvers.c:1411-1442
-        explicit_rhs_update(C, RkArgs{dt, 0.0, 0, 0, 1});
+        explicit_rhs_update(C, RkArgs{dt, 0.0, 0, 0, 1}, lean);
     } else {
         // UeqnRK4, ueqn_solvers.c:1446-1504
         const double b[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
         const double a[4] = {0.0, 0.5, 0.5, 1.0};
         for (int st = 0; st < 4; st++)
-            explicit_rhs_update(C, RkArgs{dt * b[st], st < 3 ? a[st + 1] * dt : 0.0, st == 0 ? 1 : 0, st == 3 ? 1 : 0, 0});
+            explicit_rhs_update(C, RkArgs{dt * b[st], st < 3 ? a[st + 1] * dt : 0.0, st == 0 ? 1 : 0, st == 3 ? 1 : 0, 0}, lean);
     }
     // SolveUEqn tail, ueqn.c:413-437
+    if (lean) {
+        stage_tail_tensor(C);
+        adjust_fluxes(C);
+        return rc;
+    }
     reset_no_penetration(C);
     reset_face_periodic(C, C->s.ucont);
     if (cart_tail) {
@@ -1631,7 +1549,7 @@ static int solve_u_impl(tg_ctx *C, bool cart_tail, tg_stats *st = nullptr)
         const Grid g = C->g;
         int na = std::max(g.mx, g.my) - 2, nb = std::max(g.my, g.mz) - 2;
         dim3 grid((na + 31) / 32, (nb + 7) / 8, 6);
-        TG_PROF(C, "contra_to_cart_shell", k_contra_to_cart_shell<<<grid, b2, 0, C->stream>>>(g, C->fm64, C->s, C->axis_aligned));
+        TG_PROF(C, "contra_to_cart_shell", k_contra_to_cart_shell<<<grid, b2, 0, C->stream>>>(g, C->fm64, C->s));
     }
     reset_cell_periodic(C, C->s.ucat);
     adjust_fluxes(C);                  // ueqn.c:437
@@ -1648,9 +1566,10 @@ void pressure_update_and_project(tg_ctx *C)
     update_scalar_ghosts(C, C->s.phi);
     TG_PROF(C, "update_pressure", k_update_pressure<<<gi(g), block3(), 0, C->stream>>>(g, C->s));
     update_scalar_ghosts(C, C->s.p);
+    if (C->axis_aligned) { project_tensor(C); return; }
     refresh_met32(C);
-    if (C->pol.proj32) TG_PROF(C, "project", k_project<float><<<gf(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm.dt, C->axis_aligned));
-    else TG_PROF(C, "project", k_project<double><<<gf(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm.dt, C->axis_aligned));
+    if (C->pol.proj32) TG_PROF(C, "project", k_project<float><<<gf(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm.dt));
+    else TG_PROF(C, "project", k_project<double><<<gf(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm.dt));
 }
 
 int solve_p(tg_ctx *C, tg_stats *st)
