@@ -81,13 +81,19 @@ def test_against_general_kernels(kind, nx, ny, nz, over):
         s.FormU(0.7, True)
     tol = 1e-6 if mixed else 1e-12
     assert rel_l2(a.get("RHS"), b.get("RHS")) <= (1e-4 if mixed else tol)
-    for s in (a, b):
-        s.step(3)
+    # P is the sum of the steps' phi, each solved to a relative residual: where
+    # the first step's impulse cancels afterwards the error scales with the
+    # largest P, not the last
+    big = 0.0
+    for _ in range(3):
+        for s in (a, b):
+            s.step(1)
+        big = max(big, np.linalg.norm(b.get("P")))
     implicit = case[0].ddt_scheme not in (api.DDT_FE, api.DDT_RK4)
     for f in ("UCAT", "UCONT", "NUT"):
         whole = lambda x: x                               # noqa: E731  ghost layers too
         assert rel_l2(a.get(f), b.get(f), whole) <= (1e-9 if implicit else tol), f
-    assert rel_l2(a.get("P"), b.get("P")) <= (1e-5 if mixed else 1e-8 if implicit else 1e-9)
+    assert np.linalg.norm(a.get("P") - b.get("P")) <= (1e-5 if mixed else 1e-8 if implicit else 1e-9) * big
     a.close(); b.close()
 
 
@@ -99,10 +105,7 @@ def test_against_oracle(kind, nx, ny, nz, over):
         cases.setup(s, nodes, u, p, T)
         s.FormU(1.0, True)
     assert rel_l2(g.get("RHS"), o.get("RHS")) <= 1e-12
-    # P is the sum of the steps' phi, each solved to a relative residual: where
-    # the first step's impulse cancels afterwards the error scales with the
-    # largest P, not the last
-    big = 0.0
+    big = 0.0                                              # see above
     for _ in range(3):
         for s in (g, o):
             s.step(1)

@@ -2,6 +2,7 @@
 // (FormU and its sources), explicit integrators, boundary/ghost updates,
 // projection and divergence. Each kernel restates one loop of the reference
 // (file:line at the kernel). All fields are SoA FP64 on the global DMDA extent.
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -75,43 +76,55 @@ __global__ void k_to_f32(int64_t n, const double *a, float *b)
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) b[q] = (float)a[q];
 }
 
+// points of the six boundary planes of the DMDA box, each once: blockIdx.z
+// selects the plane, 32 x 8 points per block. false outside it.
+__device__ __forceinline__ bool shell_point(const Grid &g, int &i, int &j, int &k)
+{
+    const int dir = blockIdx.z >> 1, right = blockIdx.z & 1;
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
+    if (dir == 0) { i = right ? g.mx - 1 : 0; j = a; k = b; return a < g.my && b < g.mz; }
+    if (dir == 1) { j = right ? g.my - 1 : 0; i = a + 1; k = b; return a < g.mx - 2 && b < g.mz; }
+    k = right ? g.mz - 1 : 0; i = a + 1; j = b + 1;
+    return a < g.mx - 2 && b < g.my - 2;
+}
+inline dim3 shell_grid(const Grid &g) { return dim3((std::max(g.mx, g.my) + 31) / 32, (std::max(g.my, g.mz) + 7) / 8, 6); }
+
 // ------------------------------------------------------------------------
 // resetCellPeriodicFluxes (inline.h:5453-5606): periodic ghost cells take the
-// first interior cell of the opposite side. One direction per launch; applied
-// i, then j, then k, which composes to the reference's simultaneous remap.
+// first interior cell of the opposite side, in every direction at once: a
+// point's source has no ghost index left in a periodic direction, so no
+// source is written and one launch does what a launch per direction did (a
+// launch of these planes costs 2 to 3 us whatever its size).
 // left_only: resetFacePeriodicFluxesVector (inline.h:5357-5451), face 0 <- m-2.
 // ------------------------------------------------------------------------
 template <int NC, class T>
-__global__ void k_periodic_copy(Grid g, T *a0, T *a1, T *a2, int dir, int left_only)
+__global__ void k_periodic_copy(Grid g, T *a0, T *a1, T *a2, int left_only)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
-    int na = dir == 0 ? g.my : g.mx, nb = dir == 2 ? g.my : g.mz;
-    if (a >= na || b >= nb) return;
-    for (int side = 0; side < (left_only ? 1 : 2); side++) {
-        int d, s;
-        if (dir == 0) { d = g.lin(b, a, side ? g.mx - 1 : 0); s = g.lin(b, a, side ? 1 : g.mx - 2); }
-        else if (dir == 1) { d = g.lin(b, side ? g.my - 1 : 0, a); s = g.lin(b, side ? 1 : g.my - 2, a); }
-        else { d = g.lin(side ? g.mz - 1 : 0, b, a); s = g.lin(side ? 1 : g.mz - 2, b, a); }
-        a0[d] = a0[s];
-        if (NC == 3) { a1[d] = a1[s]; a2[d] = a2[s]; }
-    }
+    int i, j, k;
+    if (!shell_point(g, i, j, k)) return;
+    auto src = [&](int l, int m, int per) { return !per ? l : l == 0 ? m - 2 : (l == m - 1 && !left_only) ? 1 : l; };
+    const int d = g.lin(k, j, i), s = g.lin(src(k, g.mz, g.pk), src(j, g.my, g.pj), src(i, g.mx, g.pi));
+    if (s == d) return;
+    a0[d] = a0[s];
+    if (NC == 3) { a1[d] = a1[s]; a2[d] = a2[s]; }
 }
 
 template <int NC, class T>
 void periodic_copy(tg_ctx *C, T *a0, T *a1, T *a2, int left_only)
 {
     const Grid g = C->g;
-    if (g.pi) TG_PROF(C, "bc_periodic_copy", k_periodic_copy<NC, T><<<g2(g.my, g.mz), b2, 0, C->stream>>>(g, a0, a1, a2, 0, left_only));
-    if (g.pj) TG_PROF(C, "bc_periodic_copy", k_periodic_copy<NC, T><<<g2(g.mx, g.mz), b2, 0, C->stream>>>(g, a0, a1, a2, 1, left_only));
-    if (g.pk) TG_PROF(C, "bc_periodic_copy", k_periodic_copy<NC, T><<<g2(g.mx, g.my), b2, 0, C->stream>>>(g, a0, a1, a2, 2, left_only));
+    if (!g.pi && !g.pj && !g.pk) return;
+    TG_PROF(C, "bc_periodic_copy", k_periodic_copy<NC, T><<<shell_grid(g), b2, 0, C->stream>>>(g, a0, a1, a2, left_only));
 }
 
 // ------------------------------------------------------------------------
 // resetNoPenetrationFluxes (inline.h:5262-5355): zero wall-normal fluxes on
-// wall patches. Plane launch per direction; range [0, m-2] in the others.
+// wall patches. blockIdx.z selects the direction; range [0, m-2] in the others.
+// walls: bit q set if patch q is a wall.
 // ------------------------------------------------------------------------
-__global__ void k_no_penetration(Grid g, State s, int dir, int left, int right)
+__global__ void k_no_penetration(Grid g, State s, int walls)
 {
+    const int dir = blockIdx.z, left = (walls >> (2 * dir)) & 1, right = (walls >> (2 * dir + 1)) & 1;
     int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
     int na = (dir == 0 ? g.my : g.mx) - 1, nb = (dir == 2 ? g.my : g.mz) - 1;
     if (a >= na || b >= nb) return;
@@ -189,23 +202,14 @@ __global__ void k_cartesian_bcs(Grid g, Metrics m, State s, Params p)
 }
 
 // ------------------------------------------------------------------------
-// UpdateContravariantBCs (boundary.c:614-822). Two passes: periodic left
-// faces take the solved right face (from the pre-call values), then the
-// right/left faces of non-wall patches are re-interpolated from Ucat and
-// wall faces zeroed.
+// UpdateContravariantBCs (boundary.c:614-822). Periodic left faces take the
+// solved right face (its value before this call), then the right/left faces of
+// non-wall patches are re-interpolated from Ucat and wall faces zeroed.
+// blockIdx.z selects the direction; each direction writes its own component.
 // ------------------------------------------------------------------------
-__global__ void k_contra_bc_periodic(Grid g, State s, int dir)
+__global__ void k_contra_bc_faces(Grid g, Metrics m, State s, Params p)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
-    int na = (dir == 0 ? g.my : g.mx) - 1, nb = (dir == 2 ? g.my : g.mz) - 1;
-    if (a >= na || b >= nb) return;
-    if (dir == 0) s.ucont.x[g.lin(b, a, 0)] = s.ucont.x[g.lin(b, a, g.mx - 2)];
-    else if (dir == 1) s.ucont.y[g.lin(b, 0, a)] = s.ucont.y[g.lin(b, g.my - 2, a)];
-    else s.ucont.z[g.lin(0, b, a)] = s.ucont.z[g.lin(g.mz - 2, b, a)];
-}
-
-__global__ void k_contra_bc_faces(Grid g, Metrics m, State s, Params p, int dir)
-{
+    const int dir = blockIdx.z;
     int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
     int na = (dir == 0 ? g.my : g.mx) - 1, nb = (dir == 2 ? g.my : g.mz) - 1;
     if (a >= na || b >= nb) return;
@@ -213,12 +217,12 @@ __global__ void k_contra_bc_faces(Grid g, Metrics m, State s, Params p, int dir)
         int patch = 2 * dir + side;
         int type = p.bc[patch];
         bool periodic = type == TG_BC_PERIODIC;
-        if (periodic && side == 0) continue;   // left periodic face handled by the copy pass
         int f, step;
         if (dir == 0) { f = g.lin(b, a, side ? g.mx - 2 : 0); step = 1; }
         else if (dir == 1) { f = g.lin(b, side ? g.my - 2 : 0, a); step = g.mx; }
         else { f = g.lin(side ? g.mz - 2 : 0, b, a); step = g.mx * g.my; }
         double *u = dir == 0 ? s.ucont.x : (dir == 1 ? s.ucont.y : s.ucont.z);
+        if (periodic && side == 0) { u[f] = u[f + step * ((dir == 0 ? g.mx : dir == 1 ? g.my : g.mz) - 2)]; continue; }
         if (is_wall(type)) { u[f] = 0.0; continue; }
         R3<double> un = ld3(s.ucat, f + step), uc = ld3(s.ucat, f);
         R3<double> S = dir == 0 ? ld3(m.icsi, f) : (dir == 1 ? ld3(m.jeta, f) : ld3(m.kzet, f));
@@ -232,26 +236,15 @@ __global__ void k_contra_bc_faces(Grid g, Metrics m, State s, Params p, int dir)
 // ------------------------------------------------------------------------
 // UpdatePhiBCs (boundary.c:3168-3255) / UpdatePressureBCs (boundary.c:3051-3166):
 // ghost cells copy the first interior cell (zero gradient) or the opposite
-// interior cell (periodic). Sequential per-direction passes compose to the
-// reference's simultaneous remap because every source is interior in the
-// remapped direction.
+// interior cell (periodic); edges and corners remap every index at once (every
+// source is an interior cell).
 // ------------------------------------------------------------------------
-__global__ void k_scalar_ghosts(Grid g, double *v, int dir)
+__global__ void k_scalar_ghosts(Grid g, double *v)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
-    int na = dir == 0 ? g.my : g.mx, nb = dir == 2 ? g.my : g.mz;
-    if (a >= na || b >= nb) return;
-    int per = dir == 0 ? g.pi : (dir == 1 ? g.pj : g.pk);
-    int m = dir == 0 ? g.mx : (dir == 1 ? g.my : g.mz);
-    for (int side = 0; side < 2; side++) {
-        int dd = side ? m - 1 : 0;
-        int ss = side ? (per ? 1 : m - 2) : (per ? m - 2 : 1);
-        int d, s;
-        if (dir == 0) { d = g.lin(b, a, dd); s = g.lin(b, a, ss); }
-        else if (dir == 1) { d = g.lin(b, dd, a); s = g.lin(b, ss, a); }
-        else { d = g.lin(dd, b, a); s = g.lin(ss, b, a); }
-        v[d] = v[s];
-    }
+    int i, j, k;
+    if (!shell_point(g, i, j, k)) return;
+    auto src = [](int l, int m, int per) { return l == 0 ? (per ? m - 2 : 1) : l == m - 1 ? (per ? 1 : m - 2) : l; };
+    v[g.lin(k, j, i)] = v[g.lin(src(k, g.mz, g.pk), src(j, g.my, g.pj), src(i, g.mx, g.pi))];
 }
 
 // ------------------------------------------------------------------------
@@ -892,12 +885,8 @@ __global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State 
 // once
 __global__ void k_rk_shell(Grid g, State s, RkArgs rk)
 {
-    const int patch = blockIdx.z, dir = patch >> 1, right = patch & 1;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
     int i, j, k;
-    if (dir == 0) { if (a >= g.my || b >= g.mz) return; i = right ? g.mx - 1 : 0; j = a; k = b; }
-    else if (dir == 1) { if (a >= g.mx - 2 || b >= g.mz) return; j = right ? g.my - 1 : 0; i = a + 1; k = b; }
-    else { if (a >= g.mx - 2 || b >= g.my - 2) return; k = right ? g.mz - 1 : 0; i = a + 1; j = b + 1; }
+    if (!shell_point(g, i, j, k)) return;
     const int c = g.lin(k, j, i);
     rk_point(s.ucont.x + c, s.utmp.x + c, s.ucont_o.x + c, 0.0, rk);
     rk_point(s.ucont.y + c, s.utmp.y + c, s.ucont_o.y + c, 0.0, rk);
@@ -983,12 +972,13 @@ __global__ void k_flux_correct(Grid g, State s, Params p, const double *sc)
     }
 }
 
-// resetNonResolvedCellFaces (inline.h:1674-1835) on the boundary planes of one
-// direction: face 0 kept only for outflow or on a zeroGradient patch, face m-1
+// resetNonResolvedCellFaces (inline.h:1674-1835) on the boundary planes of
+// direction blockIdx.z, which has its own component: face 0 kept only for outflow or on a zeroGradient patch, face m-1
 // unused, face m-2 of a non-periodic direction kept only for outflow or on a
 // zeroGradient patch.
-__global__ void k_non_resolved(Grid g, State s, Params p, int dir)
+__global__ void k_non_resolved(Grid g, State s, Params p)
 {
+    const int dir = blockIdx.z;
     int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
     int na = dir == 0 ? g.my : g.mx, nb = dir == 2 ? g.my : g.mz;
     if (a >= na || b >= nb) return;
@@ -1247,13 +1237,12 @@ void reset_no_penetration(tg_ctx *C)
 {
     const Grid g = C->g;
     const int *bc = C->prm.bc;
-    auto w = [](int t) { return t == TG_BC_NOSLIP || t == TG_BC_SLIP || t == TG_BC_WALL_SHUMANN; };
-    for (int d = 0; d < 3; d++) {
-        int l = w(bc[2 * d]), r = w(bc[2 * d + 1]);
-        if (!l && !r) continue;
-        int na = d == 0 ? g.my : g.mx, nb = d == 2 ? g.my : g.mz;
-        TG_PROF(C, "bc_no_penetration", k_no_penetration<<<g2(na, nb), b2, 0, C->stream>>>(g, C->s, d, l, r));
-    }
+    int walls = 0;
+    for (int q = 0; q < 6; q++) if (bc[q] == TG_BC_NOSLIP || bc[q] == TG_BC_SLIP || bc[q] == TG_BC_WALL_SHUMANN) walls |= 1 << q;
+    if (!walls) return;
+    dim3 gr = shell_grid(g);
+    gr.z = 3;
+    TG_PROF(C, "bc_no_penetration", k_no_penetration<<<gr, b2, 0, C->stream>>>(g, C->s, walls));
 }
 
 void update_cartesian_bcs(tg_ctx *C)
@@ -1267,11 +1256,9 @@ void update_cartesian_bcs(tg_ctx *C)
 void update_contravariant_bcs(tg_ctx *C)
 {
     const Grid g = C->g;
-    for (int d = 0; d < 3; d++) {
-        int na = d == 0 ? g.my : g.mx, nb = d == 2 ? g.my : g.mz;
-        if (C->prm.bc[2 * d] == TG_BC_PERIODIC) k_contra_bc_periodic<<<g2(na, nb), b2, 0, C->stream>>>(g, C->s, d);
-        TG_PROF(C, "bc_contravariant", k_contra_bc_faces<<<g2(na, nb), b2, 0, C->stream>>>(g, C->m, C->s, C->prm, d));
-    }
+    dim3 gr = shell_grid(g);
+    gr.z = 3;
+    TG_PROF(C, "bc_contravariant", k_contra_bc_faces<<<gr, b2, 0, C->stream>>>(g, C->m, C->s, C->prm));
 }
 
 void adjust_fluxes(tg_ctx *C)
@@ -1288,10 +1275,7 @@ void adjust_fluxes(tg_ctx *C)
 
 void update_scalar_ghosts(tg_ctx *C, double *v)
 {
-    const Grid g = C->g;
-    TG_PROF(C, "bc_scalar_ghosts", k_scalar_ghosts<<<g2(g.my, g.mz), b2, 0, C->stream>>>(g, v, 0));
-    TG_PROF(C, "bc_scalar_ghosts", k_scalar_ghosts<<<g2(g.mx, g.mz), b2, 0, C->stream>>>(g, v, 1));
-    TG_PROF(C, "bc_scalar_ghosts", k_scalar_ghosts<<<g2(g.mx, g.my), b2, 0, C->stream>>>(g, v, 2));
+    TG_PROF(C, "bc_scalar_ghosts", k_scalar_ghosts<<<shell_grid(C->g), b2, 0, C->stream>>>(C->g, v));
 }
 
 void update_nut(tg_ctx *C)
@@ -1426,9 +1410,7 @@ void explicit_rhs(tg_ctx *C, int mode)
     const Grid g = C->g;
     explicit_rhs_head(C, mode);
     rhs_faces<1>(C, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0);
-    TG_PROF(C, "bc_non_resolved", k_non_resolved<<<g2(g.my, g.mz), b2, 0, C->stream>>>(g, C->s, C->prm, 0));
-    TG_PROF(C, "bc_non_resolved", k_non_resolved<<<g2(g.mx, g.mz), b2, 0, C->stream>>>(g, C->s, C->prm, 1));
-    TG_PROF(C, "bc_non_resolved", k_non_resolved<<<g2(g.mx, g.my), b2, 0, C->stream>>>(g, C->s, C->prm, 2));
+    mask_non_resolved(C, C->s.rhs);
 }
 
 // ExplicitRhsU followed by one explicit update (an RK4 stage or the FE step)
@@ -1447,8 +1429,7 @@ static void explicit_rhs_update(tg_ctx *C, RkArgs rk, bool from_ucont)
     }
     explicit_rhs_head(C, 0);
     rhs_faces<2>(C, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0, rk);
-    dim3 grid((std::max(g.mx, g.my) + 31) / 32, (std::max(g.my, g.mz) + 7) / 8, 6);
-    TG_PROF(C, "rk_shell", k_rk_shell<<<grid, dim3(32, 8), 0, C->stream>>>(g, C->s, rk));
+    TG_PROF(C, "rk_shell", k_rk_shell<<<shell_grid(g), b2, 0, C->stream>>>(g, C->s, rk));
 }
 
 // resetNonResolvedCellFaces (inline.h:1674-1835) on an arbitrary face vector
@@ -1457,9 +1438,9 @@ void mask_non_resolved(tg_ctx *C, V3f<double> v)
     const Grid g = C->g;
     State s = C->s;
     s.rhs = v;
-    k_non_resolved<<<g2(g.my, g.mz), b2, 0, C->stream>>>(g, s, C->prm, 0);
-    k_non_resolved<<<g2(g.mx, g.mz), b2, 0, C->stream>>>(g, s, C->prm, 1);
-    k_non_resolved<<<g2(g.mx, g.my), b2, 0, C->stream>>>(g, s, C->prm, 2);
+    dim3 gr = shell_grid(g);
+    gr.z = 3;
+    TG_PROF(C, "bc_non_resolved", k_non_resolved<<<gr, b2, 0, C->stream>>>(g, s, C->prm));
 }
 
 // constant part of the Crank-Nicolson residual (UeqnSNES, ueqn_solvers.c:1097-1163):
