@@ -48,7 +48,8 @@ struct Fdm {
     int nx, ny, nz, pj;
     int64_t n;
     FdmDir x, y, z;           // y: periodic j only
-    double *my, *ky;          // j factors (non-periodic j)
+    FdmOp op;
+    double dev;               // largest relative deviation of the coefficients from the factors
     double *minv;             // 1 / pivots of the j-line systems, per mode pair
 };
 
@@ -606,15 +607,16 @@ Fdm *fdm_create(tg_ctx *C, const double *aE, const double *aN, const double *aT,
         bool ok = true;
         // rounding of the metrics leaves about 1e-15; the factors only have to
         // be close, as CG iterates on the exact operator
-        for (double v : part) ok = ok && v <= 1e-10;
+        F->dev = 0.0;
+        for (double v : part) { ok = ok && v <= 1e-10; F->dev = std::max(F->dev, v); }
         ok = ok && setup_dir(C, F->x, nx, pi, kx, mx) && setup_dir(C, F->z, nz, pk, kz, mz);
         if (ok && pj) ok = setup_dir(C, F->y, ny, true, ky, my);
         ok = ok && F->x.gs + F->z.gs <= FDM_MAX_ROWS;
         if (!ok) { delete F; return nullptr; }
-        F->ky = dv[2]; F->my = dv[3];
+        F->op = FdmOp{dv[0], dv[1], dv[2], dv[3], dv[4], dv[5]};
         if (!pj) {
             F->minv = dallocd(C, (size_t)F->n);
-            k_fdm_factors<<<dim3((nx + 31) / 32, (nz + 3) / 4), dim3(32, 4), 0, st>>>(nx, ny, nz, F->x.lam, F->z.lam, F->my, F->ky, F->minv);
+            k_fdm_factors<<<dim3((nx + 31) / 32, (nz + 3) / 4), dim3(32, 4), 0, st>>>(nx, ny, nz, F->x.lam, F->z.lam, F->op.my, F->op.ky, F->minv);
         }
         set_attrs();
         TG_CUDA(cudaGetLastError());
@@ -624,6 +626,8 @@ Fdm *fdm_create(tg_ctx *C, const double *aE, const double *aN, const double *aT,
     }
     return F;
 }
+
+bool fdm_factors(const Fdm *F, FdmOp *op) { *op = F->op; return F->dev <= 1e-13; }
 
 void fdm_destroy(Fdm *F) { delete F; }   // device buffers are owned by the context allocation list
 
@@ -646,7 +650,7 @@ void fdm_apply(tg_ctx *C, Fdm *F, const double *r, const double *d_sum, double *
         ay.ly = nullptr;
         TG_PROF(C, "fdm_y_inv", (launch_xform<true, false>(F->y, ay, st)));
     } else {
-        TG_PROF(C, "fdm_lines", launch_lines(F->ky, F->minv, z, nx, ny, nz, st));
+        TG_PROF(C, "fdm_lines", launch_lines(F->op.ky, F->minv, z, nx, ny, nz, st));
     }
     TG_PROF(C, "fdm_z_inv", (launch_xform<true, false>(F->z, az, st)));
     ax.src = z; ax.d_sum = nullptr;

@@ -8,6 +8,13 @@ namespace tg {
 
 struct Fdm;   // opaque
 
+// the factors of the face coefficients (device arrays):
+// aE = kx_i my_j mz_k, aN = mx_i ky_j mz_k, aT = mx_i my_j kz_k
+struct FdmOp { const double *kx, *mx, *ky, *my, *kz, *mz; };
+// true if the factors reproduce the coefficients to rounding (1e-13), so that
+// the operator may be evaluated from them
+bool fdm_factors(const Fdm *F, FdmOp *op);
+
 // face coefficients as for mg_create (tg_mg.cuh). nullptr when the operator
 // does not separate or a direction is outside the solver's range; the caller
 // then uses the multigrid.

@@ -356,7 +356,9 @@ void form_fp_tensor(tg_ctx *C, int mode);      // FormU passes 1 and 2, central 
 void stage_fp_tensor(tg_ctx *C);               // an explicit stage's fp from Ucont
 void stage_tail_tensor(tg_ctx *C);             // boundary planes after the last such stage
 void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk);
-void project_tensor(tg_ctx *C);
+// phi, p (less *ref if given) and the projected Ucont from the compact solution x
+void pressure_project_tensor(tg_ctx *C, const double *x, const double *ref);
+void contra_div_tensor(tg_ctx *C);             // final Ucat and the partial divergence maxima (C->d_red, red_blocks)
 
 // stage entry points (tg_step.cu)
 void metrics_from_nodes(tg_ctx *C, const double *d_nodes);
@@ -399,11 +401,14 @@ void reduce_max_abs_div(tg_ctx *C, double *d_out);
 void poisson_setup(tg_ctx *C);
 void poisson_destroy(tg_ctx *C);
 int poisson_solve(tg_ctx *C, tg_stats *st);
+bool poisson_direct(const tg_ctx *C);        // the direct solver runs (it sets SC_PREF)
 void poisson_solve_capture(tg_ctx *C);       // the same solve with device-side loop control
 // device scalar slots (C->d_scal): statistics of captured solves, as offsets
 // from a base (SC_G: forward step, SC_ADJ: transposed solve), and the step counter
 constexpr int ST_IT = 0, ST_RES0 = 1, ST_RES = 2, ST_TOT = 3, ST_NOCONV = 4, ST_NAN = 5, ST_COUNT = 6;
 constexpr int SC_G = 60, SC_ADJ = 70, SC_IT = 80;
+// p(1,1,1) before the step's pressure update: its gauge
+constexpr int SC_PREF = 17;
 // solutions in the Poisson guess history (0, 1, 2 or more: order of the extrapolation)
 constexpr int SC_PHIST = 96;
 // thetaWallFunction averaged model: plane means and the resulting qWall

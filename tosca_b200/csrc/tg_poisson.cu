@@ -44,6 +44,9 @@ struct PoissonCtx {
     int nblocks;
     MG *mg;                      // multigrid preconditioner (host object), where fdm does not apply
     Fdm *fdm;                    // direct solve on a mesh of planes, else null
+    FdmOp op;                    // its factors, used for the operator if op_exact
+    bool op_exact;
+    unsigned *count;             // arrival counter of last_block
 };
 
 namespace {
@@ -393,6 +396,249 @@ __global__ void k_cg_dir(int64_t n, const double *sc, const double *z, double *p
     if (odd_tail(n)) p[n - 1] = first ? z[n - 1] - z0 : z[n - 1] - z0 + beta * p[n - 1];
 }
 
+// ---------------------------------------------- solve with the direct solver
+// The iteration with the direct solve as preconditioner. It reduces the
+// residual to near rounding at once, so directions need no conjugation: each
+// pass takes z = M r and the step length that CG's first iteration takes,
+// alpha = (r, z) / (z, L z), and reads z where CG reads its direction p. The
+// vector work of a solve is four kernels (before: 14 launches, and at
+// 256 x 256 x 128 0.61 ms where these take 0.29 ms), each with its dot products
+// finished by the last block to arrive. Threads take rows of the compact grid (a
+// warp per row, lanes along i), so that 3-D indices cost one division per row.
+struct Rows {
+    int nx, ny, nrow, lane, row, step;
+    __device__ __forceinline__ Rows(const PoissonCtx &P)
+        : nx(P.nx), ny(P.ny), nrow(P.ny * P.nz), lane(threadIdx.x & 31),
+          row((int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5)), step((int)((gridDim.x * blockDim.x) >> 5)) {}
+};
+// true in every thread of the block that arrives last; the partials that thread 0
+// of each block wrote before are then visible (read past L1 with __ldcg). The
+// sums run over the blocks in a fixed order: the result does not depend on the
+// order of arrival.
+__device__ __forceinline__ bool last_block(unsigned *count)
+{
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last && threadIdx.x == 0) { __threadfence(); *count = 0u; }
+    return last;
+}
+// totals of N partials per block (sums; the last slot a maximum if MAX) into v of thread 0
+template <int N, bool MAX>
+__device__ __forceinline__ void total(const double *part, double (&v)[3])
+{
+    v[0] = v[1] = v[2] = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += RB) {
+        #pragma unroll
+        for (int q = 0; q < N; q++) {
+            const double x = __ldcg(part + N * b + q);
+            v[q] = (MAX && q == N - 1) ? fmax(v[q], x) : v[q] + x;
+        }
+    }
+    __syncthreads();
+    block_reduce<RB>(v, RedSum{}, RedSum{}, RedMax{});
+}
+
+// loop control, as k_cg_start / k_cg_next / k_cg_finish. CAP: the loop is a
+// conditional node of a captured step.
+struct Loop { double rtol, divtol, dt; int maxit, base; };
+template <bool CAP>
+__device__ void loop_go(double *sc, const Loop &L, int it, cudaGraphConditionalHandle h)
+{
+    if (!CAP) return;
+    const double bn = sqrt(sc[0]), rn = sqrt(sc[3]);
+    const bool conv = cg_converged(sc, L.rtol, L.divtol, L.dt);
+    const bool go = !conv && it < L.maxit && isfinite(rn);
+    sc[50] = it; sc[52] = conv ? 1.0 : 0.0;
+    if (it == 0) sc[L.base + ST_RES0] = bn > 0 ? rn / bn : rn;
+    if (!go) {
+        sc[L.base + ST_IT] = it;
+        sc[L.base + ST_TOT] += it;
+        sc[L.base + ST_RES] = bn > 0 ? rn / bn : rn;
+        if (!isfinite(rn)) sc[L.base + ST_NAN] = 1.0;
+        else if (!conv) sc[L.base + ST_NOCONV] += 1.0;
+    }
+    cudaGraphSetConditional(h, go ? 1u : 0u);
+}
+
+// SetRHS (peqn.c:1942-2063) into the compact vector, negated (L = -A), the
+// initial guess (k_extrapolate, k_hist_next) and |b|^2. keep[0] <- p(1,1,1), the
+// gauge of the pressure after the update (phi is zero at the pinned cell).
+__global__ void __launch_bounds__(RB) k_direct_begin(Grid g, State s, PoissonCtx P, double dt, double *hist, int order, double *sc, double *keep)
+{
+    const Rows R(P);
+    const double h = fmin(hist[0], (double)order);
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int row = R.row; row < R.nrow; row += R.step) {
+        const int jc = row % R.ny, kc = row / R.ny, d0 = g.lin(kc + 1, jc + 1, 1), c0 = row * R.nx;
+        for (int i = R.lane; i < R.nx; i += 32) {
+            const int c = c0 + i, d = d0 + i;
+            double val = 0;
+            val += s.ucont.x[d];
+            val -= s.ucont.x[d - 1];
+            val += s.ucont.y[d];
+            val -= s.ucont.y[d - g.mx];
+            val += s.ucont.z[d];
+            val -= s.ucont.z[d - g.mx * g.my];
+            val *= 1.0 / dt;
+            const double b = c == P.pin ? 0.0 : -val;
+            P.b[c] = b;
+            v[0] += b * b;
+            const double xn = P.x[c], xp = P.xprev[c];
+            double x = xn;
+            if (h >= 2.0) x = 3.0 * xn - 3.0 * xp + P.xprev2[c];
+            else if (h >= 1.0) x = 2.0 * xn - xp;
+            P.x[c] = c == P.pin ? 0.0 : x;
+            P.xprev2[c] = xp;
+            P.xprev[c] = xn;
+        }
+    }
+    block_reduce<RB>(v, RedSum{}, RedSum{}, RedMax{});
+    if (threadIdx.x == 0) P.part[blockIdx.x] = v[0];
+    if (last_block(P.count)) {
+        total<1, false>(P.part, v);
+        if (threadIdx.x == 0) {
+            sc[0] = v[0];
+            hist[0] = hist[0] + 1.0;
+            keep[0] = s.p[g.lin(1, 1, 1)];
+        }
+    }
+}
+
+// (L x)_c of k_apply7 at column i of a row; FAC: coefficients from their factors
+template <bool FAC>
+struct Op7 {
+    const PoissonCtx &P;
+    const double *x;
+    int c0, oN, oS, oT, oB;
+    bool hN, hS, hT, hB;
+    double e, nN, nS, tT, tB;         // row factors
+    __device__ __forceinline__ Op7(const PoissonCtx &P_, const double *x_, int row) : P(P_), x(x_)
+    {
+        const int jc = row % P.ny, kc = row / P.ny, nx = P.nx, pl = nx * P.ny;
+        c0 = row * nx;
+        oN = jc < P.ny - 1 ? nx : nx - pl; oS = jc > 0 ? -nx : pl - nx;
+        oT = kc < P.nz - 1 ? pl : pl - pl * P.nz; oB = kc > 0 ? -pl : pl * P.nz - pl;
+        hN = jc < P.ny - 1 || P.pj; hS = jc > 0 || P.pj; hT = kc < P.nz - 1 || P.pk; hB = kc > 0 || P.pk;
+        if (FAC) {
+            const double my = P.op.my[jc], mz = P.op.mz[kc];
+            e = my * mz;
+            nN = hN ? P.op.ky[jc] * mz : 0.0; nS = hS ? P.op.ky[jc > 0 ? jc - 1 : P.ny - 1] * mz : 0.0;
+            tT = hT ? P.op.kz[kc] * my : 0.0; tB = hB ? P.op.kz[kc > 0 ? kc - 1 : P.nz - 1] * my : 0.0;
+        }
+    }
+    __device__ __forceinline__ double at(int i) const
+    {
+        const int nx = P.nx, c = c0 + i, ce = i < nx - 1 ? c + 1 : c + 1 - nx, cw = i > 0 ? c - 1 : c - 1 + nx;
+        const bool hE = i < nx - 1 || P.pi, hW = i > 0 || P.pi;
+        const double xc = x[c];
+        double acc = 0.0;
+        if (FAC) {
+            const double m = P.op.mx[i];
+            if (hE) acc += (P.op.kx[i] * e) * (xc - x[ce]);
+            if (hW) acc += (P.op.kx[i > 0 ? i - 1 : nx - 1] * e) * (xc - x[cw]);
+            if (hN) acc += (m * nN) * (xc - x[c + oN]);
+            if (hS) acc += (m * nS) * (xc - x[c + oS]);
+            if (hT) acc += (m * tT) * (xc - x[c + oT]);
+            if (hB) acc += (m * tB) * (xc - x[c + oB]);
+        } else {
+            if (hE) acc += P.gE1[c] * (xc - x[ce]);
+            if (hW) acc += P.gE1[cw] * (xc - x[cw]);
+            if (hN) acc += P.gN2[c] * (xc - x[c + oN]);
+            if (hS) acc += P.gN2[c + oS] * (xc - x[c + oS]);
+            if (hT) acc += P.gT3[c] * (xc - x[c + oT]);
+            if (hB) acc += P.gT3[c + oB] * (xc - x[c + oB]);
+        }
+        return acc;
+    }
+};
+
+// r = b - L x with |r|^2, sum r and max |r aj| (sc[3..5]), and the loop's start
+template <bool FAC, bool CAP>
+__global__ void __launch_bounds__(RB) k_direct_resid(const __grid_constant__ PoissonCtx P, const double *w, double *sc, Loop L, cudaGraphConditionalHandle h)
+{
+    const Rows R(P);
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int row = R.row; row < R.nrow; row += R.step) {
+        const Op7<FAC> op(P, P.x, row);
+        for (int i = R.lane; i < R.nx; i += 32) {
+            const int c = op.c0 + i;
+            const double r = c == P.pin ? P.b[c] - P.x[c] : P.b[c] - op.at(i);
+            P.r[c] = r;
+            dot_acc(r, r, w ? w[c] : 0.0, v);
+        }
+    }
+    dot_store(v, P.part);
+    if (last_block(P.count)) {
+        total<3, true>(P.part, v);
+        if (threadIdx.x == 0) {
+            sc[3] = v[0]; sc[4] = v[1]; sc[5] = v[2];
+            loop_go<CAP>(sc, L, 0, h);
+        }
+    }
+}
+
+// q = L z (zero at the pin) with (r, z - z_0) and (z - z_0, q) (sc[6], sc[9])
+template <bool FAC>
+__global__ void __launch_bounds__(RB) k_direct_dots(const __grid_constant__ PoissonCtx P, double *sc)
+{
+    const Rows R(P);
+    const double z0 = P.z[0];
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int row = R.row; row < R.nrow; row += R.step) {
+        const Op7<FAC> op(P, P.z, row);
+        for (int i = R.lane; i < R.nx; i += 32) {
+            const int c = op.c0 + i;
+            const double q = c == P.pin ? 0.0 : op.at(i), z = P.z[c] - z0;
+            P.q[c] = q;
+            v[0] += P.r[c] * z;
+            v[1] += z * q;
+        }
+    }
+    block_reduce<RB>(v, RedSum{}, RedSum{}, RedMax{});
+    if (threadIdx.x == 0) { P.part[2 * blockIdx.x] = v[0]; P.part[2 * blockIdx.x + 1] = v[1]; }
+    if (last_block(P.count)) {
+        total<2, false>(P.part, v);
+        if (threadIdx.x == 0) { sc[6] = v[0]; sc[9] = v[1]; }
+    }
+}
+
+// x += alpha (z - z_0), r -= alpha q with the sums of k_direct_resid, and the
+// loop's next pass
+template <bool CAP>
+__global__ void __launch_bounds__(RB) k_direct_update(PoissonCtx P, const double *w, double *sc, Loop L, cudaGraphConditionalHandle h)
+{
+    const double alpha = sc[6] / sc[9], z0 = P.z[0];
+    double v[3] = {0.0, 0.0, 0.0};
+    const int64_t n = P.n, n2 = n >> 1;
+    TG_PAIRS(t, n2) {
+        const double2 xv = v2(P.x)[t], zv = v2(P.z)[t], rv = v2(P.r)[t], qv = v2(P.q)[t];
+        const double2 rn{rv.x - alpha * qv.x, rv.y - alpha * qv.y};
+        v2(P.x)[t] = double2{xv.x + alpha * (zv.x - z0), xv.y + alpha * (zv.y - z0)};
+        v2(P.r)[t] = rn;
+        const double2 wv = w ? v2(w)[t] : double2{0.0, 0.0};
+        dot_acc(rn.x, rn.x, wv.x, v);
+        dot_acc(rn.y, rn.y, wv.y, v);
+    }
+    if (odd_tail(n)) {
+        P.x[n - 1] += alpha * (P.z[n - 1] - z0);
+        const double rn = P.r[n - 1] - alpha * P.q[n - 1];
+        P.r[n - 1] = rn;
+        dot_acc(rn, rn, w ? w[n - 1] : 0.0, v);
+    }
+    dot_store(v, P.part);
+    if (last_block(P.count)) {
+        total<3, true>(P.part, v);
+        if (threadIdx.x == 0) {
+            sc[3] = v[0]; sc[4] = v[1]; sc[5] = v[2];
+            if (CAP) loop_go<CAP>(sc, L, (int)sc[50] + 1, h);
+        }
+    }
+}
+
 inline dim3 cgrid(int nx, int ny, int nz) { return grid3(nx, ny, nz); }
 inline int vblocks(int64_t n) { int64_t b = (n + RB - 1) / RB; return (int)std::min<int64_t>(b, 148 * 8); }
 
@@ -467,9 +713,11 @@ void poisson_setup(tg_ctx *C)
     TG_CUDA(cudaMemsetAsync(C->d_scal + SC_PHIST, 0, sizeof(double), C->stream));   // empty guess history
     P->nblocks = vblocks(n);
     P->part = dallocd(C, 3 * (size_t)P->nblocks);
+    P->count = (unsigned *)dalloc(C, sizeof(unsigned));
     k_gather_g<<<cgrid(P->nx, P->ny, P->nz), block3(), 0, C->stream>>>(g, C->m, *P);
 
     P->fdm = P->ortho ? fdm_create(C, P->gE1, P->gN2, P->gT3, P->nx, P->ny, P->nz, P->pi, P->pj, P->pk) : nullptr;
+    P->op_exact = P->fdm && fdm_factors(P->fdm, &P->op);
     P->mg = P->fdm ? nullptr : mg_create(C, C->cfg.precision == TG_PREC_MIXED, P->gE1, P->gN2, P->gT3,
                                          P->nx, P->ny, P->nz, P->pi, P->pj, P->pk);
     TG_CUDA(cudaGetLastError());
@@ -490,9 +738,61 @@ static void read_scal(tg_ctx *C, int off, int cnt)
     TG_CUDA(cudaStreamSynchronize(C->stream));
 }
 
+static Loop loop_of(tg_ctx *C, double rtol, double divtol, int maxit, int base) { return Loop{rtol, divtol, C->prm.dt, maxit, base}; }
+
+// one pass of the direct solver's iteration; CAP: inside the captured loop
+template <bool CAP>
+static void direct_pass(tg_ctx *C, const Loop &L, cudaGraphConditionalHandle h)
+{
+    PoissonCtx &P = *C->pois;
+    cudaStream_t s = C->stream;
+    double *sc = C->d_scal;
+    fdm_apply(C, P.fdm, P.r, sc + 4, P.z);
+    if (P.op_exact) TG_PROF(C, "pois_dots", k_direct_dots<true><<<P.nblocks, RB, 0, s>>>(P, sc));
+    else TG_PROF(C, "pois_dots", k_direct_dots<false><<<P.nblocks, RB, 0, s>>>(P, sc));
+    TG_PROF(C, "pois_update", (k_direct_update<CAP><<<P.nblocks, RB, 0, s>>>(P, L.divtol > 0 ? P.aj : nullptr, sc, L, h)));
+}
+template <bool CAP>
+static void direct_resid(tg_ctx *C, const Loop &L, cudaGraphConditionalHandle h)
+{
+    PoissonCtx &P = *C->pois;
+    const double *w = L.divtol > 0 ? P.aj : nullptr;
+    if (P.op_exact) TG_PROF(C, "pois_resid", (k_direct_resid<true, CAP><<<P.nblocks, RB, 0, C->stream>>>(P, w, C->d_scal, L, h)));
+    else TG_PROF(C, "pois_resid", (k_direct_resid<false, CAP><<<P.nblocks, RB, 0, C->stream>>>(P, w, C->d_scal, L, h)));
+}
+
+// direct solve of L x = b from the current P.x (P.b and |b|^2 in sc[0] set by the caller)
+static int direct_solve(tg_ctx *C, tg_stats *st, double rtol, double divtol, int maxit)
+{
+    const Loop L = loop_of(C, rtol, divtol, maxit, 0);
+    double *hs = C->h_scal;
+    direct_resid<false>(C, L, cudaGraphConditionalHandle{});
+    read_scal(C, 0, 6);
+    const double bn = std::sqrt(hs[0]);
+    double rn = std::sqrt(hs[3]);
+    if (st) st->poisson_initial_residual = bn > 0 ? rn / bn : rn;
+    auto converged = [&]() { return bn == 0.0 || rn / bn <= rtol || (divtol > 0 && hs[5] * L.dt <= divtol); };
+    int it = 0;
+    while (!converged() && it < maxit && std::isfinite(rn)) {
+        direct_pass<false>(C, L, cudaGraphConditionalHandle{});
+        read_scal(C, 3, 3);
+        rn = std::sqrt(hs[3]);
+        it++;
+    }
+    TG_CUDA(cudaGetLastError());
+    if (st) {
+        st->poisson_iterations = it;
+        st->poisson_total_iterations += it;
+        st->poisson_final_residual = bn > 0 ? rn / bn : rn;
+    }
+    if (!std::isfinite(rn)) return 2;
+    return converged() ? 0 : 1;
+}
+
 // Krylov solve of L x = b from the current P.x (P.b set by the caller):
-// preconditioned CG on orthogonal grids, BiCGStab otherwise. Stops at the
-// relative residual rtol or, when divtol > 0, at dt * max|r aj| <= divtol.
+// preconditioned CG on orthogonal grids (the iteration of direct_solve on a mesh
+// of planes), BiCGStab otherwise. Stops at the relative residual rtol or, when
+// divtol > 0, at dt * max|r aj| <= divtol.
 static int krylov_solve(tg_ctx *C, tg_stats *st, double rtol, double divtol, int maxit)
 {
     PoissonCtx &P = *C->pois;
@@ -503,6 +803,7 @@ static int krylov_solve(tg_ctx *C, tg_stats *st, double rtol, double divtol, int
     double *hs = C->h_scal;
 
     dot3v(C, P.b, P.b, nullptr, sc + 0);
+    if (P.fdm) return direct_solve(C, st, rtol, divtol, maxit);
     apply_op(C, P.x, P.r);
     k_resid<<<vblocks(n), RB, 0, s>>>(n, P.b, P.r);   // r = b - L x
     dot3v(C, P.r, P.r, divtol > 0 ? P.aj : nullptr, sc + 3);
@@ -613,6 +914,21 @@ static int krylov_solve(tg_ctx *C, tg_stats *st, double rtol, double divtol, int
     return ok ? 0 : 1;
 }
 
+static void direct_begin(tg_ctx *C)
+{
+    PoissonCtx &P = *C->pois;
+    TG_PROF(C, "pois_begin", k_direct_begin<<<P.nblocks, RB, 0, C->stream>>>(C->g, C->s, P, C->prm.dt, C->d_scal + SC_PHIST, guess_order(C), C->d_scal, C->d_scal + SC_PREF));
+}
+
+// phi into the DMDA; on an axis-aligned mesh the pressure update that follows
+// reads the compact solution itself
+static void phi_to_dmda(tg_ctx *C)
+{
+    PoissonCtx &P = *C->pois;
+    if (C->axis_aligned) return;
+    TG_PROF(C, "pois_phi_to_dmda", k_phi_to_dmda<<<cgrid(P.nx, P.ny, P.nz), block3(), 0, C->stream>>>(C->g, C->s, P));
+}
+
 int poisson_solve(tg_ctx *C, tg_stats *st)
 {
     PoissonCtx &P = *C->pois;
@@ -621,12 +937,18 @@ int poisson_solve(tg_ctx *C, tg_stats *st)
     const double rtol = C->cfg.poisson_rtol > 0 ? C->cfg.poisson_rtol : 1e-14;
     const int maxit = C->cfg.poisson_maxit > 0 ? C->cfg.poisson_maxit : 500;
     const dim3 cg3 = cgrid(P.nx, P.ny, P.nz);
+    if (P.fdm) {
+        direct_begin(C);
+        const int rc = direct_solve(C, st, rtol, C->cfg.poisson_div_tol, maxit);
+        phi_to_dmda(C);
+        return rc;
+    }
     TG_PROF(C, "pois_set_rhs", k_set_rhs<<<cg3, block3(), 0, s>>>(g, C->s, P, C->prm.dt));
     k_extrapolate<<<vblocks(P.n), RB, 0, s>>>(P.n, P.x, P.xprev, P.xprev2, C->d_scal + SC_PHIST, guess_order(C));
     k_hist_next<<<1, 1, 0, s>>>(C->d_scal + SC_PHIST);
     k_zero_at<<<1, 1, 0, s>>>(P.x, P.pin);            // warm start from the previous solutions
     int rc = krylov_solve(C, st, rtol, C->cfg.poisson_div_tol, maxit);
-    TG_PROF(C, "pois_phi_to_dmda", k_phi_to_dmda<<<cg3, block3(), 0, s>>>(g, C->s, P));
+    phi_to_dmda(C);
     TG_CUDA(cudaGetLastError());
     return rc;
 }
@@ -704,7 +1026,8 @@ __global__ void k_bicg_mark_restart(double *sc, double rtol, double divtol, doub
 // update (p = z on the first pass), the BiCGStab body is krylov_solve's with
 // its restarts and its true-residual check as conditional IF nodes; both perform the same
 // arithmetic in the same order. Statistics go to the ST_* slots from base.
-static void krylov_capture(tg_ctx *C, double rtol, double divtol, int maxit, int base)
+// have_bb: |b|^2 is in sc[0] already (direct solver only).
+static void krylov_capture(tg_ctx *C, double rtol, double divtol, int maxit, int base, bool have_bb = false)
 {
     PoissonCtx &P = *C->pois;
     const int64_t n = P.n;
@@ -712,6 +1035,14 @@ static void krylov_capture(tg_ctx *C, double rtol, double divtol, int maxit, int
     const double dt = C->prm.dt;
     double *sc = C->d_scal;
     const int vb = vblocks(n);
+    if (P.fdm) {
+        if (!have_bb) dot3v(C, P.b, P.b, nullptr, sc + 0);
+        const Loop L = loop_of(C, rtol, divtol, maxit, base);
+        cudaGraphConditionalHandle h = capture_handle(C);
+        direct_resid<true>(C, L, h);
+        capture_conditional(C, h, cudaGraphCondTypeWhile, C->aux[0], [&]() { direct_pass<true>(C, L, h); });
+        return;
+    }
     dot3v(C, P.b, P.b, nullptr, sc + 0);
     apply_op(C, P.x, P.r);
     k_resid<<<vb, RB, 0, s>>>(n, P.b, P.r);
@@ -798,12 +1129,16 @@ void poisson_solve_capture(tg_ctx *C)
     const double rtol = C->cfg.poisson_rtol > 0 ? C->cfg.poisson_rtol : 1e-14;
     const int maxit = C->cfg.poisson_maxit > 0 ? C->cfg.poisson_maxit : 500;
     const dim3 cg3 = cgrid(P.nx, P.ny, P.nz);
-    k_set_rhs<<<cg3, block3(), 0, s>>>(g, C->s, P, C->prm.dt);
-    k_extrapolate<<<vblocks(P.n), RB, 0, s>>>(P.n, P.x, P.xprev, P.xprev2, C->d_scal + SC_PHIST, guess_order(C));
-    k_hist_next<<<1, 1, 0, s>>>(C->d_scal + SC_PHIST);
-    k_zero_at<<<1, 1, 0, s>>>(P.x, P.pin);
-    krylov_capture(C, rtol, C->cfg.poisson_div_tol, maxit, SC_G);
-    k_phi_to_dmda<<<cg3, block3(), 0, s>>>(g, C->s, P);
+    if (P.fdm) {
+        direct_begin(C);
+    } else {
+        k_set_rhs<<<cg3, block3(), 0, s>>>(g, C->s, P, C->prm.dt);
+        k_extrapolate<<<vblocks(P.n), RB, 0, s>>>(P.n, P.x, P.xprev, P.xprev2, C->d_scal + SC_PHIST, guess_order(C));
+        k_hist_next<<<1, 1, 0, s>>>(C->d_scal + SC_PHIST);
+        k_zero_at<<<1, 1, 0, s>>>(P.x, P.pin);
+    }
+    krylov_capture(C, rtol, C->cfg.poisson_div_tol, maxit, SC_G, P.fdm != nullptr);
+    phi_to_dmda(C);
     TG_CUDA(cudaGetLastError());
 }
 
@@ -858,6 +1193,7 @@ void adjoint_guess(tg_ctx *C, double *lam, double *lp, double *lp2, double *hist
 }
 
 // compact Poisson solution vectors (the next solve extrapolates x, xprev, xprev2): snapshots
+bool poisson_direct(const tg_ctx *C) { return C->pois->fdm != nullptr; }
 double *poisson_x(tg_ctx *C) { return C->pois->x; }
 double *poisson_xprev(tg_ctx *C) { return C->pois->xprev; }
 double *poisson_xprev2(tg_ctx *C) { return C->pois->xprev2; }

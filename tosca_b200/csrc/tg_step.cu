@@ -1540,23 +1540,31 @@ static int solve_u_impl(tg_ctx *C, bool cart_tail, tg_stats *st = nullptr)
 void solve_u(tg_ctx *C) { solve_u_impl(C, true); }
 
 // SolvePEqn (peqn.c:3777-3971) after the Poisson solve: phi ghosts, pressure
-// update and ghosts, projection
-void pressure_update_and_project(tg_ctx *C)
+// update and ghosts, projection. gauge: on a mesh of planes the update takes
+// SyncPressureAcrossDomains with it (phi is zero at the cell of the gauge), true
+// is returned then.
+static bool pressure_update_and_project(tg_ctx *C, bool gauge)
 {
     const Grid g = C->g;
+    if (C->axis_aligned) {
+        double *ref = C->d_scal + SC_PREF;
+        if (gauge && !poisson_direct(C)) k_copy1<<<1, 1, 0, C->stream>>>(C->s.p + g.lin(1, 1, 1), ref);
+        pressure_project_tensor(C, poisson_x(C), gauge ? ref : nullptr);
+        return gauge;
+    }
     update_scalar_ghosts(C, C->s.phi);
     TG_PROF(C, "update_pressure", k_update_pressure<<<gi(g), block3(), 0, C->stream>>>(g, C->s));
     update_scalar_ghosts(C, C->s.p);
-    if (C->axis_aligned) { project_tensor(C); return; }
     refresh_met32(C);
     if (C->pol.proj32) TG_PROF(C, "project", k_project<float><<<gf(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm.dt));
     else TG_PROF(C, "project", k_project<double><<<gf(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm.dt));
+    return false;
 }
 
 int solve_p(tg_ctx *C, tg_stats *st)
 {
     int rc = poisson_solve(C, st);
-    pressure_update_and_project(C);
+    pressure_update_and_project(C, false);
     return rc;
 }
 
@@ -1565,6 +1573,12 @@ void reduce_max_abs_div(tg_ctx *C, double *d_out)
     const int nb = C->red_blocks;
     TG_PROF(C, "div_max", k_div_partial<<<nb, 256, 0, C->stream>>>(C->g, C->m, C->s, C->d_red));
     k_max_final<<<1, 256, 0, C->stream>>>(C->d_red, nb, d_out);
+}
+
+static void contra_div_final(tg_ctx *C)
+{
+    contra_div_tensor(C);
+    k_max_final<<<1, 256, 0, C->stream>>>(C->d_red, C->red_blocks, C->d_scal + 16);
 }
 
 double continuity_error(tg_ctx *C)
@@ -1579,8 +1593,8 @@ void sync_pressure(tg_ctx *C)
 {
     const Grid g = C->g;
     const int64_t G = g.size();
-    k_copy1<<<1, 1, 0, C->stream>>>(C->s.p + g.lin(1, 1, 1), C->d_scal + 17);
-    TG_PROF(C, "gauge", k_gauge<<<nblk(G), 256, 0, C->stream>>>(G, C->s.p, C->d_scal + 17));
+    k_copy1<<<1, 1, 0, C->stream>>>(C->s.p + g.lin(1, 1, 1), C->d_scal + SC_PREF);
+    TG_PROF(C, "gauge", k_gauge<<<nblk(G), 256, 0, C->stream>>>(G, C->s.p, C->d_scal + SC_PREF));
 }
 
 void init_from_cartesian(tg_ctx *C)
@@ -1631,15 +1645,18 @@ static int step_body(tg_ctx *C, tg_stats *st, bool capture)
     else rc = poisson_solve(C, st);
     if (urc == 2) rc = 2;
     else if (rc != 2) rc |= urc;
-    pressure_update_and_project(C);
-    contra_to_cart(C);
+    const bool gauged = pressure_update_and_project(C, true);
+    // final Ucat; on a mesh of planes with the divergence maximum, whose faces it
+    // reads anyway (nothing below changes Ucont before the boundary conditions)
+    if (C->axis_aligned) contra_div_final(C);
+    else contra_to_cart(C);
     if (C->prm.teqn) {                  // main.c:194-205
         update_wall_models_t(C);
         const int trc = solve_t(C);
         if (trc == 2) rc = 2;
         else if (rc != 2) rc |= trc;
     }
-    reduce_max_abs_div(C, C->d_scal + 16);
+    if (!C->axis_aligned) reduce_max_abs_div(C, C->d_scal + 16);
     if (C->cfg.ddt_scheme == TG_DDT_CN) {   // main.c:214-272: Rhs_o for the next step
         TG_CUDA(cudaMemsetAsync(C->s.rhs_o.x, 0, 3 * sizeof(double) * G, C->stream));
         form_u(C, C->s.rhs_o, 1.0);
@@ -1647,7 +1664,7 @@ static int step_body(tg_ctx *C, tg_stats *st, bool capture)
     if (C->prm.teqn) update_temperature_bcs(C);   // main.c:274-278
     update_cartesian_bcs(C);
     update_contravariant_bcs(C);
-    sync_pressure(C);
+    if (!gauged) sync_pressure(C);
     k_incr_scalar<<<1, 1, 0, C->stream>>>(C->d_scal + SC_IT);
     return rc;
 }

@@ -780,18 +780,70 @@ __global__ void __launch_bounds__(256, 8) k_rhs_tensor(Grid g, Tensor t, State s
     }
 }
 
-// -------------------------------------------------------- ProjectVelocity
-// k_project (peqn.c:2495-2905)
-__global__ void k_project_tensor(Grid g, Tensor t, State s, double dt)
+// ------------------------------------ pressure update and ProjectVelocity
+// From the compact Poisson solution x in one pass: phi and p with their ghosts
+// (phiToPhi, UpdatePressure, UpdatePhiBCs, UpdatePressureBCs; peqn.c:1579-1636,
+// 2909-2962, boundary.c:3051-3255), the gauge p -= *ref if ref is given
+// (SyncPressureAcrossDomains, overset.c:263-315), and the projection of the faces
+// (peqn.c:2495-2905). A cell writes its own value to the ghost points that copy
+// it, so no point is read after another thread wrote it. 80 bytes per cell; the
+// separate passes (two conversions, six ghost launches, update, projection,
+// gauge) took 0.30 ms at 256 x 256 x 128.
+__global__ void __launch_bounds__(256) k_pressure_project(Grid g, Tensor t, State s, const double *x, const double *ref, double dt)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
-    const int f = g.lin(k, j, i);
-    // neighbours of faces 0 .. m-2 lie inside the DMDA
-    const double pc = s.phi[f], dx = t.dx[k], dy = t.dy[i], dz = t.dz[j];
-    if (j > 0 && k > 0 && ((i > 0 && i < g.mx - 2) || g.pi)) s.ucont.x[f] -= ((s.phi[f + 1] - pc) * (dx * dz * t.rdyf[i])) * dt;
-    if (i > 0 && k > 0 && ((j > 0 && j < g.my - 2) || g.pj)) s.ucont.y[f] -= ((s.phi[f + g.mx] - pc) * (dx * dy * t.rdzf[j])) * dt;
-    if (i > 0 && j > 0 && ((k > 0 && k < g.mz - 2) || g.pk)) s.ucont.z[f] -= ((s.phi[f + g.mx * g.my] - pc) * (dy * dz * t.rdxf[k])) * dt;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
+    const int mx = g.mx, my = g.my, mz = g.mz;
+    if (i > mx - 2 || j > my - 2 || k > mz - 2) return;
+    const int nx = mx - 2, ny = my - 2, nz = mz - 2, pl = mx * my, cpl = nx * ny;
+    const int c = g.lin(k, j, i), cc = (k - 1) * cpl + (j - 1) * nx + i - 1;
+    const double phi = x[cc], dx = t.dx[k], dy = t.dy[i], dz = t.dz[j];
+    double p = s.p[c] + phi;
+    if (ref) p -= ref[0];
+    const double fi = dx * dz, fj = dx * dy, fk = dy * dz;
+    if (i < mx - 2 || g.pi) s.ucont.x[c] -= ((x[i < mx - 2 ? cc + 1 : cc + 1 - nx] - phi) * (fi * t.rdyf[i])) * dt;
+    if (j < my - 2 || g.pj) s.ucont.y[c] -= ((x[j < my - 2 ? cc + nx : cc + nx - cpl] - phi) * (fj * t.rdzf[j])) * dt;
+    if (k < mz - 2 || g.pk) s.ucont.z[c] -= ((x[k < mz - 2 ? cc + cpl : cc + cpl - cpl * nz] - phi) * (fk * t.rdxf[k])) * dt;
+    // face 0 of a periodic direction
+    if (i == 1 && g.pi) s.ucont.x[c - 1] -= ((phi - x[cc + nx - 1]) * (fi * t.rdyf[0])) * dt;
+    if (j == 1 && g.pj) s.ucont.y[c - mx] -= ((phi - x[cc + cpl - nx]) * (fj * t.rdzf[0])) * dt;
+    if (k == 1 && g.pk) s.ucont.z[c - pl] -= ((phi - x[cc + cpl * nz - cpl]) * (fk * t.rdxf[0])) * dt;
+    // the indices that copy this cell's: its own, and the ghost next to it or
+    // (periodic) opposite
+    auto image = [](int l, int m, int per) { return l == 1 ? (per ? m - 1 : 0) : l == m - 2 ? (per ? 0 : m - 1) : l; };
+    const int gi_ = image(i, mx, g.pi), gj_ = image(j, my, g.pj), gk_ = image(k, mz, g.pk);
+    s.phi[c] = phi;
+    s.p[c] = p;
+    if (gi_ == i && gj_ == j && gk_ == k) return;
+    for (int b = 1; b < 8; b++) {
+        if (((b & 1) && gi_ == i) || ((b & 2) && gj_ == j) || ((b & 4) && gk_ == k)) continue;
+        const int q = g.lin((b & 4) ? gk_ : k, (b & 2) ? gj_ : j, (b & 1) ? gi_ : i);
+        s.phi[q] = phi;
+        s.p[q] = p;
+    }
+}
+
+// contravariantToCartesian of the projected Ucont with the divergence maximum of
+// ContinuityErrorsOptimized (peqn.c:4114-4181), block partials: both read the six
+// faces of a cell
+__global__ void __launch_bounds__(256) k_contra_div_tensor(Grid g, Tensor t, State s, double *part)
+{
+    const int lane = threadIdx.x & 31, nJ = g.my - 2, nrow = nJ * (g.mz - 2), pl = g.mx * g.my;
+    double v[1] = {0.0};
+    for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrow; row += (gridDim.x * blockDim.x) >> 5) {
+        const int j = row % nJ + 1, k = row / nJ + 1;
+        const double rx = t.rdx[k], rz = t.rdz[j], rxz = rx * rz;
+        for (int i = 1 + lane; i <= g.mx - 2; i += 32) {
+            const int c = g.lin(k, j, i);
+            const double ry = t.rdy[i];
+            const double x1 = s.ucont.x[c], x0 = s.ucont.x[c - 1], y1 = s.ucont.y[c], y0 = s.ucont.y[c - g.mx], z1 = s.ucont.z[c], z0 = s.ucont.z[c - pl];
+            s.ucat.x[c] = (0.5 * (z0 + z1)) * (ry * rz);
+            s.ucat.y[c] = (0.5 * (x0 + x1)) * rxz;
+            s.ucat.z[c] = (0.5 * (y0 + y1)) * (rx * ry);
+            v[0] = nanmax(v[0], fabs((x1 - x0 + y1 - y0 + z1 - z0) * (rxz * ry)));
+        }
+    }
+    block_reduce<256>(v, RedNanMax{});
+    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
 }
 
 inline dim3 gi(const Grid &g) { return grid3(g.mx - 2, g.my - 2, g.mz - 2); }
@@ -941,10 +993,13 @@ void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab
     else if (kind == 1) TG_PROF(C, "formu_rhs_faces", k_rhs_tensor<1><<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
     else TG_PROF(C, "formu_rhs_faces", k_rhs_tensor<2><<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
 }
-void project_tensor(tg_ctx *C)
+void pressure_project_tensor(tg_ctx *C, const double *x, const double *ref)
 {
-    const Grid g = C->g;
-    TG_PROF(C, "project", k_project_tensor<<<grid3(g.mx - 1, g.my - 1, g.mz - 1), block3(), 0, C->stream>>>(g, C->ts, C->s, C->prm.dt));
+    TG_PROF(C, "pressure_project", k_pressure_project<<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->ts, C->s, x, ref, C->prm.dt));
+}
+void contra_div_tensor(tg_ctx *C)
+{
+    TG_PROF(C, "contra_div_final", k_contra_div_tensor<<<C->red_blocks, 256, 0, C->stream>>>(C->g, C->ts, C->s, C->d_red));
 }
 
 }  // namespace tg
