@@ -1497,6 +1497,7 @@ static int solve_u_impl(tg_ctx *C, bool cart_tail, tg_stats *st = nullptr)
     // stages read Ucont alone; a taped step records the Ucat of every stage
     const bool lean = !cart_tail && !C->taping && C->axis_aligned && C->prm.div_scheme == TG_DIV_CENTRAL &&
                       (C->cfg.ddt_scheme == TG_DDT_FE || C->cfg.ddt_scheme == TG_DDT_RK4);
+    if (lean) reset_no_penetration(C);
     if (C->cfg.ddt_scheme == TG_DDT_CN) {
         // UeqnSNES, ueqn_solvers.c:1087-1199
         rc = solve_u_cn(C, st);

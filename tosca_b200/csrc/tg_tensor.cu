@@ -366,19 +366,21 @@ __global__ void __launch_bounds__(PX * PY, 2) k_fp_tensor(Grid g, Tensor t, Stat
 // again after the projection.
 //
 // The resets are index rules here. Periodic directions are read through the
-// wrap 0 -> m-2, m-1 -> 1 of cells and faces, wall faces read as zero, and the
-// ghost cells of non-periodic directions come from Ucat, where they keep the
-// values of the previous step's UpdateCartesianBCs as in the reference.
+// wrap 0 -> m-2, m-1 -> 1 of cells and faces; wall faces are zero, set once
+// before the first stage and again by each update (k_rhs_tensor); and the ghost
+// cells of non-periodic directions come from Ucat, where they keep the values
+// of the previous step's UpdateCartesianBCs as in the reference.
 //
 // A block marches its 32 x 8 columns through a chunk of planes. Ucont and nut of
 // plane k+3 are copied asynchronously into a ring of four planes while plane k
-// is worked on; each plane is converted once into a ring of three planes of
-// Ucat. At 256 x 256 x 128 a launch takes 302 us, as long as the kernels it
-// replaces (conversion 90, budgets 220 and 27 for boundary cells) without their
-// 10 launches of boundary kernels per stage, which is what bounds small grids
-// (Taylor-Green 32^3 0.255 -> 0.167 ms a step). It is bound by the latency of its
-// FP64 and shared-memory chains at two blocks per SM (44 % of issue slots, DRAM
-// at 20 %).
+// is worked on; each plane is converted once into a ring of four planes of
+// Ucat. At 256 x 256 x 128 a launch takes 235 us (302 with two barriers per plane
+// and ring slots from a modulus) against 90 + 220 + 27 for the conversion, the
+// tile kernel and the boundary cells that it replaces, without their 10 launches
+// of boundary kernels per stage, which is what bounds small grids (Taylor-Green
+// 32^3 0.255 -> 0.167 ms a step). 462 instructions per cell; it is bound by the
+// latency of its FP64 and shared-memory chains at two blocks per SM (43 % of
+// issue slots, DRAM at 25 %).
 __device__ __forceinline__ bool wall_patch(const Params &p, int q)
 {
     const int t = p.bc[q];
@@ -500,11 +502,11 @@ __device__ void fp_edge_cell(const Grid &g, const Tensor &t, const State &s, con
     if (on && q == 0) st3(fp, g.lin(k, j, i), R3<double>{F[2], F[0], F[1]});
 }
 
-// shared memory of k_stage_fp, in doubles: per plane of the ring X (35 x 10),
+// shared memory of k_stage_fp, in doubles: per plane of the Ucont ring X (35 x 10),
 // Y (34 x 11), Z and nut (34 x 10); per plane of the Ucat ring three of 34 x 10
 constexpr int SXW = PX + 3, SXN = SXW * PTY, SYN = PTX * (PTY + 1), SZN = PTX * PTY;
-constexpr int SPL = SXN + SYN + SZN + SZN, SRING = 4, SUN = 3 * SZN;
-constexpr int STAGE_SMEM = (SRING * SPL + 3 * SUN + PTX + PTY + 2) * 8;
+constexpr int OY = SXN, OZ = SXN + SYN, ON = OZ + SZN, SPL = ON + SZN, SUN = 3 * SZN;
+constexpr int STAGE_SMEM = (4 * SPL + 4 * SUN + PTX + PTY + 2) * 8;
 
 template <bool LES>
 __global__ void __launch_bounds__(PX * PY, 2) k_stage_fp(const __grid_constant__ Grid g, const __grid_constant__ Tensor t, const __grid_constant__ State s,
@@ -512,92 +514,86 @@ __global__ void __launch_bounds__(PX * PY, 2) k_stage_fp(const __grid_constant__
 {
     if ((int)blockIdx.x < nedge) { fp_edge_cell(g, t, s, fp, p, blockIdx.x * (PX * PY) + threadIdx.y * PX + threadIdx.x); return; }
     extern __shared__ double sh[];
-    double *const raw = sh, *const uc = sh + SRING * SPL, *const sry = uc + 3 * SUN, *const srz = sry + PTX;
+    double *const raw = sh, *const uc = sh + 4 * SPL, *const sry = uc + 4 * SUN, *const srz = sry + PTX;
     const int mx = g.mx, my = g.my, mz = g.mz, pl = mx * my;
     const int blk = blockIdx.x - nedge, br = blk / nbi;
     const int i0 = 1 + (blk % nbi) * PX, j0 = 1 + (br % nbj) * PY, k0 = 1 + (br / nbj) * kc, k1 = min(k0 + kc - 1, mz - 2);
     const int tid = threadIdx.y * PX + threadIdx.x;
-    // ---- what this thread copies of every plane: in-plane offsets of up to two
-    // elements per array (-1: none, -2: a wall face, zero)
-    int dX[2], dY[2], dZ[2], dN[2];
+    // ---- what this thread copies of every plane: in-plane offsets of elements
+    // tid and tid + 256 of each array. Elements outside the domain are never
+    // used; they read the plane's first element.
+    int dX[2], dY[2], dN[2];
+    bool ghost[2];                 // a ghost of a non-periodic direction (or outside)
     auto inr = [](int l, int a, int b) { return l >= a && l <= b; };
     #pragma unroll
     for (int q = 0; q < 2; q++) {
         const int e = tid + q * (PX * PY);
-        dX[q] = dY[q] = dZ[q] = dN[q] = -1;
-        if (e < SXN) {
+        {
             const int j = wrap1(j0 - 1 + e / SXW, my, g.pj), f = wrap1(i0 - 2 + e % SXW, mx, g.pi);
-            if (inr(j, 1, my - 2) && inr(f, 0, mx - 2))
-                dX[q] = ((f == 0 && wall_patch(p, TG_ILEFT)) || (f == mx - 2 && wall_patch(p, TG_IRIGHT))) ? -2 : j * mx + f;
+            dX[q] = inr(j, 0, my - 1) && inr(f, 0, mx - 1) ? j * mx + f : 0;
         }
-        if (e < SYN) {
+        {
             const int f = wrap1(j0 - 2 + e / PTX, my, g.pj), i = wrap1(i0 - 1 + e % PTX, mx, g.pi);
-            if (inr(f, 0, my - 2) && inr(i, 1, mx - 2))
-                dY[q] = ((f == 0 && wall_patch(p, TG_JLEFT)) || (f == my - 2 && wall_patch(p, TG_JRIGHT))) ? -2 : f * mx + i;
+            dY[q] = inr(f, 0, my - 1) && inr(i, 0, mx - 1) ? f * mx + i : 0;
         }
-        if (e < SZN) {
-            const int j = wrap1(j0 - 1 + e / PTX, my, g.pj), i = wrap1(i0 - 1 + e % PTX, mx, g.pi);
-            if (inr(j, 0, my - 1) && inr(i, 0, mx - 1)) {
-                dN[q] = j * mx + i;
-                if (inr(j, 1, my - 2) && inr(i, 1, mx - 2)) dZ[q] = dN[q];
-            }
-        }
+        const int j = wrap1(j0 - 1 + e / PTX, my, g.pj), i = wrap1(i0 - 1 + e % PTX, mx, g.pi);
+        dN[q] = inr(j, 0, my - 1) && inr(i, 0, mx - 1) ? j * mx + i : 0;
+        ghost[q] = !(inr(j, 1, my - 2) && inr(i, 1, mx - 2));
     }
     if (tid < PTX) { const int i = wrap1(i0 - 1 + tid, mx, g.pi); sry[tid] = i <= mx - 1 ? t.rdy[i] : 0.0; }
     if (tid < PTY) { const int j = wrap1(j0 - 1 + tid, my, g.pj); srz[tid] = j <= my - 1 ? t.rdz[j] : 0.0; }
-    // plane q of Ucont and nut into its slot of the ring
-    auto load = [&](int q) {
+    // plane q of Ucont and nut into a slot of the ring
+    auto load = [&](int q, double *d) {
         const int w = wrap1(q, mz, g.pk);
         if (w < 0 || w > mz - 1) return;
-        double *d = raw + (q & 3) * SPL;
-        const int64_t o = (int64_t)w * pl;
-        const bool zwall = (w == 0 && wall_patch(p, TG_KLEFT)) || (w == mz - 2 && wall_patch(p, TG_KRIGHT));
-        #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int e = tid + u * (PX * PY);
-            if (dX[u] >= 0) cp_async8(d + e, s.ucont.x + o + dX[u]);
-            else if (dX[u] == -2) d[e] = 0.0;
-            if (dY[u] >= 0) cp_async8(d + SXN + e, s.ucont.y + o + dY[u]);
-            else if (dY[u] == -2) d[SXN + e] = 0.0;
-            if (dZ[u] >= 0) {
-                if (zwall) d[SXN + SYN + e] = 0.0;
-                else cp_async8(d + SXN + SYN + e, s.ucont.z + o + dZ[u]);
+        const int o = w * pl;
+        d += tid;
+        cp_async8(d, s.ucont.x + o + dX[0]);
+        cp_async8(d + OY, s.ucont.y + o + dY[0]);
+        cp_async8(d + OZ, s.ucont.z + o + dN[0]);
+        if (LES) cp_async8(d + ON, s.nut + o + dN[0]);
+        d += PX * PY;
+        if (tid < SYN - PX * PY) {
+            cp_async8(d + OY, s.ucont.y + o + dY[1]);
+            if (tid < SXN - PX * PY) cp_async8(d, s.ucont.x + o + dX[1]);
+            if (tid < SZN - PX * PY) {
+                cp_async8(d + OZ, s.ucont.z + o + dN[1]);
+                if (LES) cp_async8(d + ON, s.nut + o + dN[1]);
             }
-            if (LES && dN[u] >= 0) cp_async8(d + SXN + SYN + SZN + e, s.nut + o + dN[u]);
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
-    // Ucat of plane q from its Ucont (and the k faces of the plane below)
-    auto convert = [&](int q) {
+    // Ucat of plane q from its Ucont d and the k faces of the plane below, zb
+    auto convert = [&](int q, double rx, const double *d, const double *zb, double *u) {
         const int w = wrap1(q, mz, g.pk);
         if (w > mz - 1) return;
         const bool zghost = w < 1 || w > mz - 2;
-        const double *d = raw + (q & 3) * SPL, *zb = raw + ((q - 1) & 3) * SPL + SXN + SYN;
-        double *u = uc + ((q + 3) % 3) * SUN;
-        const double rx = t.rdx[w];
         #pragma unroll
         for (int e2 = 0; e2 < 2; e2++) {
             const int e = tid + e2 * (PX * PY);
-            if (dN[e2] < 0) continue;
-            if (zghost || dZ[e2] < 0) {                      // ghost cell of a non-periodic direction
-                const int64_t o = (int64_t)w * pl + dN[e2];
+            if (e2 && tid >= SZN - PX * PY) break;
+            if (zghost || ghost[e2]) {
+                const int o = w * pl + dN[e2];
                 u[e] = s.ucat.x[o]; u[SZN + e] = s.ucat.y[o]; u[2 * SZN + e] = s.ucat.z[o];
                 continue;
             }
             const int r = e / PTX, c = e - r * PTX;
             const double ry = sry[c], rz = srz[r];
-            const double *x = d + r * SXW + c, *y = d + SXN + e;
-            u[e] = (0.5 * (zb[e] + d[SXN + SYN + e])) * (ry * rz);
+            const double *x = d + r * SXW + c, *y = d + OY + e;
+            u[e] = (0.5 * (zb[OZ + e] + d[OZ + e])) * (ry * rz);
             u[SZN + e] = (0.5 * (x[0] + x[1])) * (rx * rz);
             u[2 * SZN + e] = (0.5 * (y[0] + y[PTX])) * (rx * ry);
         }
     };
-    load(k0 - 2); load(k0 - 1); load(k0); load(k0 + 1);
+    auto rdx = [&](int q) { return t.rdx[min(wrap1(q, mz, g.pk), mz - 1)]; };
+    // planes k0-2 .. k0+1 in slots 0 .. 3; Ucat of k0-1, k0 and k0+1 in slots 1, 2, 3
+    #pragma unroll
+    for (int q = 0; q < 4; q++) load(k0 - 2 + q, raw + q * SPL);
     commit();
     cp_async_wait_all();
     __syncthreads();
-    convert(k0 - 1);
-    convert(k0);
+    #pragma unroll
+    for (int q = 1; q < 4; q++) convert(k0 - 2 + q, rdx(k0 - 2 + q), raw + q * SPL, raw + (q - 1) * SPL, uc + q * SUN);
     __syncthreads();
     const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
     const bool on = i <= mx - 2 && j <= my - 2;
@@ -608,6 +604,9 @@ __global__ void __launch_bounds__(PX * PY, 2) k_stage_fp(const __grid_constant__
     const bool offW = LES && i == 1 && p.bc[TG_ILEFT] == TG_BC_SLIP, offE = LES && i == mx - 2 && p.bc[TG_IRIGHT] == TG_BC_SLIP;
     const bool offS = LES && j == 1 && p.bc[TG_JLEFT] == TG_BC_SLIP, offN = LES && j == my - 2 && p.bc[TG_JRIGHT] == TG_BC_SLIP;
     const bool wmS = LES && j == 1 && p.bc[TG_JLEFT] == TG_BC_WALL_SHUMANN, wmN = LES && j == my - 2 && p.bc[TG_JRIGHT] == TG_BC_WALL_SHUMANN;
+    // edge_cell by parts: along this column, and at the first and last plane
+    const bool bi = i == 1 || i == mx - 2, bj = j == 1 || j == my - 2;
+    const bool edge = bi && bj && !(g.pi && g.pj), kedge = edge || (bi && !(g.pi && g.pk)) || (bj && !(g.pj && g.pk));
     const int a = (threadIdx.y + 1) * PTX + threadIdx.x + 1, ax = (threadIdx.y + 1) * SXW + threadIdx.x + 1;
     auto kface = [&](const double *lo, const double *hi, double n, double z, double K1) {
         const double x0 = lo[a], x1 = hi[a], y0 = lo[SZN + a], y1 = hi[SZN + a], z0 = lo[2 * SZN + a], z1 = hi[2 * SZN + a];
@@ -621,64 +620,73 @@ __global__ void __launch_bounds__(PX * PY, 2) k_stage_fp(const __grid_constant__
     };
     R3<double> bot{0.0, 0.0, 0.0};
     if (on) {
-        const double *lo = uc + ((k0 + 2) % 3) * SUN, *hi = uc + (k0 % 3) * SUN;
-        const double *rl = raw + ((k0 - 1) & 3) * SPL, *rh = raw + (k0 & 3) * SPL;
-        double n = LES ? nu + 0.5 * (rl[SXN + SYN + SZN + a] + rh[SXN + SYN + SZN + a]) : nu;
+        const double *rl = raw + SPL, *rh = raw + 2 * SPL;
+        double n = LES ? nu + 0.5 * (rl[ON + a] + rh[ON + a]) : nu;
         if (LES && k0 == 1 && p.bc[TG_KLEFT] == TG_BC_SLIP) n = 0.0;
-        bot = kface(lo, hi, n, rl[SXN + SYN + a], dydz * t.rdxf[(k0 == 1 && g.pk) ? mz - 2 : k0 - 1]);
+        bot = kface(uc + SUN, uc + 2 * SUN, n, rl[OZ + a], dydz * t.rdxf[(k0 == 1 && g.pk) ? mz - 2 : k0 - 1]);
     }
     __syncthreads();
-    load(k0 + 2);
+    load(k0 + 2, raw);
     commit();
-    for (int k = k0; k <= k1; k++) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");     // plane k+1 is there
-        __syncthreads();
-        convert(k + 1);
-        if (k < k1 - 1) load(k + 3);
-        commit();
-        __syncthreads();
-        if (!on) continue;
-        const double *um = uc + ((k + 2) % 3) * SUN, *u0 = uc + (k % 3) * SUN, *up = uc + ((k + 1) % 3) * SUN;
-        const double *r0 = raw + (k & 3) * SPL, *rp = raw + ((k + 1) & 3) * SPL;
-        const double *N = r0 + SXN + SYN + SZN;
-        const double dx = t.dx[k], qdx = 0.25 * dx, dxdz = dx * dz, dxdy = dx * dy;
-        const double nc = LES ? N[a] : 0.0;
-        double nt = LES ? nu + 0.5 * (nc + rp[SXN + SYN + SZN + a]) : nu;
-        if (LES && k == mz - 2 && p.bc[TG_KRIGHT] == TG_BC_SLIP) nt = 0.0;
-        const R3<double> top = kface(u0, up, nt, r0[SXN + SYN + a], dydz * t.rdxf[k]);
-        R3<double> f = top - bot;
-        bot = top;
-        const double *U0 = u0, *U1 = u0 + SZN, *U2 = u0 + 2 * SZN;
-        // i faces: e = +1 (east of a), w = the face west of a, flux from point b to b + 1
-        auto iface = [&](int b, double x, double n, double I1, double sg) {
-            const int e = b + 1;
-            const double x0 = U0[b], x1 = U0[e], y0 = U1[b], y1 = U1[e], z0 = U2[b], z1 = U2[e];
-            const double h = -0.5 * x, w = n * I1;
-            const double vx = (up[SZN + e] + up[SZN + b]) - (um[SZN + e] + um[SZN + b]), vz = (U1[e + PTX] + U1[b + PTX]) - (U1[e - PTX] + U1[b - PTX]);
-            f.x += sg * (h * (x0 + x1) + w * (x1 - x0) + (n * qdz) * vx);
-            f.y += sg * (h * (y0 + y1) + (2.0 * w) * (y1 - y0));
-            f.z += sg * (h * (z0 + z1) + w * (z1 - z0) + (n * qdx) * vz);
-        };
-        auto jface = [&](int b, double y, double n, double J1, double sg) {
-            const int e = b + PTX;
-            const double x0 = U0[b], x1 = U0[e], y0 = U1[b], y1 = U1[e], z0 = U2[b], z1 = U2[e];
-            const double h = -0.5 * y, w = n * J1;
-            const double wx = (up[2 * SZN + e] + up[2 * SZN + b]) - (um[2 * SZN + e] + um[2 * SZN + b]), wy = (U2[e + 1] + U2[b + 1]) - (U2[e - 1] + U2[b - 1]);
-            f.x += sg * (h * (x0 + x1) + w * (x1 - x0) + (n * qdy) * wx);
-            f.y += sg * (h * (y0 + y1) + w * (y1 - y0) + (n * qdx) * wy);
-            f.z += sg * (h * (z0 + z1) + (2.0 * w) * (z1 - z0));
-        };
-        const double *X = r0 + ax, *Y = r0 + SXN + a;
-        iface(a, X[1], offE ? 0.0 : LES ? nu + 0.5 * (nc + N[a + 1]) : nu, dxdz * ryE, 1.0);
-        iface(a - 1, X[0], offW ? 0.0 : LES ? nu + 0.5 * (nc + N[a - 1]) : nu, dxdz * ryW, -1.0);
-        jface(a, Y[PTX], offN ? 0.0 : wmN ? nu : LES ? nu + 0.5 * (nc + N[a + PTX]) : nu, dxdy * rzN, 1.0);
-        jface(a - PTX, Y[0], offS ? 0.0 : wmS ? nu : LES ? nu + 0.5 * (nc + N[a - PTX]) : nu, dxdy * rzS, -1.0);
-        if (wmS || wmN) {
-            const int w = k * mx + i;
-            const double sg = (wmS ? 1.0 : 0.0) - (wmN ? 1.0 : 0.0);
-            f.x += sg * s.twx[w]; f.y += sg * s.twy[w]; f.z += sg * s.twz[w];
+    // Plane k = k0 + t is in slots (t + 2) & 3; four planes per trip so that every
+    // slot is a constant offset. One barrier per plane: Ucat of plane k+2 and the
+    // copy of plane k+3 go to slots that plane k does not read.
+    for (int kb = k0; kb <= k1; kb += 4) {
+        #pragma unroll
+        for (int ph = 0; ph < 4; ph++) {
+            const int k = kb + ph;
+            if (k > k1) break;
+            const double dx = t.dx[k], rxf = t.rdxf[k], rx2 = rdx(k + 2);
+            cp_async_wait_all();                                     // plane k+2 is there
+            __syncthreads();
+            if (k < k1) {
+                convert(k + 2, rx2, raw + (ph & 3) * SPL, raw + ((ph + 3) & 3) * SPL, uc + (ph & 3) * SUN);
+                if (k < k1 - 1) load(k + 3, raw + ((ph + 1) & 3) * SPL);
+                commit();
+            }
+            if (!on) continue;
+            const double *um = uc + ((ph + 1) & 3) * SUN, *u0 = uc + ((ph + 2) & 3) * SUN, *up = uc + ((ph + 3) & 3) * SUN;
+            const double *r0 = raw + ((ph + 2) & 3) * SPL, *rp = raw + ((ph + 3) & 3) * SPL;
+            const double *N = r0 + ON;
+            const double qdx = 0.25 * dx, dxdz = dx * dz, dxdy = dx * dy;
+            const double nc = LES ? N[a] : 0.0;
+            double nt = LES ? nu + 0.5 * (nc + rp[ON + a]) : nu;
+            if (LES && k == mz - 2 && p.bc[TG_KRIGHT] == TG_BC_SLIP) nt = 0.0;
+            const R3<double> top = kface(u0, up, nt, r0[OZ + a], dydz * rxf);
+            R3<double> f = top - bot;
+            bot = top;
+            const double *U0 = u0, *U1 = u0 + SZN, *U2 = u0 + 2 * SZN;
+            // i face between tile points b and b + 1 (sg: + for the cell's + side)
+            auto iface = [&](int b, double x, double n, double I1, double sg) {
+                const int e = b + 1;
+                const double x0 = U0[b], x1 = U0[e], y0 = U1[b], y1 = U1[e], z0 = U2[b], z1 = U2[e];
+                const double h = -0.5 * x, w = n * I1;
+                const double vx = (up[SZN + e] + up[SZN + b]) - (um[SZN + e] + um[SZN + b]), vz = (U1[e + PTX] + U1[b + PTX]) - (U1[e - PTX] + U1[b - PTX]);
+                f.x += sg * (h * (x0 + x1) + w * (x1 - x0) + (n * qdz) * vx);
+                f.y += sg * (h * (y0 + y1) + (2.0 * w) * (y1 - y0));
+                f.z += sg * (h * (z0 + z1) + w * (z1 - z0) + (n * qdx) * vz);
+            };
+            auto jface = [&](int b, double y, double n, double J1, double sg) {
+                const int e = b + PTX;
+                const double x0 = U0[b], x1 = U0[e], y0 = U1[b], y1 = U1[e], z0 = U2[b], z1 = U2[e];
+                const double h = -0.5 * y, w = n * J1;
+                const double wx = (up[2 * SZN + e] + up[2 * SZN + b]) - (um[2 * SZN + e] + um[2 * SZN + b]), wy = (U2[e + 1] + U2[b + 1]) - (U2[e - 1] + U2[b - 1]);
+                f.x += sg * (h * (x0 + x1) + w * (x1 - x0) + (n * qdy) * wx);
+                f.y += sg * (h * (y0 + y1) + w * (y1 - y0) + (n * qdx) * wy);
+                f.z += sg * (h * (z0 + z1) + (2.0 * w) * (z1 - z0));
+            };
+            const double *X = r0 + ax, *Y = r0 + OY + a;
+            iface(a, X[1], offE ? 0.0 : LES ? nu + 0.5 * (nc + N[a + 1]) : nu, dxdz * ryE, 1.0);
+            iface(a - 1, X[0], offW ? 0.0 : LES ? nu + 0.5 * (nc + N[a - 1]) : nu, dxdz * ryW, -1.0);
+            jface(a, Y[PTX], offN ? 0.0 : wmN ? nu : LES ? nu + 0.5 * (nc + N[a + PTX]) : nu, dxdy * rzN, 1.0);
+            jface(a - PTX, Y[0], offS ? 0.0 : wmS ? nu : LES ? nu + 0.5 * (nc + N[a - PTX]) : nu, dxdy * rzS, -1.0);
+            if (wmS || wmN) {
+                const int w = k * mx + i;
+                const double sg = (wmS ? 1.0 : 0.0) - (wmN ? 1.0 : 0.0);
+                f.x += sg * s.twx[w]; f.y += sg * s.twy[w]; f.z += sg * s.twz[w];
+            }
+            if (!((k == 1 || k == mz - 2) ? kedge : edge)) st3(fp, (k * my + j) * mx + i, f);
         }
-        if (!edge_cell(g, k, j, i)) st3(fp, (k * my + j) * mx + i, f);
     }
 }
 
@@ -775,6 +783,10 @@ __global__ void __launch_bounds__(256, 8) k_rhs_tensor(Grid g, Tensor t, State s
         rk_point(s.ucont.x + c, s.utmp.x + c, s.ucont_o.x + c, o.x, rk);
         rk_point(s.ucont.y + c, s.utmp.y + c, s.ucont_o.y + c, o.y, rk);
         rk_point(s.ucont.z + c, s.utmp.z + c, s.ucont_o.z + c, o.z, rk);
+        // resetNoPenetrationFluxes, which follows every stage
+        if (i == g.mx - 2 && wall_patch(p, TG_IRIGHT)) s.ucont.x[c] = 0.0;
+        if (j == g.my - 2 && wall_patch(p, TG_JRIGHT)) s.ucont.y[c] = 0.0;
+        if (k == g.mz - 2 && wall_patch(p, TG_KRIGHT)) s.ucont.z[c] = 0.0;
     } else {
         st3(R, c, o);
     }
