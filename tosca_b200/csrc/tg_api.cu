@@ -301,7 +301,8 @@ tg_status tg_create(const tg_config *cfg, tg_ctx **out)
         for (auto **v : ss) *v = dallocd(C, G);
         if (cfg->ddt_scheme == TG_DDT_CN) st.rhs_o = dalloc3(C, G);
         if (cfg->teqn) {
-            st.tdiv = dalloc3(C, G); st.tvisc = dalloc3(C, G);
+            st.tflux = dalloc3(C, G);
+            if (cfg->les) st.trd2 = dalloc3(C, G);
             st.trhs = dallocd(C, G); st.tmprt_o = dallocd(C, G); st.ttmp = dallocd(C, G);
             if (cfg->t_ddt_scheme == TG_TDDT_ABBE) { C->tconv = dallocd(C, G); C->tconv_o = dallocd(C, G); }
             if (cfg->t_ddt_scheme == TG_TDDT_BDF2) C->tmprt_oo = dallocd(C, G);
@@ -312,6 +313,7 @@ tg_status tg_create(const tg_config *cfg, tg_ctx **out)
         C->red_blocks = 148 * 4;
         C->d_red = dallocd(C, 4 * (size_t)C->red_blocks + 64);
         C->d_scal = dallocd(C, 128);
+        C->d_count = (unsigned *)dalloc(C, 4 * sizeof(unsigned));
         set_device_step(C);
         TG_CUDA(cudaMallocHost((void **)&C->h_scal, 128 * sizeof(double)));
         std::memset(C->h_scal, 0, 128 * sizeof(double));
@@ -373,6 +375,7 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
         TG_CUDA(cudaStreamSynchronize(C->stream));
         metrics_from_nodes(C, dn);
         refresh_filter(C);
+        refresh_teqn_mesh(C);
         if (C->cfg.p_tilde) {
             if (!C->node_z) C->node_z = dallocd(C, G);
             TG_CUDA(cudaMemcpy2DAsync(C->node_z, sizeof(double), dn + 2, 3 * sizeof(double), sizeof(double), G,
@@ -455,6 +458,7 @@ tg_status tg_set_field(tg_ctx *C, int32_t w, const double *host, int32_t halo)
         if (w == TG_F_DP) C->clear_dp = true;
         if ((w >= TG_F_CSI && w <= TG_F_KZET) || (w >= TG_F_AJ && w <= TG_F_KAJ)) {
             C->met32_stale = true;
+            if (w >= TG_F_AJ) refresh_teqn_mesh(C);
             if (C->axis_aligned) {         // the caller's metrics need not be those of a mesh of planes
                 C->axis_aligned = false;
                 graph_destroy(C);

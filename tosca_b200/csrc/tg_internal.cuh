@@ -80,6 +80,8 @@ struct Tensor {
     const double *dx, *dy, *dz, *dxf, *dyf, *dzf;
     const double *rdx, *rdy, *rdz, *rdxf, *rdyf, *rdzf;
     const double *qx, *qy, *qz;
+    // reciprocal factors of the cells and of the face distances (tg_teqn.cu)
+    const double *rqx, *rqy, *rqz, *rqxf, *rqyf, *rqzf;
 };
 
 // FormU work planes at storage precision T: face fluxes per direction and
@@ -94,8 +96,9 @@ struct State {
     V3f<double> ucont, ucont_o, ucat, rhs, dp, btheta, btheta_o, gcont, utmp, snap;
     V3f<double> source;          // ueqn->sourceU, cell-centred Cartesian body force
     V3f<double> farmcont;        // farm->sourceFarmCont, contravariant turbine body force (tg_farm.cu)
-    // temperature transport (tg_teqn.cu): lDivT, lViscT face fluxes, Rhs, Tmprt_o, TmprtTmp
-    V3f<double> tdiv, tvisc;
+    // temperature transport (tg_teqn.cu): face fluxes (lDivT + lViscT), 1/delta^2 of
+    // the faces (with LES), Rhs, Tmprt_o, TmprtTmp
+    V3f<double> tflux, trd2;
     double *trhs, *tmprt_o, *ttmp;
     V3f<double> rhs_o;           // ueqn->Rhs_o: FormU of the last step's final state (CN)
     double *p, *phi, *nut, *tmprt, *ssnap;
@@ -178,6 +181,7 @@ struct tg_ctx {
     std::vector<void *> allocs;          // every device allocation of this context
     double *d_red = nullptr;             // reduction scratch (partials)
     double *d_scal = nullptr;            // device scalars
+    unsigned *d_count = nullptr;         // arrival counters of last_block: 0 wall model, 1 thermal wall model
     double *h_scal = nullptr;            // pinned host mirror of scalars
     double *stage = nullptr;             // staging buffer for AoS host transfers
     size_t stage_bytes = 0;
@@ -309,6 +313,37 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV], Ops... ops)
             ((v[q] = ops(v[q], __shfl_down_sync(0xffffffffu, v[q], o)), q++), ...);
         }
     }
+}
+
+// True in every thread of the block that arrives last at the counter (zero
+// before the launch and after it). What thread 0 of each block wrote before is
+// then visible to that block (read it past L1, __ldcg): the blocks' partials can
+// be finished without another launch, in a fixed order whatever the order of
+// arrival.
+__device__ __forceinline__ bool last_block(unsigned *count)
+{
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last && threadIdx.x == 0) { __threadfence(); *count = 0u; }
+    return last;
+}
+// sums of the NV partials per block at part[NV * block ..], in thread 0 of a
+// block of NT threads
+template <int NT, int NV>
+__device__ __forceinline__ void sum_partials(const double *part, double (&v)[NV])
+{
+    #pragma unroll
+    for (int q = 0; q < NV; q++) v[q] = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += NT)
+        #pragma unroll
+        for (int q = 0; q < NV; q++) v[q] += __ldcg(part + NV * b + q);
+    __syncthreads();           // block_reduce's shared memory may still be read
+    static_assert(NV == 3, "three sums");
+    block_reduce<NT>(v, RedSum{}, RedSum{}, RedSum{});
 }
 
 // block_reduce of one sum, returned to every thread of the block
@@ -450,6 +485,7 @@ void imex_destroy(tg_ctx *C);
 void cn_build_bu(tg_ctx *C, V3f<double> bu, bool half_rhs_o);   // tg_step.cu
 void mask_non_resolved(tg_ctx *C, V3f<double> v);               // resetNonResolvedCellFaces on v
 void contra_to_cart_stage(tg_ctx *C);
+void refresh_teqn_mesh(tg_ctx *C);      // face filter widths after a change of aj
 int solve_t(tg_ctx *C);      // 0, or the ABBE GMRES status (1 iteration cap, 2 breakdown)
 void update_temperature_bcs(tg_ctx *C);
 void update_wall_models_t(tg_ctx *C);   // UpdateWallModelsT: jLeft thetaWallFunction qWall

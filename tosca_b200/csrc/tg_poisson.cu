@@ -411,21 +411,6 @@ struct Rows {
         : nx(P.nx), ny(P.ny), nrow(P.ny * P.nz), lane(threadIdx.x & 31),
           row((int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5)), step((int)((gridDim.x * blockDim.x) >> 5)) {}
 };
-// true in every thread of the block that arrives last; the partials that thread 0
-// of each block wrote before are then visible (read past L1 with __ldcg). The
-// sums run over the blocks in a fixed order: the result does not depend on the
-// order of arrival.
-__device__ __forceinline__ bool last_block(unsigned *count)
-{
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(count, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) { __threadfence(); *count = 0u; }
-    return last;
-}
 // totals of N partials per block (sums; the last slot a maximum if MAX) into v of thread 0
 template <int N, bool MAX>
 __device__ __forceinline__ void total(const double *part, double (&v)[3])

@@ -333,9 +333,10 @@ __device__ __forceinline__ void wall_parallel(Grid g, Metrics m, State s, int k,
     Up = U - dot3(U, n) * n;
 }
 
-// per-block partial sums of |U_par|, the wall distance and (coupled) qWall
-// over the j=1 plane
-__global__ void __launch_bounds__(256) k_wall_plane_sums(Grid g, Metrics m, State s, Params p, double *part)
+// sums of |U_par|, the wall distance and (coupled) qWall over the j=1 plane, and
+// in the last block u* = uStarShumann(<|U_par|>, <s>, <qWall>) into out[2] (a
+// separate one-thread launch walked the 148 partials in 11 us)
+__global__ void __launch_bounds__(256) k_wall_plane_sums(Grid g, Metrics m, State s, Params p, double *part, unsigned *count, double *out)
 {
     int nI = g.mx - 2, nK = g.mz - 2;
     double su = 0.0, sd = 0.0, sq = 0.0;
@@ -351,18 +352,13 @@ __global__ void __launch_bounds__(256) k_wall_plane_sums(Grid g, Metrics m, Stat
     double v[3] = {su, sd, sq};
     block_reduce<256>(v, RedSum{}, RedSum{}, RedSum{});
     if (threadIdx.x == 0) { part[3 * blockIdx.x] = v[0]; part[3 * blockIdx.x + 1] = v[1]; part[3 * blockIdx.x + 2] = v[2]; }
-}
-
-// final sums (deterministic order) and u* = uStarShumann(<|U_par|>, <s>, qWall)
-__global__ void k_wall_ustar(Grid g, Params p, const double *part, int nb, double *out)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double su = 0.0, sd = 0.0, sq = 0.0;
-    for (int b = 0; b < nb; b++) { su += part[3 * b]; sd += part[3 * b + 1]; sq += part[3 * b + 2]; }
-    double cnt = (double)(g.mx - 2) * (double)(g.mz - 2);
-    double Umean = su / cnt, dist = sd / cnt, q = sq / cnt;
-    double us = mo::ustar(Umean, dist, p.z0, p.wall_gamma_m, p.kappa, p.wall_coupled ? q : 0.0, p.wall_theta_ref);
-    out[0] = Umean; out[1] = dist; out[2] = us;
+    if (!last_block(count)) return;
+    sum_partials<256>(part, v);
+    if (threadIdx.x != 0) return;
+    const double cnt = (double)nI * (double)nK;
+    const double Umean = v[0] / cnt, dist = v[1] / cnt, q = v[2] / cnt;
+    out[0] = Umean; out[1] = dist;
+    out[2] = mo::ustar(Umean, dist, p.z0, p.wall_gamma_m, p.kappa, p.wall_coupled ? q : 0.0, p.wall_theta_ref);
 }
 
 __global__ void k_wall_init_filter(Grid g, Metrics m, State s)
@@ -1296,8 +1292,7 @@ void update_wall_models(tg_ctx *C)
     if (!C->prm.les || C->prm.bc[TG_JLEFT] != TG_BC_WALL_SHUMANN) return;
     const Grid g = C->g;
     const int nb = 148;
-    TG_PROF(C, "wall_plane_sums", k_wall_plane_sums<<<nb, 256, 0, C->stream>>>(g, C->m, C->s, C->prm, C->d_red));
-    k_wall_ustar<<<1, 32, 0, C->stream>>>(g, C->prm, C->d_red, nb, C->d_scal + 8);
+    TG_PROF(C, "wall_plane_sums", k_wall_plane_sums<<<nb, 256, 0, C->stream>>>(g, C->m, C->s, C->prm, C->d_red, C->d_count, C->d_scal + 8));
     dim3 grid((g.mx - 2 + 31) / 32, (g.mz - 2 + 7) / 8);
     if (!C->ufilt_set) {
         k_wall_init_filter<<<grid, b2, 0, C->stream>>>(g, C->m, C->s);

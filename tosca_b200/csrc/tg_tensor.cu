@@ -932,26 +932,31 @@ bool tensor_setup(tg_ctx *C)
     const int n[3] = {g.mz, g.mx, g.my};                       // x, y, z
     const int64_t first[3] = {o - pl, o - 1, o - g.mx}, stride[3] = {pl, 1, g.mx};
     const double *area[3] = {m.zet.x, m.csi.y, m.eta.z}, *farea[3] = {m.kzet.x, m.icsi.y, m.jeta.z}, *fj[3] = {m.kaj, m.iaj, m.jaj};
-    if (!C->ts_mem) C->ts_mem = dallocd(C, 5 * ((size_t)g.mx + g.my + g.mz));
+    constexpr int NA = 7;        // arrays per direction
+    if (!C->ts_mem) C->ts_mem = dallocd(C, NA * ((size_t)g.mx + g.my + g.mz));
     double *mem = C->ts_mem;
-    const double **d[3][5] = {{&C->ts.dx, &C->ts.rdx, &C->ts.dxf, &C->ts.rdxf, &C->ts.qx},
-                              {&C->ts.dy, &C->ts.rdy, &C->ts.dyf, &C->ts.rdyf, &C->ts.qy},
-                              {&C->ts.dz, &C->ts.rdz, &C->ts.dzf, &C->ts.rdzf, &C->ts.qz}};
+    Tensor &t = C->ts;
+    const double **d[3][NA] = {{&t.dx, &t.rdx, &t.dxf, &t.rdxf, &t.qx, &t.rqx, &t.rqxf},
+                               {&t.dy, &t.rdy, &t.dyf, &t.rdyf, &t.qy, &t.rqy, &t.rqyf},
+                               {&t.dz, &t.rdz, &t.dzf, &t.rdzf, &t.qz, &t.rqz, &t.rqzf}};
     for (int q = 0; q < 3; q++) {
         // size = volume / area at the cells of the line through (1, 1, 1), with
         // its ghosts, and across the faces 0 .. m-2
         const std::vector<double> aj = line(m.aj, first[q], stride[q], n[q]), a = line(area[q], first[q], stride[q], n[q]),
                                   fa = line(farea[q], first[q], stride[q], n[q]), fv = line(fj[q], first[q], stride[q], n[q]);
-        std::vector<double> h(5 * (size_t)n[q], 0.0);
+        std::vector<double> h(NA * (size_t)n[q], 0.0);
         for (int l = 0; l < n[q]; l++) {
             const double r = aj[l] * a[l], rf = fv[l] * fa[l];
             h[l] = 1.0 / r; h[n[q] + l] = r;
             if (l < n[q] - 1) { h[2 * n[q] + l] = 1.0 / rf; h[3 * n[q] + l] = rf; }
-            h[4 * n[q] + l] = std::cbrt(h[l]) * std::cbrt(h[l]);    // (dx dy dz)^(2/3) by factors
+            auto sq = [](double x) { return std::cbrt(x) * std::cbrt(x); };
+            h[4 * n[q] + l] = sq(h[l]);                         // (dx dy dz)^(2/3) by factors
+            h[5 * n[q] + l] = sq(r);
+            if (l < n[q] - 1) h[6 * n[q] + l] = sq(rf);
         }
         TG_CUDA(cudaMemcpyAsync(mem, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, st));
         TG_CUDA(cudaStreamSynchronize(st));
-        for (int e = 0; e < 5; e++) *d[q][e] = mem + (size_t)e * n[q];
+        for (int e = 0; e < NA; e++) *d[q][e] = mem + (size_t)e * n[q];
         mem += h.size();
     }
     k_tensor_check<<<C->red_blocks, 256, 0, st>>>(g, m, C->ts, C->d_red);

@@ -12,6 +12,7 @@
 // thetaWallFunction's heat flux (UpdateWallModelsT, boundary.c:3858-4178)
 // replaces the diffusive flux of the jLeft wall faces. FP64 in every
 // precision mode.
+#include <algorithm>
 #include <cmath>
 
 #include "tg_internal.cuh"
@@ -44,18 +45,14 @@ __device__ __forceinline__ double weno3(double f0, double f1, double f2, double 
 // derivative. With Smagorinsky, nu_t / Pr_t with Pr_t = 1 / (1 + 2 l/delta)
 // and, in stable stratification, l/delta = min(1, 7.6 nu_t sqrt(tRef/|g
 // dT/deta|) / delta^2), delta = (1/ajc)^(1/3): evaluated as nu_t (1 + 2
-// l/delta) with 1/delta^2 = cbrt(ajc)^2, the same value up to rounding in
-// one cube root, one division and one square root (the literal form takes
-// five more divisions; the kernel issues about 1700 instructions per cell)
-__device__ __forceinline__ double kappa_eff(const Params &p, double nut, double dtde, double ajc)
+// l/delta) with rd2 = 1/delta^2 from the mesh (k_t_width: a cube root per face
+// and stage was a tenth of the kernel) and one reciprocal square root
+__device__ __forceinline__ double kappa_eff(const Params &p, double nut, double dtde, double rd2, double sqt)
 {
     if (!p.les) return p.nu / p.prandtl;
     const double gradTdotG = dtde * (-9.81);
     double ratio = 1.0;                                    // l / delta
-    if (gradTdotG < 0.) {
-        const double cr = cbrt(ajc);                       // 1 / delta
-        ratio = fmin(1.0, 7.6 * nut * (cr * cr) * sqrt(p.t_ref / fabs(gradTdotG)));
-    }
+    if (gradTdotG < 0.) ratio = fmin(1.0, 7.6 * nut * rd2 * (sqt * rsqrt(-gradTdotG)));
     return nut * (1.0 + 2.0 * ratio);
 }
 
@@ -70,28 +67,28 @@ __device__ __forceinline__ void stencil4(int i, int m, int per, int &L, int &R)
     } else { L = i - 1; R = i + 2; }
 }
 
-// pass 1: convective and diffusive fluxes at the faces of the interior
-// cells. One thread per interior cell (k, j, i) forms the i, j and k faces on
-// the cell's + side, and a cell next to a non-periodic 0 boundary also the
-// face on its - side (face 0; face 0 of a periodic direction is read from
-// face m-2 by the budget and is not formed). T and nut are staged in a
-// shared-memory tile of the block's cells with one cell below and two above
-// in every direction (the DMDA wrap of periodic directions applied once, at
-// staging), so every stencil read is a fixed tile offset; the WENO points of
-// the boundary faces, which may lie outside the tile (periodic i = mx + 2 and
-// i = -3), are read from global memory.
+// pass 1: the flux at the faces of the interior cells, convective plus diffusive
+// (mode 0), convective (1) or diffusive (2). One thread per interior cell
+// (k, j, i) forms the i, j and k faces on the cell's + side, and a cell next to
+// a non-periodic 0 boundary also the face on its - side (face 0; face 0 of a
+// periodic direction is read from face m-2 by the budget and is not formed). T
+// and nut are staged in a shared-memory tile of the block's cells with one cell
+// below and two above in every direction (the DMDA wrap of periodic directions
+// applied once, at staging), so every stencil read is a fixed tile offset; the
+// WENO points of the boundary faces, which may lie outside the tile (periodic
+// i = mx + 2 and i = -3), are read from global memory.
 //
-// AX: the mesh is axis-aligned (csi || y, eta || z, zet || x; tg_mesh_info):
-// the metric tensor of a face is its normal component squared, g11 = csi.y^2
-// at i faces, g21 = eta.z^2 at j faces, g31 = zet.x^2 at k faces, and the
-// cross terms, zero up to the round-off of the metric evaluation, are left
-// out with the derivatives they multiply; kappa_eff still reads the eta
-// derivative of every face (the stability correction of Pr_t).
+// AX: a mesh of planes: the metric tensor of a face is its normal component
+// squared, and with aj a product of spacings (tg_tensor.cu, t), so no metric is
+// read; the cross terms are left out with the derivatives they multiply;
+// kappa_eff still reads the eta derivative of every face (the stability
+// correction of Pr_t). rd2: 1/delta^2 of the i, j and k faces (k_t_width), on a
+// mesh of planes a product of factors as well.
 constexpr int TBX = 32, TBY = 4, TBZ = 2, TBN = TBX * TBY * TBZ;
 constexpr int TTX = TBX + 3, TTY = TBY + 3, TTZ = TBZ + 3, TTN = TTX * TTY * TTZ;
 
-template <bool AX>
-__global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State s, Params p, V3f<double> dv, V3f<double> vs)
+template <bool AX, int mode>
+__global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, Tensor t, State s, Params p, V3f<double> rd2, V3f<double> fl)
 {
     __shared__ double st[TTN];
     __shared__ double sn[TTN];
@@ -130,6 +127,7 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State 
     auto T = [&](int dk, int dj, int di) { return st[t0 + (dk * TTY + dj) * TTX + di]; };
     auto NUT = [&](int dk, int dj, int di) { return sn[t0 + (dk * TTY + dj) * TTX + di]; };
     auto TG = [&](int kk, int jj, int ii) { return s.tmprt[g.id(kk, jj, ii)]; };
+    const double sqt = sqrt(p.t_ref);
 
     // ---- i face fi = i + e (Compute_dscalar_i, inline.h:3210-3247)
     auto iface = [&](int fi, int e) {
@@ -145,24 +143,28 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State 
             else if (k == 1 && edge && (npk || npi))  dtdz = (T(1, 0, e + 1) + T(1, 0, e) - T(0, 0, e + 1) - T(0, 0, e)) * 0.5;
             else                                      dtdz = (T(1, 0, e + 1) + T(1, 0, e) - T(-1, 0, e + 1) - T(-1, 0, e)) * 0.25;
         }
-        const double uc = s.ucont.x[f];
-        double w;
-        if (edge) {
-            int iL, iR;
-            stencil4(fi, mx, g.pi, iL, iR);
-            w = weno3(TG(k, j, iL), T(0, 0, e), T(0, 0, e + 1), TG(k, j, iR), uc);
-        } else w = weno3(T(0, 0, e - 1), T(0, 0, e), T(0, 0, e + 1), T(0, 0, e + 2), uc);
-        dv.x[f] = -uc * w;
-        const double ajc = m.iaj[f];
-        const double ke = kappa_eff(p, p.les ? 0.5 * (NUT(0, 0, e) + NUT(0, 0, e + 1)) : 0.0, dtde, ajc);
+        double o = 0.0;
+        if (mode != 2) {
+            const double uc = s.ucont.x[f];
+            double w;
+            if (edge) {
+                int iL, iR;
+                stencil4(fi, mx, g.pi, iL, iR);
+                w = weno3(TG(k, j, iL), T(0, 0, e), T(0, 0, e + 1), TG(k, j, iR), uc);
+            } else w = weno3(T(0, 0, e - 1), T(0, 0, e), T(0, 0, e + 1), T(0, 0, e + 2), uc);
+            o = -uc * w;
+        }
+        if (mode == 1) { fl.x[f] = o; return; }
+        const double wd = !p.les ? 0.0 : AX ? t.rqx[k] * t.rqyf[fi] * t.rqz[j] : rd2.x[f];
+        const double ke = kappa_eff(p, p.les ? 0.5 * (NUT(0, 0, e) + NUT(0, 0, e + 1)) : 0.0, dtde, wd, sqt);
         if (AX) {
-            const double cs = m.icsi.y[f];
-            vs.x[f] = 0.0 + ((cs * cs) * dtdc) * ajc * ke;
+            fl.x[f] = o + (t.dx[k] * t.dz[j] * t.rdyf[fi] * dtdc) * ke;
         } else {
+            const double ajc = m.iaj[f];
             const R3<double> cs = ld3(m.icsi, f), et = ld3(m.ieta, f), ze = ld3(m.izet, f);
             const double g11 = cs.x * cs.x + cs.y * cs.y + cs.z * cs.z, g21 = et.x * cs.x + et.y * cs.y + et.z * cs.z,
                          g31 = ze.x * cs.x + ze.y * cs.y + ze.z * cs.z;
-            vs.x[f] = 0.0 + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
+            fl.x[f] = o + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
         }
     };
     // ---- j face fj = j + e (Compute_dscalar_j, inline.h:3252-3289)
@@ -179,16 +181,20 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State 
             else if (k == 1 && edge && (npk || npj))  dtdz = (T(1, e + 1, 0) + T(1, e, 0) - T(0, e + 1, 0) - T(0, e, 0)) * 0.5;
             else                                      dtdz = (T(1, e + 1, 0) + T(1, e, 0) - T(-1, e + 1, 0) - T(-1, e, 0)) * 0.25;
         }
-        const double uc = s.ucont.y[f];
-        double w;
-        if (edge) {
-            int jL, jR;
-            stencil4(fj, my, g.pj, jL, jR);
-            w = weno3(TG(k, jL, i), T(0, e, 0), T(0, e + 1, 0), TG(k, jR, i), uc);
-        } else w = weno3(T(0, e - 1, 0), T(0, e, 0), T(0, e + 1, 0), T(0, e + 2, 0), uc);
-        dv.y[f] = -uc * w;
-        const double ajc = m.jaj[f];
-        double ke = kappa_eff(p, p.les ? 0.5 * (NUT(0, e, 0) + NUT(0, e + 1, 0)) : 0.0, dtde, ajc);
+        double o = 0.0;
+        if (mode != 2) {
+            const double uc = s.ucont.y[f];
+            double w;
+            if (edge) {
+                int jL, jR;
+                stencil4(fj, my, g.pj, jL, jR);
+                w = weno3(TG(k, jL, i), T(0, e, 0), T(0, e + 1, 0), TG(k, jR, i), uc);
+            } else w = weno3(T(0, e - 1, 0), T(0, e, 0), T(0, e + 1, 0), T(0, e + 2, 0), uc);
+            o = -uc * w;
+        }
+        if (mode == 1) { fl.y[f] = o; return; }
+        const double wd = !p.les ? 0.0 : AX ? t.rqx[k] * t.rqy[i] * t.rqzf[fj] : rd2.y[f];
+        double ke = kappa_eff(p, p.les ? 0.5 * (NUT(0, e, 0) + NUT(0, e + 1, 0)) : 0.0, dtde, wd, sqt);
         double v0 = 0.0;
         if (p.t_wall && fj == 0) {
             // thetaWallFunction (teqn_solvers.c:337-352): the modelled flux
@@ -198,13 +204,13 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State 
             ke = 0.0;
         }
         if (AX) {
-            const double et = m.jeta.z[f];
-            vs.y[f] = v0 + ((et * et) * dtde) * ajc * ke;
+            fl.y[f] = o + (v0 + (t.dx[k] * t.dy[i] * t.rdzf[fj] * dtde) * ke);
         } else {
+            const double ajc = m.jaj[f];
             const R3<double> cs = ld3(m.jcsi, f), et = ld3(m.jeta, f), ze = ld3(m.jzet, f);
             const double g11 = cs.x * et.x + cs.y * et.y + cs.z * et.z, g21 = et.x * et.x + et.y * et.y + et.z * et.z,
                          g31 = ze.x * et.x + ze.y * et.y + ze.z * et.z;
-            vs.y[f] = v0 + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
+            fl.y[f] = o + (v0 + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke);
         }
     };
     // ---- k face fk = k + e (Compute_dscalar_k, inline.h:3294-3331)
@@ -221,24 +227,28 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State 
         else if (j == 1 && edge && (npj || npk))      dtde = (T(e + 1, 1, 0) + T(e, 1, 0) - T(e + 1, 0, 0) - T(e, 0, 0)) * 0.5;
         else                                          dtde = (T(e + 1, 1, 0) + T(e, 1, 0) - T(e + 1, -1, 0) - T(e, -1, 0)) * 0.25;
         const double dtdz = T(e + 1, 0, 0) - T(e, 0, 0);
-        const double uc = s.ucont.z[f];
-        double w;
-        if (edge) {
-            int kL, kR;
-            stencil4(fk, mz, g.pk, kL, kR);
-            w = weno3(TG(kL, j, i), T(e, 0, 0), T(e + 1, 0, 0), TG(kR, j, i), uc);
-        } else w = weno3(T(e - 1, 0, 0), T(e, 0, 0), T(e + 1, 0, 0), T(e + 2, 0, 0), uc);
-        dv.z[f] = -uc * w;
-        const double ajc = m.kaj[f];
-        const double ke = kappa_eff(p, p.les ? 0.5 * (NUT(e, 0, 0) + NUT(e + 1, 0, 0)) : 0.0, dtde, ajc);
+        double o = 0.0;
+        if (mode != 2) {
+            const double uc = s.ucont.z[f];
+            double w;
+            if (edge) {
+                int kL, kR;
+                stencil4(fk, mz, g.pk, kL, kR);
+                w = weno3(TG(kL, j, i), T(e, 0, 0), T(e + 1, 0, 0), TG(kR, j, i), uc);
+            } else w = weno3(T(e - 1, 0, 0), T(e, 0, 0), T(e + 1, 0, 0), T(e + 2, 0, 0), uc);
+            o = -uc * w;
+        }
+        if (mode == 1) { fl.z[f] = o; return; }
+        const double wd = !p.les ? 0.0 : AX ? t.rqxf[fk] * t.rqy[i] * t.rqz[j] : rd2.z[f];
+        const double ke = kappa_eff(p, p.les ? 0.5 * (NUT(e, 0, 0) + NUT(e + 1, 0, 0)) : 0.0, dtde, wd, sqt);
         if (AX) {
-            const double ze = m.kzet.x[f];
-            vs.z[f] = 0.0 + ((ze * ze) * dtdz) * ajc * ke;
+            fl.z[f] = o + (t.dy[i] * t.dz[j] * t.rdxf[fk] * dtdz) * ke;
         } else {
+            const double ajc = m.kaj[f];
             const R3<double> cs = ld3(m.kcsi, f), et = ld3(m.keta, f), ze = ld3(m.kzet, f);
             const double g11 = cs.x * ze.x + cs.y * ze.y + cs.z * ze.z, g21 = et.x * ze.x + et.y * ze.y + et.z * ze.z,
                          g31 = ze.x * ze.x + ze.y * ze.y + ze.z * ze.z;
-            vs.z[f] = 0.0 + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
+            fl.z[f] = o + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
         }
     };
     const int ni = (i == 1 && npi) ? 2 : 1, nj = (j == 1 && npj) ? 2 : 1, nk = (k == 1 && npk) ? 2 : 1;
@@ -251,32 +261,69 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, State 
 }
 
 // FormT pass 1 on the context's stream
+template <int mode>
 void t_face_fluxes(tg_ctx *C)
 {
     const Grid g = C->g;
     const dim3 gr((g.mx - 2 + TBX - 1) / TBX, (g.my - 2 + TBY - 1) / TBY, (g.mz - 2 + TBZ - 1) / TBZ), bl(TBX, TBY, TBZ);
     State &s = C->s;
     if (C->axis_aligned)
-        TG_PROF(C, "teqn_face_fluxes", k_t_face_fluxes<true><<<gr, bl, 0, C->stream>>>(g, C->m, s, C->prm, s.tdiv, s.tvisc));
+        TG_PROF(C, "teqn_face_fluxes", (k_t_face_fluxes<true, mode><<<gr, bl, 0, C->stream>>>(g, C->m, C->ts, s, C->prm, s.trd2, s.tflux)));
     else
-        TG_PROF(C, "teqn_face_fluxes", k_t_face_fluxes<false><<<gr, bl, 0, C->stream>>>(g, C->m, s, C->prm, s.tdiv, s.tvisc));
+        TG_PROF(C, "teqn_face_fluxes", (k_t_face_fluxes<false, mode><<<gr, bl, 0, C->stream>>>(g, C->m, C->ts, s, C->prm, s.trd2, s.tflux)));
 }
 
-// pass 2 (teqn_solvers.c:520-566): rhs = (div budget + visc budget) aj at
-// interior cells, face 0 of a periodic direction read from face m-2
-// (resetFacePeriodicFluxesVector); formMode 1 keeps the convective budget
-// only, 2 the diffusive one
-__global__ void k_t_rhs(Grid g, Metrics m, V3f<double> dv, V3f<double> vs, double *rhs, int mode)
+// pass 2 (teqn_solvers.c:520-566): the flux budget of interior cell c times aj,
+// face 0 of a periodic direction read from face m-2 (resetFacePeriodicFluxesVector)
+__device__ __forceinline__ double t_budget(const Grid &g, const V3f<double> &fl, int k, int j, int i, int c)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
-    const int c = g.lin(k, j, i), pl = g.mx * g.my;
+    const int pl = g.mx * g.my;
     const int iw = (i == 1 && g.pi) ? c + g.mx - 3 : c - 1;
     const int js = (j == 1 && g.pj) ? c + (g.my - 3) * g.mx : c - g.mx;
     const int kb = (k == 1 && g.pk) ? c + (g.mz - 3) * pl : c - pl;
-    const double divBudget = dv.x[c] - dv.x[iw] + dv.y[c] - dv.y[js] + dv.z[c] - dv.z[kb];
-    const double viscBudget = vs.x[c] - vs.x[iw] + vs.y[c] - vs.y[js] + vs.z[c] - vs.z[kb];
-    rhs[c] = 1.0 * ((mode != 2 ? divBudget : 0.0) + (mode != 1 ? viscBudget : 0.0)) * m.aj[c];
+    return fl.x[c] - fl.x[iw] + fl.y[c] - fl.y[js] + fl.z[c] - fl.z[kb];
+}
+__global__ void k_t_rhs(Grid g, Metrics m, V3f<double> fl, double *rhs)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
+    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
+    const int c = g.lin(k, j, i);
+    rhs[c] = t_budget(g, fl, k, j, i, c) * m.aj[c];
+}
+
+// pass 2 with the RK4 bookkeeping after stage st: Ttmp (+)= dt b Rhs, next stage
+// T = T_o + a dt Rhs, last T = Ttmp. The right-hand side is zero off the
+// interior, so T keeps its T_o there but for the periodic ghosts, which a cell
+// writes with its own value (resetCellPeriodicFluxes). 80 bytes per cell where
+// the budget, the update of every point and the ghost copies moved 152 in up to
+// five launches.
+__global__ void k_t_rk(Grid g, Metrics m, V3f<double> fl, double *t, const double *to, double *ttmp, double cb, double ca, int first, int last)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
+    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
+    const int c = g.lin(k, j, i);
+    const double r = t_budget(g, fl, k, j, i, c) * m.aj[c], o = (first || !last) ? to[c] : 0.0;
+    const double tt = (first ? o : ttmp[c]) + cb * r;
+    double v = tt;
+    if (!last) { ttmp[c] = tt; v = ca * r + o; }
+    t[c] = v;
+    auto image = [](int l, int mm, int per) { return !per ? l : l == 1 ? mm - 1 : l == mm - 2 ? 0 : l; };
+    const int gi = image(i, g.mx, g.pi), gj = image(j, g.my, g.pj), gk = image(k, g.mz, g.pk);
+    if (gi == i && gj == j && gk == k) return;
+    for (int b = 1; b < 8; b++) {
+        if (((b & 1) && gi == i) || ((b & 2) && gj == j) || ((b & 4) && gk == k)) continue;
+        t[g.lin((b & 4) ? gk : k, (b & 2) ? gj : j, (b & 1) ? gi : i)] = v;
+    }
+}
+
+// 1/delta^2 = ajc^(2/3) of every face of an interior cell
+__global__ void k_t_width(Grid g, Metrics m, V3f<double> rd2)
+{
+    const int64_t n = g.size();
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
+        const double a = cbrt(m.iaj[q]), b = cbrt(m.jaj[q]), c = cbrt(m.kaj[q]);
+        rd2.x[q] = a * a; rd2.y[q] = b * b; rd2.z[q] = c * c;
+    }
 }
 
 // TeqnABBE steps 3-5 (teqn_solvers.c:835-880): bT = 3/2 Conv - 1/2 Conv_o
@@ -315,20 +362,12 @@ __global__ void k_t_abbe_av(int64_t n, double *Av, const double *v, const double
         Av[q] = v[q] + -1.0 * (d[q] * dt);
 }
 
-// TeqnRK4 bookkeeping after stage st: Ttmp (+)= dt b Rhs, next stage T = T_o + a dt Rhs, last T = Ttmp
-__global__ void k_t_rk(int64_t n, double *t, const double *to, double *ttmp, const double *rhs, double cb, double ca, int first, int last)
-{
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-        const double tt = (first ? to[q] : ttmp[q]) + cb * rhs[q];
-        if (last) t[q] = tt;
-        else { ttmp[q] = tt; t[q] = ca * rhs[q] + to[q]; }
-    }
-}
-
 // UpdateTemperatureBCs (boundary.c:2052-2616) on the face ghosts of one patch
-// pair (dir: 0 i, 1 j, 2 k), from the interior next to them
-__global__ void k_t_bcs(Grid g, Metrics m, Params p, double *t, int dir, const double *series_st, const double *d_it, double it_start)
+// pair (blockIdx.z: 0 i, 1 j, 2 k), from the interior next to them: no ghost is
+// read, so the three directions share a launch
+__global__ void k_t_bcs(Grid g, Metrics m, Params p, double *t, const double *series_st, const double *d_it, double it_start)
 {
+    const int dir = blockIdx.z;
     const int a = blockIdx.x * blockDim.x + threadIdx.x + 1, b = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int na = dir == 0 ? g.my : g.mx, nb = dir == 2 ? g.my : g.mz;
     if (a > na - 2 || b > nb - 2) return;
@@ -419,9 +458,11 @@ __global__ void k_twall_local(Grid g, Metrics m, State s, Params p, const double
                            s.tmprt[g.lin(k, 1, i)] - st, p.tw_kappa);
 }
 
-// -3 averaged, pass 1: surfaceTheta += heatingRate dt and per-block partial
-// sums of T(j=1) - surfaceTheta, |U_par| and the wall distance
-__global__ void __launch_bounds__(256) k_twall_sums(Grid g, Metrics m, State s, Params p, double *part, const double *sts)
+// -3 averaged: surfaceTheta += heatingRate dt, the sums of T(j=1) - surfaceTheta,
+// |U_par| and the wall distance, and in the last block qWallShumann once from
+// the plane means, the result into every wall cell (a separate launch whose one
+// thread walked the 148 partials took 17 us)
+__global__ void __launch_bounds__(256) k_twall_sums(Grid g, Metrics m, State s, Params p, double *part, const double *sts, unsigned *count, double *sc)
 {
     const int nI = g.mx - 2, nK = g.mz - 2;
     double sT = 0.0, sU = 0.0, sD = 0.0;
@@ -440,27 +481,25 @@ __global__ void __launch_bounds__(256) k_twall_sums(Grid g, Metrics m, State s, 
     block_reduce<256>(v, RedSum{}, RedSum{}, RedSum{});
     if (threadIdx.x == 0)
         for (int q = 0; q < 3; q++) part[3 * blockIdx.x + q] = v[q];
-}
-
-// -3 averaged, pass 2 (one block): the plane means in a fixed order,
-// qWallShumann once, the result into every wall cell; -2 (fixed): the
-// prescribed flux into every wall cell (nb = 0)
-__global__ void k_twall_fill(Grid g, Params p, const double *part, int nb, double *sc, State s)
-{
-    __shared__ double q;
+    if (!last_block(count)) return;
+    sum_partials<256>(part, v);
+    __shared__ double qw;
     if (threadIdx.x == 0) {
-        if (nb > 0) {
-            double sT = 0.0, sU = 0.0, sD = 0.0;
-            for (int b = 0; b < nb; b++) { sT += part[3 * b]; sU += part[3 * b + 1]; sD += part[3 * b + 2]; }
-            const double n = (double)(g.mx - 2) * (double)(g.mz - 2);
-            sc[0] = sT / n; sc[1] = sU / n; sc[2] = sD / n;
-            q = mo::qwall(sU / n, sD / n, p.tw_z0, p.tw_gamma_m, p.tw_gamma_h, p.tw_alpha_h, p.tw_theta_ref, sT / n, p.tw_kappa);
-        } else q = p.tw_qwall;
-        sc[3] = q;
+        const double n = (double)nI * (double)nK;
+        sc[0] = v[0] / n; sc[1] = v[1] / n; sc[2] = v[2] / n;
+        qw = mo::qwall(v[1] / n, v[2] / n, p.tw_z0, p.tw_gamma_m, p.tw_gamma_h, p.tw_alpha_h, p.tw_theta_ref, v[0] / n, p.tw_kappa);
+        sc[3] = qw;
     }
     __syncthreads();
-    const int nI = g.mx - 2, nK = g.mz - 2;
-    for (int t = threadIdx.x; t < nI * nK; t += blockDim.x) s.qwall[(t / nI + 1) * g.mx + t % nI + 1] = q;
+    for (int t = threadIdx.x; t < nI * nK; t += blockDim.x) s.qwall[(t / nI + 1) * g.mx + t % nI + 1] = qw;
+}
+
+// -2 (fixed): the prescribed flux into every wall cell
+__global__ void k_twall_fill(Grid g, Params p, double *sc, State s)
+{
+    const int nI = g.mx - 2, nK = g.mz - 2, t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) sc[3] = p.tw_qwall;
+    if (t < nI * nK) s.qwall[(t / nI + 1) * g.mx + t % nI + 1] = p.tw_qwall;
 }
 
 }  // namespace
@@ -481,8 +520,8 @@ static int solve_t_abbe(tg_ctx *C)
     if (!C->tgm) C->tgm = gmres_alloc(C, G, C->cfg.t_gmres_restart > 0 ? C->cfg.t_gmres_restart : 30);
     // Steps 1-2: periodic ghosts, convective right-hand side at T^n
     reset_cell_periodic_s(C, s.tmprt);
-    t_face_fluxes(C);
-    TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tdiv, s.tvisc, C->tconv, 1));
+    t_face_fluxes<1>(C);
+    TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tflux, C->tconv));
     // Steps 3-4: b (in Ttmp) and the guess; as in the reference the solution
     // goes into RhsConv_o, whose AB2 history this kernel consumes first
     double *b = s.ttmp, *x = C->tconv_o;
@@ -492,8 +531,8 @@ static int solve_t_abbe(tg_ctx *C)
     auto A = [&](const double *v, double *Av) {
         TG_CUDA(cudaMemcpyAsync(s.tmprt, v, sizeof(double) * G, cudaMemcpyDeviceToDevice, C->stream));
         reset_cell_periodic_s(C, s.tmprt);
-        t_face_fluxes(C);
-        TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tdiv, s.tvisc, s.trhs, 2));
+        t_face_fluxes<2>(C);
+        TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tflux, s.trhs));
         TG_PROF(C, "teqn_abbe_av", k_t_abbe_av<<<nblk(G), 256, 0, C->stream>>>(G, Av, v, s.trhs, dt));
     };
     int its = 0;
@@ -524,8 +563,8 @@ static int solve_t_snes(tg_ctx *C)
     auto Feval = [&](const double *t, double *F) {
         TG_CUDA(cudaMemcpyAsync(s.tmprt, t, sizeof(double) * G, cudaMemcpyDeviceToDevice, C->stream));
         reset_cell_periodic_s(C, s.tmprt);
-        t_face_fluxes(C);
-        TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tdiv, s.tvisc, s.trhs, 0));
+        t_face_fluxes<0>(C);
+        TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tflux, s.trhs));
         TG_PROF(C, "teqn_snes_f", k_t_snes_f<<<nblk(G), 256, 0, C->stream>>>(G, F, s.trhs, t, s.tmprt_o,
                                                                            bdf2 ? C->tmprt_oo : s.tmprt_o, dt, bdf2));
     };
@@ -542,7 +581,6 @@ static int solve_t_snes(tg_ctx *C)
 int solve_t(tg_ctx *C)
 {
     const Grid g = C->g;
-    const int64_t G = g.size();
     State &s = C->s;
     const double dt = C->prm.dt;
     if (C->cfg.t_ddt_scheme == TG_TDDT_BE || C->cfg.t_ddt_scheme == TG_TDDT_BDF2) {
@@ -557,15 +595,14 @@ int solve_t(tg_ctx *C)
     }
     const double b[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
     const double a[4] = {0.0, 0.5, 0.5, 1.0};
-    for (int st = 0; st < 4; st++) {
-        // FormExplicitRhsT: periodic ghosts, FormT (Rhs zero off the interior)
-        reset_cell_periodic_s(C, s.tmprt);
-        t_face_fluxes(C);
-        TG_PROF(C, "teqn_rhs", k_t_rhs<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tdiv, s.tvisc, s.trhs, 0));
-        TG_PROF(C, "teqn_rk_update", k_t_rk<<<nblk(G), 256, 0, C->stream>>>(G, s.tmprt, s.tmprt_o, s.ttmp, s.trhs,
-                                                                          dt * b[st], st < 3 ? a[st + 1] * dt : 0.0, st == 0, st == 3));
-    }
+    // FormExplicitRhsT's periodic ghosts: copied before the first stage, then
+    // written by each stage's update
     reset_cell_periodic_s(C, s.tmprt);
+    for (int st = 0; st < 4; st++) {
+        t_face_fluxes<0>(C);
+        TG_PROF(C, "teqn_rk_update", k_t_rk<<<gint(g), block3(), 0, C->stream>>>(g, C->m, s.tflux, s.tmprt, s.tmprt_o, s.ttmp,
+                                                                               dt * b[st], st < 3 ? a[st + 1] * dt : 0.0, st == 0, st == 3));
+    }
     return 0;
 }
 
@@ -574,7 +611,7 @@ int solve_t(tg_ctx *C)
 // follows and the velocity wall function of the next step. -2: the
 // prescribed flux. -3: surfaceTheta is seeded from the wall value on the
 // first call and rises by heatingRate * dt on every call; qWallShumann once
-// from the plane means ("averaged", two launches) or per cell ("localized")
+// from the plane means ("averaged") or per cell ("localized")
 // -4: the surface temperature of the step into its device slot (nullptr
 // when the series is not set yet: the steps refuse to run then, and the ghost
 // update at initialisation, on the first step's clock, is zero-gradient)
@@ -601,7 +638,7 @@ void update_wall_models_t(tg_ctx *C)
     const Grid g = C->g;
     const dim3 b2(32, 8), grid((g.mx - 2 + 31) / 32, (g.mz - 2 + 7) / 8);
     if (C->prm.t_wall == TG_TWALL_FIXED_FLUX) {
-        TG_PROF(C, "twall_fill", k_twall_fill<<<1, 256, 0, C->stream>>>(g, C->prm, C->d_red, 0, C->d_scal + SC_TWALL, C->s));
+        TG_PROF(C, "twall_fill", k_twall_fill<<<((g.mx - 2) * (g.mz - 2) + 255) / 256, 256, 0, C->stream>>>(g, C->prm, C->d_scal + SC_TWALL, C->s));
         return;
     }
     const double *sts = series_surface(C);
@@ -616,20 +653,23 @@ void update_wall_models_t(tg_ctx *C)
         return;
     }
     const int nb = 148;
-    TG_PROF(C, "twall_sums", k_twall_sums<<<nb, 256, 0, C->stream>>>(g, C->m, C->s, C->prm, C->d_red, sts));
-    TG_PROF(C, "twall_fill", k_twall_fill<<<1, 256, 0, C->stream>>>(g, C->prm, C->d_red, nb, C->d_scal + SC_TWALL, C->s));
+    TG_PROF(C, "twall_sums", k_twall_sums<<<nb, 256, 0, C->stream>>>(g, C->m, C->s, C->prm, C->d_red, sts, C->d_count + 1, C->d_scal + SC_TWALL));
 }
 
 void update_temperature_bcs(tg_ctx *C)
 {
     const Grid g = C->g;
     const dim3 b2(32, 8);
-    auto g2 = [](int na, int nb) { return dim3((na - 2 + 31) / 32, (nb - 2 + 7) / 8); };
+    const dim3 gr((std::max(g.mx, g.my) - 2 + 31) / 32, (std::max(g.my, g.mz) - 2 + 7) / 8, 3);
     const double *sts = series_surface(C);
-    const double *dit = C->d_scal + SC_IT, its = (double)C->cfg.it_start;
-    TG_PROF(C, "teqn_bcs", k_t_bcs<<<g2(g.my, g.mz), b2, 0, C->stream>>>(g, C->m, C->prm, C->s.tmprt, 0, sts, dit, its));
-    TG_PROF(C, "teqn_bcs", k_t_bcs<<<g2(g.mx, g.mz), b2, 0, C->stream>>>(g, C->m, C->prm, C->s.tmprt, 1, sts, dit, its));
-    TG_PROF(C, "teqn_bcs", k_t_bcs<<<g2(g.mx, g.my), b2, 0, C->stream>>>(g, C->m, C->prm, C->s.tmprt, 2, sts, dit, its));
+    TG_PROF(C, "teqn_bcs", k_t_bcs<<<gr, b2, 0, C->stream>>>(g, C->m, C->prm, C->s.tmprt, sts, C->d_scal + SC_IT, (double)C->cfg.it_start));
+}
+
+void refresh_teqn_mesh(tg_ctx *C)
+{
+    if (!C->prm.teqn || !C->prm.les) return;
+    k_t_width<<<nblk(C->g.size()), 256, 0, C->stream>>>(C->g, C->m, C->s.trd2);
+    TG_CUDA(cudaGetLastError());
 }
 
 }  // namespace tg
