@@ -335,7 +335,7 @@ __device__ __forceinline__ void wall_parallel(Grid g, Metrics m, State s, int k,
 
 // sums of |U_par|, the wall distance and (coupled) qWall over the j=1 plane, and
 // in the last block u* = uStarShumann(<|U_par|>, <s>, <qWall>) into out[2] (a
-// separate one-thread launch walked the 148 partials in 11 us)
+// separate launch walked the 148 partials in one thread)
 __global__ void __launch_bounds__(256) k_wall_plane_sums(Grid g, Metrics m, State s, Params p, double *part, unsigned *count, double *out)
 {
     int nI = g.mx - 2, nK = g.mz - 2;

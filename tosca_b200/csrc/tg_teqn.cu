@@ -45,8 +45,8 @@ __device__ __forceinline__ double weno3(double f0, double f1, double f2, double 
 // derivative. With Smagorinsky, nu_t / Pr_t with Pr_t = 1 / (1 + 2 l/delta)
 // and, in stable stratification, l/delta = min(1, 7.6 nu_t sqrt(tRef/|g
 // dT/deta|) / delta^2), delta = (1/ajc)^(1/3): evaluated as nu_t (1 + 2
-// l/delta) with rd2 = 1/delta^2 from the mesh (k_t_width: a cube root per face
-// and stage was a tenth of the kernel) and one reciprocal square root
+// l/delta) with rd2 = 1/delta^2 from the mesh (k_t_width: no cube root per face
+// and stage) and one reciprocal square root
 __device__ __forceinline__ double kappa_eff(const Params &p, double nut, double dtde, double rd2, double sqt)
 {
     if (!p.les) return p.nu / p.prandtl;
