@@ -390,7 +390,7 @@ void grad_p_tensor(tg_ctx *C);
 void form_fp_tensor(tg_ctx *C, int mode);      // FormU passes 1 and 2, central convection
 void stage_fp_tensor(tg_ctx *C);               // an explicit stage's fp from Ucont
 void stage_tail_tensor(tg_ctx *C);             // boundary planes after the last such stage
-void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk);
+void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk, bool from_p = false);
 // phi, p (less *ref if given) and the projected Ucont from the compact solution x
 void pressure_project_tensor(tg_ctx *C, const double *x, const double *ref);
 void contra_div_tensor(tg_ctx *C);             // final Ucat and the partial divergence maxima (C->d_red, red_blocks)

@@ -1419,7 +1419,7 @@ static void explicit_rhs_update(tg_ctx *C, RkArgs rk, bool from_ucont)
     if (from_ucont) {
         stage_fp_tensor(C);
         clear_rhs(C);
-        rhs_faces<2>(C, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0, rk);
+        rhs_faces_tensor(C, 2, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0, rk, true);
         return;
     }
     explicit_rhs_head(C, 0);

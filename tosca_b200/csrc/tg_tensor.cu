@@ -97,21 +97,24 @@ __global__ void k_smagorinsky_tensor(Grid g, Tensor t, State s, double cs)
 }
 
 // ------------------------------------------------------------------ GradP
-// k_grad_p (peqn.c:3437-3773)
+// k_grad_p (peqn.c:3437-3773) at the + faces of interior cell c
+__device__ __forceinline__ R3<double> grad_p_cell(const Grid &g, const Tensor &t, const double *p, int k, int j, int i, int c)
+{
+    const int pl = g.mx * g.my;
+    const double dx = t.dx[k], dy = t.dy[i], dz = t.dz[j], pc = p[c];
+    // the + neighbours lie inside the DMDA except across a periodic seam, where
+    // index m + 1 wraps to 1
+    const double pi = i == g.mx - 2 ? p[g.pi ? g.lin(k, j, 1) : c] : p[c + 1];
+    const double pj = j == g.my - 2 ? p[g.pj ? g.lin(k, 1, i) : c] : p[c + g.mx];
+    const double pk = k == g.mz - 2 ? p[g.pk ? g.lin(1, j, i) : c] : p[c + pl];
+    return R3<double>{(pi - pc) * (dx * dz * t.rdyf[i]), (pj - pc) * (dx * dy * t.rdzf[j]), (pk - pc) * (dy * dz * t.rdxf[k])};
+}
 __global__ void k_grad_p_tensor(Grid g, Tensor t, State s)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
-    const int c = g.lin(k, j, i), pl = g.mx * g.my;
-    const double dx = t.dx[k], dy = t.dy[i], dz = t.dz[j], pc = s.p[c];
-    // the + neighbours lie inside the DMDA except across a periodic seam, where
-    // index m + 1 wraps to 1
-    const double pi = i == g.mx - 2 ? s.p[g.pi ? g.lin(k, j, 1) : c] : s.p[c + 1];
-    const double pj = j == g.my - 2 ? s.p[g.pj ? g.lin(k, 1, i) : c] : s.p[c + g.mx];
-    const double pk = k == g.mz - 2 ? s.p[g.pk ? g.lin(1, j, i) : c] : s.p[c + pl];
-    s.dp.x[c] = (pi - pc) * (dx * dz * t.rdyf[i]);
-    s.dp.y[c] = (pj - pc) * (dx * dy * t.rdzf[j]);
-    s.dp.z[c] = (pk - pc) * (dy * dz * t.rdxf[k]);
+    const int c = g.lin(k, j, i);
+    st3(s.dp, c, grad_p_cell(g, t, s.p, k, j, i, c));
 }
 
 // ------------------------------------------------- FormU: cell budgets
@@ -735,8 +738,11 @@ __global__ void __launch_bounds__(256) k_stage_tail(const __grid_constant__ Grid
 // face value scale * aj_face * central(S . fp) needs one component of fp at
 // the two cells of the face, weighted by the inverse distance across it.
 // kind as there: 0 R += scale FormU; 1 ExplicitRhsU stored in R; 2 masked at
-// the non-resolved faces and applied by the explicit update.
-template <int kind>
+// the non-resolved faces and applied by the explicit update. from_p: dP is
+// formed again from p (the same products; a stage of a step, where dP is that of
+// p), one value and its neighbours instead of three: a step of 256 x 256 x 128
+// 3.125 -> 3.098 ms, of 192 x 128 x 64 0.825 -> 0.818 ms.
+template <int kind, bool from_p>
 __global__ void __launch_bounds__(256, 8) k_rhs_tensor(Grid g, Tensor t, State s, V3f<double> fp, V3f<double> R, double scale, Params p, int ab2, RkArgs rk)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -746,7 +752,8 @@ __global__ void __launch_bounds__(256, 8) k_rhs_tensor(Grid g, Tensor t, State s
     if (kind == 0) {
         o = ld3(R, c);
     } else {
-        o = R3<double>{0.0 - s.dp.x[c], 0.0 - s.dp.y[c], 0.0 - s.dp.z[c]};
+        const R3<double> dp = from_p ? grad_p_cell(g, t, s.p, k, j, i, c) : ld3(s.dp, c);
+        o = R3<double>{0.0 - dp.x, 0.0 - dp.y, 0.0 - dp.z};
         if (p.buoyancy) {
             const R3<double> b = ld3(s.btheta, c);
             if (ab2) { o = o + (3.0 / 2.0) * b; o = o + (-1.0 / 2.0) * ld3(s.btheta_o, c); }
@@ -1002,13 +1009,17 @@ void stage_tail_tensor(tg_ctx *C)
     const dim3 gr((std::max(g.mx, g.my) + 31) / 32, (std::max(g.my, g.mz) + 7) / 8, 6);
     TG_PROF(C, "stage_tail", k_stage_tail<<<gr, dim3(32, 8), 0, C->stream>>>(g, C->ts, C->s, C->prm));
 }
-void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk)
+void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk, bool from_p)
 {
     const Grid g = C->g;
     const V3f<double> fp = C->fw64.fp;
-    if (kind == 0) TG_PROF(C, "formu_rhs_faces", k_rhs_tensor<0><<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
-    else if (kind == 1) TG_PROF(C, "formu_rhs_faces", k_rhs_tensor<1><<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
-    else TG_PROF(C, "formu_rhs_faces", k_rhs_tensor<2><<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
+    auto go = [&](auto kernel) {
+        TG_PROF(C, "formu_rhs_faces", kernel<<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
+    };
+    if (kind == 0) go(k_rhs_tensor<0, false>);
+    else if (kind == 1) go(k_rhs_tensor<1, false>);
+    else if (from_p) go(k_rhs_tensor<2, true>);
+    else go(k_rhs_tensor<2, false>);
 }
 void pressure_project_tensor(tg_ctx *C, const double *x, const double *ref)
 {
