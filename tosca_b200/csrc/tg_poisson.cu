@@ -102,83 +102,53 @@ __global__ void k_apply7(PoissonCtx P, const double *__restrict__ x, double *__r
 
 enum { CP, EP, WP, NP, SP, TP, BP, NE, SE, NW, SW, TN, BN, TS, BS, TE, BE, TW, BW, NST };
 
-// 19 coefficients of one row of SetCoeffMatrix (peqn.c:889-1388)
-__device__ void row19(const PoissonCtx &P, const Cg &q, int ic, int jc, int kc, double vol[NST])
+// 19 coefficients of one row of SetCoeffMatrix (peqn.c:889-1388). The derivative
+// of a face value along a tangential direction is
+//     hi (x_+ + ..) + own (x_0 + ..) - lo (x_- + ..)
+// with weights of the cell's position in that direction: 1/4, 0, 1/4 inside,
+// 0, 1/2, 1/2 at the last cell and 1/2, -1/2, 0 at the first (the last wins in
+// a direction of one cell). Weights instead of the reference's branches: every
+// lane of a warp runs the same 90 products where rows that meet a domain end
+// used to run the interior and the end branches one after the other.
+struct CrossW {
+    double hi, own, lo;
+    __device__ __forceinline__ CrossW(int l, int n)
+    {
+        const bool last = l == n - 1, first = l == 0 && !last;
+        hi = last ? 0.0 : first ? 0.5 : 0.25;
+        own = last ? 0.5 : first ? -0.5 : 0.0;
+        lo = first ? 0.0 : last ? 0.5 : 0.25;
+    }
+};
+__device__ __forceinline__ void row19(const PoissonCtx &P, const Cg &q, int ic, int jc, int kc, double (&vol)[NST])
 {
+    #pragma unroll
     for (int m = 0; m < NST; m++) vol[m] = 0.0;
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const bool jr = jc == ny - 1, jl = jc == 0, kr = kc == nz - 1, kl = kc == 0, ir = ic == nx - 1, il = ic == 0;
-    int c = (kc * ny + jc) * nx + ic;
-    if (!ir || P.pi) {   // east
-        double a = P.gE1[c], b = P.gE2[c], cc = P.gE3[c];
-        vol[CP] -= a; vol[EP] += a;
-        if (jr)      { vol[CP] += b * 0.5; vol[EP] += b * 0.5; vol[SP] -= b * 0.5; vol[SE] -= b * 0.5; }
-        else if (jl) { vol[NP] += b * 0.5; vol[NE] += b * 0.5; vol[CP] -= b * 0.5; vol[EP] -= b * 0.5; }
-        else         { vol[NP] += b * 0.25; vol[NE] += b * 0.25; vol[SP] -= b * 0.25; vol[SE] -= b * 0.25; }
-        if (kr)      { vol[CP] += cc * 0.5; vol[EP] += cc * 0.5; vol[BP] -= cc * 0.5; vol[BE] -= cc * 0.5; }
-        else if (kl) { vol[TP] += cc * 0.5; vol[TE] += cc * 0.5; vol[CP] -= cc * 0.5; vol[EP] -= cc * 0.5; }
-        else         { vol[TP] += cc * 0.25; vol[TE] += cc * 0.25; vol[BP] -= cc * 0.25; vol[BE] -= cc * 0.25; }
-    }
-    if (!il || P.pi) {   // west
-        int w = q.id(kc, jc, ic - 1);
-        double a = P.gE1[w], b = P.gE2[w], cc = P.gE3[w];
-        vol[CP] -= a; vol[WP] += a;
-        if (jr)      { vol[CP] -= b * 0.5; vol[WP] -= b * 0.5; vol[SP] += b * 0.5; vol[SW] += b * 0.5; }
-        else if (jl) { vol[NP] -= b * 0.5; vol[NW] -= b * 0.5; vol[CP] += b * 0.5; vol[WP] += b * 0.5; }
-        else         { vol[NP] -= b * 0.25; vol[NW] -= b * 0.25; vol[SP] += b * 0.25; vol[SW] += b * 0.25; }
-        if (kr)      { vol[CP] -= cc * 0.5; vol[WP] -= cc * 0.5; vol[BP] += cc * 0.5; vol[BW] += cc * 0.5; }
-        else if (kl) { vol[TP] -= cc * 0.5; vol[TW] -= cc * 0.5; vol[CP] += cc * 0.5; vol[WP] += cc * 0.5; }
-        else         { vol[TP] -= cc * 0.25; vol[TW] -= cc * 0.25; vol[BP] += cc * 0.25; vol[BW] += cc * 0.25; }
-    }
-    if (!jr || P.pj) {   // north
-        double a = P.gN1[c], b = P.gN2[c], cc = P.gN3[c];
-        if (ir)      { vol[CP] += a * 0.5; vol[NP] += a * 0.5; vol[WP] -= a * 0.5; vol[NW] -= a * 0.5; }
-        else if (il) { vol[EP] += a * 0.5; vol[NE] += a * 0.5; vol[CP] -= a * 0.5; vol[NP] -= a * 0.5; }
-        else         { vol[EP] += a * 0.25; vol[NE] += a * 0.25; vol[WP] -= a * 0.25; vol[NW] -= a * 0.25; }
-        vol[CP] -= b; vol[NP] += b;
-        if (kr)      { vol[CP] += cc * 0.5; vol[NP] += cc * 0.5; vol[BP] -= cc * 0.5; vol[BN] -= cc * 0.5; }
-        else if (kl) { vol[TP] += cc * 0.5; vol[TN] += cc * 0.5; vol[CP] -= cc * 0.5; vol[NP] -= cc * 0.5; }
-        else         { vol[TP] += cc * 0.25; vol[TN] += cc * 0.25; vol[BP] -= cc * 0.25; vol[BN] -= cc * 0.25; }
-    }
-    if (!jl || P.pj) {   // south
-        int s = q.id(kc, jc - 1, ic);
-        double a = P.gN1[s], b = P.gN2[s], cc = P.gN3[s];
-        if (ir)      { vol[CP] -= a * 0.5; vol[SP] -= a * 0.5; vol[WP] += a * 0.5; vol[SW] += a * 0.5; }
-        else if (il) { vol[EP] -= a * 0.5; vol[SE] -= a * 0.5; vol[CP] += a * 0.5; vol[SP] += a * 0.5; }
-        else         { vol[EP] -= a * 0.25; vol[SE] -= a * 0.25; vol[WP] += a * 0.25; vol[SW] += a * 0.25; }
-        vol[CP] -= b; vol[SP] += b;
-        if (kr)      { vol[CP] -= cc * 0.5; vol[SP] -= cc * 0.5; vol[BP] += cc * 0.5; vol[BS] += cc * 0.5; }
-        else if (kl) { vol[TP] -= cc * 0.5; vol[TS] -= cc * 0.5; vol[CP] += cc * 0.5; vol[SP] += cc * 0.5; }
-        else         { vol[TP] -= cc * 0.25; vol[TS] -= cc * 0.25; vol[BP] += cc * 0.25; vol[BS] += cc * 0.25; }
-    }
-    if (!kr || P.pk) {   // top
-        double a = P.gT1[c], b = P.gT2[c], cc = P.gT3[c];
-        if (ir)      { vol[CP] += a * 0.5; vol[TP] += a * 0.5; vol[WP] -= a * 0.5; vol[TW] -= a * 0.5; }
-        else if (il) { vol[EP] += a * 0.5; vol[TE] += a * 0.5; vol[CP] -= a * 0.5; vol[TP] -= a * 0.5; }
-        else         { vol[EP] += a * 0.25; vol[TE] += a * 0.25; vol[WP] -= a * 0.25; vol[TW] -= a * 0.25; }
-        if (jr)      { vol[CP] += b * 0.5; vol[TP] += b * 0.5; vol[SP] -= b * 0.5; vol[TS] -= b * 0.5; }
-        else if (jl) { vol[NP] += b * 0.5; vol[TN] += b * 0.5; vol[CP] -= b * 0.5; vol[TP] -= b * 0.5; }
-        else         { vol[NP] += b * 0.25; vol[TN] += b * 0.25; vol[SP] -= b * 0.25; vol[TS] -= b * 0.25; }
-        vol[CP] -= cc; vol[TP] += cc;
-    }
-    if (!kl || P.pk) {   // bottom
-        int bb = q.id(kc - 1, jc, ic);
-        double a = P.gT1[bb], b = P.gT2[bb], cc = P.gT3[bb];
-        if (ir)      { vol[CP] -= a * 0.5; vol[BP] -= a * 0.5; vol[WP] += a * 0.5; vol[BW] += a * 0.5; }
-        else if (il) { vol[EP] -= a * 0.5; vol[BE] -= a * 0.5; vol[CP] += a * 0.5; vol[BP] += a * 0.5; }
-        else         { vol[EP] -= a * 0.25; vol[BE] -= a * 0.25; vol[WP] += a * 0.25; vol[BW] += a * 0.25; }
-        if (jr)      { vol[CP] -= b * 0.5; vol[BP] -= b * 0.5; vol[SP] += b * 0.5; vol[BS] += b * 0.5; }
-        else if (jl) { vol[NP] -= b * 0.5; vol[BN] -= b * 0.5; vol[CP] += b * 0.5; vol[BP] += b * 0.5; }
-        else         { vol[NP] -= b * 0.25; vol[BN] -= b * 0.25; vol[SP] += b * 0.25; vol[BS] += b * 0.25; }
-        vol[CP] -= cc; vol[BP] += cc;
-    }
+    const int nx = P.nx, ny = P.ny, nz = P.nz, c = (kc * ny + jc) * nx + ic;
+    const CrossW wi(ic, nx), wj(jc, ny), wk(kc, nz);
+    // tangential term t of a face whose other cell is `nb`: `pi`/`mi` the + and -
+    // neighbours of this cell along the tangent, `pn`/`mn` those of `nb`
+    auto cross = [&](double t, const CrossW &w, int nb, int pi, int pn, int mi, int mn) {
+        vol[CP] += t * w.own; vol[nb] += t * w.own;
+        vol[pi] += t * w.hi; vol[pn] += t * w.hi;
+        vol[mi] -= t * w.lo; vol[mn] -= t * w.lo;
+    };
+    // face f of this cell (on: it carries a flux; sg: +1 for its + side)
+    auto face = [&](bool on, const double *gn, const double *gt1, const double *gt2, int f, double sg, int nb, const CrossW &w1, int p1, int pn1,
+                    int m1, int mn1, const CrossW &w2, int p2, int pn2, int m2, int mn2) {
+        if (!on) return;
+        const double a = gn[f];
+        vol[CP] -= a; vol[nb] += a;
+        cross(sg * gt1[f], w1, nb, p1, pn1, m1, mn1);
+        cross(sg * gt2[f], w2, nb, p2, pn2, m2, mn2);
+    };
+    face(ic < nx - 1 || P.pi, P.gE1, P.gE2, P.gE3, c, 1.0, EP, wj, NP, NE, SP, SE, wk, TP, TE, BP, BE);
+    face(ic > 0 || P.pi, P.gE1, P.gE2, P.gE3, q.id(kc, jc, ic - 1), -1.0, WP, wj, NP, NW, SP, SW, wk, TP, TW, BP, BW);
+    face(jc < ny - 1 || P.pj, P.gN2, P.gN1, P.gN3, c, 1.0, NP, wi, EP, NE, WP, NW, wk, TP, TN, BP, BN);
+    face(jc > 0 || P.pj, P.gN2, P.gN1, P.gN3, q.id(kc, jc - 1, ic), -1.0, SP, wi, EP, SE, WP, SW, wk, TP, TS, BP, BS);
+    face(kc < nz - 1 || P.pk, P.gT3, P.gT1, P.gT2, c, 1.0, TP, wi, EP, TE, WP, TW, wj, NP, TN, SP, TS);
+    face(kc > 0 || P.pk, P.gT3, P.gT1, P.gT2, q.id(kc - 1, jc, ic), -1.0, BP, wi, EP, BE, WP, BW, wj, NP, BN, SP, BS);
 }
-
-__constant__ int c_off[NST][3] = {   // (dk, dj, di) of each stencil point
-    {0,0,0},{0,0,1},{0,0,-1},{0,1,0},{0,-1,0},{1,0,0},{-1,0,0},
-    {0,1,1},{0,-1,1},{0,1,-1},{0,-1,-1},
-    {1,1,0},{-1,1,0},{1,-1,0},{-1,-1,0},
-    {1,0,1},{-1,0,1},{1,0,-1},{-1,0,-1}};
 
 // 19-point: y = -(A x) on non-pinned rows (entries |v| <= 1e-10 dropped as
 // at peqn.c:1410-1418), y = x on the pinned row
@@ -191,13 +161,19 @@ __global__ void k_apply19(PoissonCtx P, const double *__restrict__ x, double *__
     if (c == P.pin) { y[c] = x[c]; return; }
     double vol[NST];
     row19(P, q, ic, jc, kc, vol);
-    double acc = 0.0;
-    #pragma unroll
-    for (int m = 0; m < NST; m++) {
-        int kk = kc + c_off[m][0], jj = jc + c_off[m][1], ii = ic + c_off[m][2];
-        if (m != CP && (!(fabs(vol[m]) > 1.e-10) || !q.in(kk, jj, ii))) continue;
-        acc += vol[m] * x[q.id(kk, jj, ii)];
-    }
+    // the wrapped row and plane offsets once; a neighbour outside the domain has a
+    // zero coefficient (its face carries no flux and its tangential weight is zero)
+    // and reads the cell itself
+    const int pl = P.nx * P.ny;
+    const int ie = ic < P.nx - 1 ? 1 : P.pi ? 1 - P.nx : 0, iw = ic > 0 ? -1 : P.pi ? P.nx - 1 : 0;
+    const int jn = jc < P.ny - 1 ? P.nx : P.pj ? P.nx - pl : 0, js = jc > 0 ? -P.nx : P.pj ? pl - P.nx : 0;
+    const int kt = kc < P.nz - 1 ? pl : P.pk ? pl - pl * P.nz : 0, kb = kc > 0 ? -pl : P.pk ? pl * P.nz - pl : 0;
+    double acc = vol[CP] * x[c];
+    auto add = [&](int m, int o) { if (fabs(vol[m]) > 1.e-10) acc += vol[m] * x[c + o]; };
+    add(EP, ie); add(WP, iw); add(NP, jn); add(SP, js); add(TP, kt); add(BP, kb);
+    add(NE, jn + ie); add(SE, js + ie); add(NW, jn + iw); add(SW, js + iw);
+    add(TN, kt + jn); add(BN, kb + jn); add(TS, kt + js); add(BS, kb + js);
+    add(TE, kt + ie); add(BE, kb + ie); add(TW, kt + iw); add(BW, kb + iw);
     y[c] = -acc;
 }
 
