@@ -458,6 +458,7 @@ tg_status tg_set_field(tg_ctx *C, int32_t w, const double *host, int32_t halo)
         if (w == TG_F_DP) C->clear_dp = true;
         if ((w >= TG_F_CSI && w <= TG_F_KZET) || (w >= TG_F_AJ && w <= TG_F_KAJ)) {
             C->met32_stale = true;
+            refresh_gtensor(C);
             if (w >= TG_F_AJ) refresh_teqn_mesh(C);
             if (C->axis_aligned) {         // the caller's metrics need not be those of a mesh of planes
                 C->axis_aligned = false;

@@ -217,8 +217,6 @@ struct tg_ctx {
         bool flux32 = false;         // FormU face-flux planes stored in FP32
         bool rhs32 = false;          // FormU face assembly metrics
         bool smag32 = false;         // Smagorinsky eddy viscosity
-        bool gradp32 = false;        // GradP
-        bool proj32 = false;         // ProjectVelocity (FP64 arithmetic)
     } pol;
     bool met32_stale = true;             // metrics changed since the FP32 copies were made
     tg::FaceMet<double> fm64{};
@@ -397,6 +395,7 @@ void contra_div_tensor(tg_ctx *C);             // final Ucat and the partial div
 
 // stage entry points (tg_step.cu)
 void metrics_from_nodes(tg_ctx *C, const double *d_nodes);
+void refresh_gtensor(tg_ctx *C);              // g11 .. g33 from the face metrics
 void alloc_precision_work(tg_ctx *C);         // FP64 views, FP32 copies (mixed mode)
 void refresh_met32(tg_ctx *C);
 void refresh_filter(tg_ctx *C);          // FP64 Smagorinsky filter widths after a mesh change                // FP32 metric copies from the FP64 fields

@@ -200,6 +200,13 @@ __global__ void k_gtensor(Grid g, Metrics m)
 
 }  // namespace
 
+void refresh_gtensor(tg_ctx *C)
+{
+    const Grid g = C->g;
+    k_gtensor<<<grid3(g.mx, g.my, g.mz), block3(), 0, C->stream>>>(g, C->m);
+    TG_CUDA(cudaGetLastError());
+}
+
 void metrics_from_nodes(tg_ctx *C, const double *d_nodes)
 {
     const Grid g = C->g;

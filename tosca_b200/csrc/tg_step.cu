@@ -422,8 +422,13 @@ __global__ void k_wall_stress(Grid g, Metrics m, State s, Params p, const double
 // buoyancy sum +3/2 b - 1/2 b_o reads -3/2 ghGradRhok + 1/2 ghGradRhok_o
 // (ueqn_solvers.c:1314-1324); the products are associated as (g z) (grad .
 // S) aj, the reference's g z (grad . S) aj up to rounding
-template <class M, bool GH = false>
-__global__ void k_grad_p(Grid g, FaceMet<M> m, State s, const double *node_z = nullptr, double t_ref = 0.0)
+//
+// The nine products of the face metric tensor with the face Jacobian are read
+// from SetCoeffMatrix's arrays (at the faces of interior cells they are those of
+// the face itself) in FP64 in both modes: 72 bytes per cell instead of 240, or
+// 120 in FP32.
+template <bool GH>
+__global__ void k_grad_p(Grid g, Metrics m, State s, const double *node_z = nullptr, double t_ref = 0.0)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
@@ -433,14 +438,7 @@ __global__ void k_grad_p(Grid g, FaceMet<M> m, State s, const double *node_z = n
         return GH ? (t_ref - v) / t_ref : v;
     };
     const int mx = g.mx, my = g.my, mz = g.mz;
-    R3<M> ic = ld3(m.icsi, c), ie = ld3(m.ieta, c), iz = ld3(m.izet, c);
-    R3<M> jc = ld3(m.jcsi, c), je = ld3(m.jeta, c), jz = ld3(m.jzet, c);
-    R3<M> kc = ld3(m.kcsi, c), ke = ld3(m.keta, c), kz = ld3(m.kzet, c);
-    M g11 = dot3(ic, ic), g12 = dot3(ie, ic), g13 = dot3(iz, ic);
-    M g21 = dot3(jc, je), g22 = dot3(je, je), g23 = dot3(jz, je);
-    M g31 = dot3(kc, kz), g32 = dot3(ke, kz), g33 = dot3(kz, kz);
-    double dpdc, dpde, dpdz;
-    M ox, oy, oz;
+    double dpdc, dpde, dpdz, ox, oy, oz;
     dpdc = (i == mx - 2 && g.pi) ? P(k, j, mx + 1) - P(k, j, i) : P(k, j, i + 1) - P(k, j, i);
     if (j == my - 2 && i == mx - 2)  dpde = (P(k, j, i) - P(k, j - 1, i) + P(k, j, i + 1) - P(k, j - 1, i + 1)) * 0.5;
     else if (j == 1 && i == mx - 2)  dpde = (P(k, j + 1, i) - P(k, j, i) + P(k, j + 1, i + 1) - P(k, j, i + 1)) * 0.5;
@@ -448,7 +446,7 @@ __global__ void k_grad_p(Grid g, FaceMet<M> m, State s, const double *node_z = n
     if (k == mz - 2 && i == mx - 2)  dpdz = (P(k, j, i) - P(k - 1, j, i) + P(k, j, i + 1) - P(k - 1, j, i + 1)) * 0.5;
     else if (k == 1 && i == mx - 2)  dpdz = (P(k + 1, j, i) - P(k, j, i) + P(k + 1, j, i + 1) - P(k, j, i + 1)) * 0.5;
     else                             dpdz = (P(k + 1, j, i) - P(k - 1, j, i) + P(k + 1, j, i + 1) - P(k - 1, j, i + 1)) * 0.25;
-    ox = ((M)dpdc * g11 + (M)dpde * g12 + (M)dpdz * g13) * m.iaj[c];
+    ox = dpdc * m.g11[c] + dpde * m.g12[c] + dpdz * m.g13[c];
     if (i == mx - 2 && j == my - 2)  dpdc = (P(k, j, i) - P(k, j, i - 1) + P(k, j + 1, i) - P(k, j + 1, i - 1)) * 0.5;
     else if (i == 1 && j == my - 2)  dpdc = (P(k, j, i + 1) - P(k, j, i) + P(k, j + 1, i + 1) - P(k, j + 1, i)) * 0.5;
     else                             dpdc = (P(k, j, i + 1) - P(k, j, i - 1) + P(k, j + 1, i + 1) - P(k, j + 1, i - 1)) * 0.25;
@@ -456,7 +454,7 @@ __global__ void k_grad_p(Grid g, FaceMet<M> m, State s, const double *node_z = n
     if (k == mz - 2 && j == my - 2)  dpdz = (P(k, j, i) - P(k - 1, j, i) + P(k, j + 1, i) - P(k - 1, j + 1, i)) * 0.5;
     else if (k == 1 && j == my - 2)  dpdz = (P(k + 1, j, i) - P(k, j, i) + P(k + 1, j + 1, i) - P(k, j + 1, i)) * 0.5;
     else                             dpdz = (P(k + 1, j, i) - P(k - 1, j, i) + P(k + 1, j + 1, i) - P(k - 1, j + 1, i)) * 0.25;
-    oy = ((M)dpdc * g21 + (M)dpde * g22 + (M)dpdz * g23) * m.jaj[c];
+    oy = dpdc * m.g21[c] + dpde * m.g22[c] + dpdz * m.g23[c];
     if (i == mx - 2 && k == mz - 2)  dpdc = (P(k, j, i) - P(k, j, i - 1) + P(k + 1, j, i) - P(k + 1, j, i - 1)) * 0.5;
     else if (i == 1 && k == mz - 2)  dpdc = (P(k, j, i + 1) - P(k, j, i) + P(k + 1, j, i + 1) - P(k + 1, j, i)) * 0.5;
     else                             dpdc = (P(k, j, i + 1) - P(k, j, i - 1) + P(k + 1, j, i + 1) - P(k + 1, j, i - 1)) * 0.25;
@@ -464,16 +462,16 @@ __global__ void k_grad_p(Grid g, FaceMet<M> m, State s, const double *node_z = n
     else if (j == 1 && k == mz - 2)  dpde = (P(k, j + 1, i) - P(k, j, i) + P(k + 1, j + 1, i) - P(k + 1, j, i)) * 0.5;
     else                             dpde = (P(k, j + 1, i) - P(k, j - 1, i) + P(k + 1, j + 1, i) - P(k + 1, j - 1, i)) * 0.25;
     dpdz = (k == mz - 2 && g.pk) ? P(mz + 1, j, i) - P(k, j, i) : P(k + 1, j, i) - P(k, j, i);
-    oz = ((M)dpdc * g31 + (M)dpde * g32 + (M)dpdz * g33) * m.kaj[c];
+    oz = dpdc * m.g31[c] + dpde * m.g32[c] + dpdz * m.g33[c];
     if (!g.pi && i == mx - 2) ox = 0;
     if (!g.pj && j == my - 2) oy = 0;
     if (!g.pk && k == mz - 2) oz = 0;
     if (GH) {
         const double gz = -9.81 * node_z[c];
-        s.btheta.x[c] = -(gz * (double)ox); s.btheta.y[c] = -(gz * (double)oy); s.btheta.z[c] = -(gz * (double)oz);
+        s.btheta.x[c] = -(gz * ox); s.btheta.y[c] = -(gz * oy); s.btheta.z[c] = -(gz * oz);
         return;
     }
-    s.dp.x[c] = (double)ox; s.dp.y[c] = (double)oy; s.dp.z[c] = (double)oz;
+    s.dp.x[c] = ox; s.dp.y[c] = oy; s.dp.z[c] = oz;
 }
 
 // ------------------------------------------------------------------------
@@ -992,10 +990,11 @@ __global__ void k_non_resolved(Grid g, State s, Params p)
 
 // ------------------------------------------------------------------------
 // ProjectVelocity (peqn.c:2495-2905): V = V* - dt G(phi) with the full
-// metric tensor; faces 0 and m-2 skipped unless periodic.
+// metric tensor; faces 0 and m-2 skipped unless periodic. The tensor's products
+// with the face Jacobian are SetCoeffMatrix's own arrays, 9 values per cell where
+// the face metrics are 30.
 // ------------------------------------------------------------------------
-template <class M>
-__global__ void k_project(Grid g, FaceMet<M> m, State s, double dt)
+__global__ void k_project(Grid g, Metrics m, State s, double dt)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z * blockDim.z + threadIdx.z;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
@@ -1010,11 +1009,13 @@ __global__ void k_project(Grid g, FaceMet<M> m, State s, double dt)
         if (k == mz - 2)      dpdz = (F(k, j, i) + F(k, j, i + 1) - F(k - 1, j, i) - F(k - 1, j, i + 1)) * 0.5;
         else if (k == 1)      dpdz = (F(k + 1, j, i) + F(k + 1, j, i + 1) - F(k, j, i) - F(k, j, i + 1)) * 0.5;
         else                  dpdz = (F(k + 1, j, i) + F(k + 1, j, i + 1) - F(k - 1, j, i) - F(k - 1, j, i + 1)) * 0.25;
-        R3<double> c1 = cvta<double>(ld3(m.icsi, f)), e1 = cvta<double>(ld3(m.ieta, f)), z1 = cvta<double>(ld3(m.izet, f));
-        double a = (double)m.iaj[f];
-        s.ucont.x[f] -= (dpdc * (c1.x * c1.x + c1.y * c1.y + c1.z * c1.z) * a
-                       + dpde * (e1.x * c1.x + e1.y * c1.y + e1.z * c1.z) * a
-                       + dpdz * (z1.x * c1.x + z1.y * c1.y + z1.z * c1.z) * a) * dt;
+        double a = m.g11[f], b = m.g12[f], c = m.g13[f];
+        if (i == 0) {                // face 0 of a periodic direction has its own metrics
+            const R3<double> q = ld3(m.icsi, f);
+            const double w = m.iaj[f];
+            a = dot3(ld3(m.icsi, f), q) * w; b = dot3(ld3(m.ieta, f), q) * w; c = dot3(ld3(m.izet, f), q) * w;
+        }
+        s.ucont.x[f] -= (dpdc * a + dpde * b + dpdz * c) * dt;
     }
     if (i > 0 && k > 0 && ((j > 0 && j < my - 2) || g.pj)) {
         double dpdc, dpde = F(k, j + 1, i) - F(k, j, i), dpdz;
@@ -1024,11 +1025,13 @@ __global__ void k_project(Grid g, FaceMet<M> m, State s, double dt)
         if (k == mz - 2)      dpdz = (F(k, j, i) + F(k, j + 1, i) - F(k - 1, j, i) - F(k - 1, j + 1, i)) * 0.5;
         else if (k == 1)      dpdz = (F(k + 1, j, i) + F(k + 1, j + 1, i) - F(k, j, i) - F(k, j + 1, i)) * 0.5;
         else                  dpdz = (F(k + 1, j, i) + F(k + 1, j + 1, i) - F(k - 1, j, i) - F(k - 1, j + 1, i)) * 0.25;
-        R3<double> c2 = cvta<double>(ld3(m.jcsi, f)), e2 = cvta<double>(ld3(m.jeta, f)), z2 = cvta<double>(ld3(m.jzet, f));
-        double a = (double)m.jaj[f];
-        s.ucont.y[f] -= (dpdc * (c2.x * e2.x + c2.y * e2.y + c2.z * e2.z) * a
-                       + dpde * (e2.x * e2.x + e2.y * e2.y + e2.z * e2.z) * a
-                       + dpdz * (z2.x * e2.x + z2.y * e2.y + z2.z * e2.z) * a) * dt;
+        double a = m.g21[f], b = m.g22[f], c = m.g23[f];
+        if (j == 0) {                // face 0 of a periodic direction has its own metrics
+            const R3<double> q = ld3(m.jeta, f);
+            const double w = m.jaj[f];
+            a = dot3(ld3(m.jcsi, f), q) * w; b = dot3(ld3(m.jeta, f), q) * w; c = dot3(ld3(m.jzet, f), q) * w;
+        }
+        s.ucont.y[f] -= (dpdc * a + dpde * b + dpdz * c) * dt;
     }
     if (i > 0 && j > 0 && ((k > 0 && k < mz - 2) || g.pk)) {
         double dpdc, dpde, dpdz = F(k + 1, j, i) - F(k, j, i);
@@ -1038,11 +1041,13 @@ __global__ void k_project(Grid g, FaceMet<M> m, State s, double dt)
         if (j == my - 2)      dpde = (F(k, j, i) + F(k + 1, j, i) - F(k, j - 1, i) - F(k + 1, j - 1, i)) * 0.5;
         else if (j == 1)      dpde = (F(k, j + 1, i) + F(k + 1, j + 1, i) - F(k, j, i) - F(k + 1, j, i)) * 0.5;
         else                  dpde = (F(k, j + 1, i) + F(k + 1, j + 1, i) - F(k, j - 1, i) - F(k + 1, j - 1, i)) * 0.25;
-        R3<double> c3 = cvta<double>(ld3(m.kcsi, f)), e3 = cvta<double>(ld3(m.keta, f)), z3 = cvta<double>(ld3(m.kzet, f));
-        double a = (double)m.kaj[f];
-        s.ucont.z[f] -= (dpdc * (c3.x * z3.x + c3.y * z3.y + c3.z * z3.z) * a
-                       + dpde * (e3.x * z3.x + e3.y * z3.y + e3.z * z3.z) * a
-                       + dpdz * (z3.x * z3.x + z3.y * z3.y + z3.z * z3.z) * a) * dt;
+        double a = m.g31[f], b = m.g32[f], c = m.g33[f];
+        if (k == 0) {                // face 0 of a periodic direction has its own metrics
+            const R3<double> q = ld3(m.kzet, f);
+            const double w = m.kaj[f];
+            a = dot3(ld3(m.kcsi, f), q) * w; b = dot3(ld3(m.keta, f), q) * w; c = dot3(ld3(m.kzet, f), q) * w;
+        }
+        s.ucont.z[f] -= (dpdc * a + dpde * b + dpdz * c) * dt;
     }
 }
 
@@ -1161,8 +1166,6 @@ static void set_policy(tg_ctx *C)
     C->pol.flux32 = false;
     C->pol.rhs32 = C->mixed;
     C->pol.smag32 = C->mixed;
-    C->pol.gradp32 = C->mixed;
-    C->pol.proj32 = false;
 }
 
 // Smagorinsky filter width squared of every cell from its Jacobian, in the
@@ -1311,14 +1314,13 @@ void grad_p(tg_ctx *C)
     }
     refresh_met32(C);
     if (C->axis_aligned) grad_p_tensor(C);
-    else if (C->pol.gradp32) TG_PROF(C, "grad_p", k_grad_p<float><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
-    else TG_PROF(C, "grad_p", k_grad_p<double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
+    else TG_PROF(C, "grad_p", k_grad_p<false><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->m, C->s));
 }
 
 void buoyancy(tg_ctx *C)
 {
     if (C->cfg.p_tilde)   // ghGradRhoK (teqn.c:278), FP64
-        TG_PROF(C, "gh_grad_rhok", (k_grad_p<double, true><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s, C->node_z, C->prm.t_ref)));
+        TG_PROF(C, "gh_grad_rhok", (k_grad_p<true><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->m, C->s, C->node_z, C->prm.t_ref)));
     else
         k_buoyancy<<<ga(C->g), block3(), 0, C->stream>>>(C->g, C->m, C->s, C->prm);
 }
@@ -1551,9 +1553,7 @@ static bool pressure_update_and_project(tg_ctx *C, bool gauge)
     update_scalar_ghosts(C, C->s.phi);
     TG_PROF(C, "update_pressure", k_update_pressure<<<gi(g), block3(), 0, C->stream>>>(g, C->s));
     update_scalar_ghosts(C, C->s.p);
-    refresh_met32(C);
-    if (C->pol.proj32) TG_PROF(C, "project", k_project<float><<<gf(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm.dt));
-    else TG_PROF(C, "project", k_project<double><<<gf(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm.dt));
+    TG_PROF(C, "project", k_project<<<gf(g), block3(), 0, C->stream>>>(g, C->m, C->s, C->prm.dt));
     return false;
 }
 

@@ -82,7 +82,9 @@ __device__ __forceinline__ void stencil4(int i, int m, int per, int &L, int &R)
 // squared, and with aj a product of spacings (tg_tensor.cu, t), so no metric is
 // read; the cross terms are left out with the derivatives they multiply;
 // kappa_eff still reads the eta derivative of every face (the stability
-// correction of Pr_t). rd2: 1/delta^2 of the i, j and k faces (k_t_width), on a
+// correction of Pr_t). Elsewhere the products of the metric tensor with the face
+// Jacobian are SetCoeffMatrix's arrays (9 values per cell, the face metrics 30).
+// rd2: 1/delta^2 of the i, j and k faces (k_t_width), on a
 // mesh of planes a product of factors as well.
 constexpr int TBX = 32, TBY = 4, TBZ = 2, TBN = TBX * TBY * TBZ;
 constexpr int TTX = TBX + 3, TTY = TBY + 3, TTZ = TBZ + 3, TTN = TTX * TTY * TTZ;
@@ -160,11 +162,14 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, Tensor
         if (AX) {
             fl.x[f] = o + (t.dx[k] * t.dz[j] * t.rdyf[fi] * dtdc) * ke;
         } else {
-            const double ajc = m.iaj[f];
-            const R3<double> cs = ld3(m.icsi, f), et = ld3(m.ieta, f), ze = ld3(m.izet, f);
-            const double g11 = cs.x * cs.x + cs.y * cs.y + cs.z * cs.z, g21 = et.x * cs.x + et.y * cs.y + et.z * cs.z,
-                         g31 = ze.x * cs.x + ze.y * cs.y + ze.z * cs.z;
-            fl.x[f] = o + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
+            double a = 0.0, b = 0.0, c = 0.0;
+            if (e == 0) { a = m.g11[f]; b = m.g12[f]; c = m.g13[f]; }
+            else {                       // face 0 has its own metrics
+                const R3<double> n = ld3(m.icsi, f);
+                const double w = m.iaj[f];
+                a = dot3(ld3(m.icsi, f), n) * w; b = dot3(ld3(m.ieta, f), n) * w; c = dot3(ld3(m.izet, f), n) * w;
+            }
+            fl.x[f] = o + (a * dtdc + b * dtde + c * dtdz) * ke;
         }
     };
     // ---- j face fj = j + e (Compute_dscalar_j, inline.h:3252-3289)
@@ -206,11 +211,14 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, Tensor
         if (AX) {
             fl.y[f] = o + (v0 + (t.dx[k] * t.dy[i] * t.rdzf[fj] * dtde) * ke);
         } else {
-            const double ajc = m.jaj[f];
-            const R3<double> cs = ld3(m.jcsi, f), et = ld3(m.jeta, f), ze = ld3(m.jzet, f);
-            const double g11 = cs.x * et.x + cs.y * et.y + cs.z * et.z, g21 = et.x * et.x + et.y * et.y + et.z * et.z,
-                         g31 = ze.x * et.x + ze.y * et.y + ze.z * et.z;
-            fl.y[f] = o + (v0 + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke);
+            double a = 0.0, b = 0.0, c = 0.0;
+            if (e == 0) { a = m.g21[f]; b = m.g22[f]; c = m.g23[f]; }
+            else {                       // face 0 has its own metrics
+                const R3<double> n = ld3(m.jeta, f);
+                const double w = m.jaj[f];
+                a = dot3(ld3(m.jcsi, f), n) * w; b = dot3(ld3(m.jeta, f), n) * w; c = dot3(ld3(m.jzet, f), n) * w;
+            }
+            fl.y[f] = o + (v0 + (a * dtdc + b * dtde + c * dtdz) * ke);
         }
     };
     // ---- k face fk = k + e (Compute_dscalar_k, inline.h:3294-3331)
@@ -244,11 +252,14 @@ __global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, Tensor
         if (AX) {
             fl.z[f] = o + (t.dy[i] * t.dz[j] * t.rdxf[fk] * dtdz) * ke;
         } else {
-            const double ajc = m.kaj[f];
-            const R3<double> cs = ld3(m.kcsi, f), et = ld3(m.keta, f), ze = ld3(m.kzet, f);
-            const double g11 = cs.x * ze.x + cs.y * ze.y + cs.z * ze.z, g21 = et.x * ze.x + et.y * ze.y + et.z * ze.z,
-                         g31 = ze.x * ze.x + ze.y * ze.y + ze.z * ze.z;
-            fl.z[f] = o + (g11 * dtdc + g21 * dtde + g31 * dtdz) * ajc * ke;
+            double a = 0.0, b = 0.0, c = 0.0;
+            if (e == 0) { a = m.g31[f]; b = m.g32[f]; c = m.g33[f]; }
+            else {                       // face 0 has its own metrics
+                const R3<double> n = ld3(m.kzet, f);
+                const double w = m.kaj[f];
+                a = dot3(ld3(m.kcsi, f), n) * w; b = dot3(ld3(m.keta, f), n) * w; c = dot3(ld3(m.kzet, f), n) * w;
+            }
+            fl.z[f] = o + (a * dtdc + b * dtde + c * dtdz) * ke;
         }
     };
     const int ni = (i == 1 && npi) ? 2 : 1, nj = (j == 1 && npj) ? 2 : 1, nk = (k == 1 && npk) ? 2 : 1;
