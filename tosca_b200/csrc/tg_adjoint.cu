@@ -105,7 +105,6 @@ struct AdjState {
 namespace {
 
 constexpr int TB = 256;
-inline int nblk1(int64_t n) { int64_t b = (n + TB - 1) / TB; return (int)std::min<int64_t>(b, 148 * 16); }
 inline dim3 g2(int na, int nb) { return dim3((na + 31) / 32, (nb + 7) / 8); }
 const dim3 b2(32, 8);
 inline dim3 gall(const Grid &g) { return grid3(g.mx, g.my, g.mz); }
@@ -124,12 +123,6 @@ __device__ __forceinline__ bool interior(const Grid &g, int k, int j, int i)
 }
 
 // ------------------------------------------------------------- elementwise
-__global__ void k_axpy3(int64_t n, V3f<double> y, double a, V3f<double> x)
-{
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-        y.x[q] += a * x.x[q]; y.y[q] += a * x.y[q]; y.z[q] += a * x.z[q];
-    }
-}
 __global__ void k_sum_partial(int64_t n, const double *a, double *part)
 {
     __shared__ double sh[TB];
@@ -140,13 +133,13 @@ __global__ void k_sum_partial(int64_t n, const double *a, double *part)
     for (int w = TB / 2; w > 0; w >>= 1) { if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w]; __syncthreads(); }
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
-// syncPressure transpose: p_adj[ref] -= sum(p_adj)
-__global__ void k_gauge_adj(const double *part, int nb, double *pa, int ref)
+// syncPressure transpose: p_adj[ref] -= sum(p_adj), one block of TB threads
+__global__ void __launch_bounds__(TB) k_gauge_adj(const double *part, int nb, double *pa, int ref)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int b = 0; b < nb; b++) s += part[b];
-    pa[ref] -= s;
+    double s[1] = {0.0};
+    for (int b = threadIdx.x; b < nb; b += TB) s[0] += part[b];
+    block_reduce<TB>(s, RedSum{});
+    if (threadIdx.x == 0) pa[ref] -= s[0];
 }
 
 // ------------------------------------------------ periodic / ghost copies
@@ -216,25 +209,38 @@ __global__ void k_adj_nut_bcs(Grid g, double *na, Params p)
         aadd(na + src, v);
     }
 }
-// resetNoPenetrationFluxes: wall-normal faces of wall patches zeroed
-__global__ void k_adj_no_penetration(Grid g, V3f<double> a, Params p)
+// resetNoPenetrationFluxes: wall-normal faces of wall patches zeroed; SUM: and
+// the result added to sum, ghosts included (the two as one pass over a)
+template <bool SUM>
+__global__ void k_adj_no_penetration(Grid g, V3f<double> a, Params p, V3f<double> sum)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
+    if (i >= g.mx || j >= g.my || k >= g.mz) return;
     int q = g.lin(k, j, i);
-    if ((i == 0 && is_wall(p.bc[TG_ILEFT])) || (i == g.mx - 2 && is_wall(p.bc[TG_IRIGHT]))) a.x[q] = 0.0;
-    if ((j == 0 && is_wall(p.bc[TG_JLEFT])) || (j == g.my - 2 && is_wall(p.bc[TG_JRIGHT]))) a.y[q] = 0.0;
-    if ((k == 0 && is_wall(p.bc[TG_KLEFT])) || (k == g.mz - 2 && is_wall(p.bc[TG_KRIGHT]))) a.z[q] = 0.0;
+    const bool face = i <= g.mx - 2 && j <= g.my - 2 && k <= g.mz - 2;
+    const bool zx = face && ((i == 0 && is_wall(p.bc[TG_ILEFT])) || (i == g.mx - 2 && is_wall(p.bc[TG_IRIGHT])));
+    const bool zy = face && ((j == 0 && is_wall(p.bc[TG_JLEFT])) || (j == g.my - 2 && is_wall(p.bc[TG_JRIGHT])));
+    const bool zz = face && ((k == 0 && is_wall(p.bc[TG_KLEFT])) || (k == g.mz - 2 && is_wall(p.bc[TG_KRIGHT])));
+    if (zx) a.x[q] = 0.0; else if (SUM) sum.x[q] += a.x[q];
+    if (zy) a.y[q] = 0.0; else if (SUM) sum.y[q] += a.y[q];
+    if (zz) a.z[q] = 0.0; else if (SUM) sum.z[q] += a.z[q];
 }
 
 // ------------------------------------------------- contravariantToCartesian
-// (a) per interior cell: q_adj = M^-T ucat_adj (Cramer on the transpose), ucat_adj = 0
-__global__ void k_adj_contra_cells(Grid g, Metrics m, V3f<double> ca, V3f<double> qa)
+// (a) per interior cell: q_adj = M^-T ucat_adj (Cramer on the transpose), ucat_adj = 0;
+// SUM: the ghosts, which it leaves, are added to sum
+template <bool SUM>
+__global__ void k_adj_contra_cells(Grid g, Metrics m, V3f<double> ca, V3f<double> qa, V3f<double> sum)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
+    constexpr int o = SUM ? 0 : 1;
+    int i = blockIdx.x * blockDim.x + threadIdx.x + o, j = blockIdx.y * blockDim.y + threadIdx.y + o, k = blockIdx.z * blockDim.z + threadIdx.z + o;
+    if (i > g.mx - 2 + SUM || j > g.my - 2 + SUM || k > g.mz - 2 + SUM) return;
     int c = g.lin(k, j, i);
     R3<double> gv = ld3(ca, c);
+    if (SUM && !interior(g, k, j, i)) {
+        sum.x[c] += gv.x; sum.y[c] += gv.y; sum.z[c] += gv.z;
+        return;
+    }
     st3(ca, c, R3<double>{0.0, 0.0, 0.0});
     R3<double> s = ld3(m.csi, c), e = ld3(m.eta, c), z = ld3(m.zet, c);
     double a00 = s.x, a01 = e.x, a02 = z.x, a10 = s.y, a11 = e.y, a12 = z.y, a20 = s.z, a21 = e.z, a22 = z.z;
@@ -935,11 +941,22 @@ __global__ void __launch_bounds__(256) k_adj_wall_fwd(Grid g, Metrics m, V3f<dou
     }
     block_sum2(su, sd, part);
 }
-// wsc <- Umean, dist, u*, S, D, logLaw
-__global__ void k_adj_wall_fwd_final(Grid g, Params p, const double *part, double *wsc)
+// the two totals of the WNB block sums, in thread 0 of a block of 256 threads
+__device__ __forceinline__ void plane_totals(const double *part, double (&v)[2])
 {
-    double su = 0.0, sd = 0.0;
-    for (int b = 0; b < WNB; b++) { su += part[2 * b]; sd += part[2 * b + 1]; }
+    static_assert(WNB <= 256, "one block sum per thread");
+    const int b = threadIdx.x;
+    v[0] = b < WNB ? part[2 * b] : 0.0;
+    v[1] = b < WNB ? part[2 * b + 1] : 0.0;
+    block_reduce<256>(v, RedSum{}, RedSum{});
+}
+// wsc <- Umean, dist, u*, S, D, logLaw
+__global__ void __launch_bounds__(256) k_adj_wall_fwd_final(Grid g, Params p, const double *part, double *wsc)
+{
+    double v[2];
+    plane_totals(part, v);
+    if (threadIdx.x != 0) return;
+    const double su = v[0], sd = v[1];
     const double cnt = (double)(g.mx - 2) * (double)(g.mz - 2);
     const double Umean = su / cnt, dist = sd / cnt, logLaw = log(dist / p.z0);
     const double us = fmax(0.0, (p.kappa * Umean) / logLaw);
@@ -986,10 +1003,12 @@ __global__ void __launch_bounds__(256) k_adj_wall_local(Grid g, Metrics m, Param
     block_sum2(sa, da, part);
 }
 // wsc[6] <- adjoint of Umean
-__global__ void k_adj_wall_mean(Grid g, Params p, const double *part, double *wsc)
+__global__ void __launch_bounds__(256) k_adj_wall_mean(Grid g, Params p, const double *part, double *wsc)
 {
-    double sa = 0.0, da = 0.0;
-    for (int b = 0; b < WNB; b++) { sa += part[2 * b]; da += part[2 * b + 1]; }
+    double v[2];
+    plane_totals(part, v);
+    if (threadIdx.x != 0) return;
+    const double sa = v[0], da = v[1];
     const double Umean = wsc[0], us = wsc[2], logLaw = wsc[5];
     wsc[6] = (us > 0.0 ? sa * 2.0 * us * p.kappa / logLaw : 0.0) + (Umean > 1e-5 ? da : 0.0);
 }
@@ -1167,11 +1186,12 @@ static void adj_scalar_ghosts(tg_ctx *C, double *v)
     k_adj_scalar_ghosts<<<g2(g.mx, g.mz), b2, 0, C->stream>>>(g, v, 1);
     k_adj_scalar_ghosts<<<g2(g.my, g.mz), b2, 0, C->stream>>>(g, v, 0);
 }
-static void adj_contra(tg_ctx *C, V3f<double> ca, V3f<double> ua)
+static void adj_contra(tg_ctx *C, V3f<double> ca, V3f<double> ua, const V3f<double> *sum = nullptr)
 {
     AdjState &A = *C->adj;
     const Grid g = C->g;
-    k_adj_contra_cells<<<gint(g), block3(), 0, C->stream>>>(g, C->m, ca, A.qa);
+    if (sum) k_adj_contra_cells<true><<<gall(g), block3(), 0, C->stream>>>(g, C->m, ca, A.qa, *sum);
+    else k_adj_contra_cells<false><<<gint(g), block3(), 0, C->stream>>>(g, C->m, ca, A.qa, ca);
     k_adj_contra_faces<<<gfc(g), block3(), 0, C->stream>>>(g, A.qa, ua);
 }
 
@@ -1203,7 +1223,7 @@ static int adjoint_reverse_body(tg_ctx *C, bool capture)
     cudaStream_t st = C->stream;
     const double dt = C->prm.dt;
     TG_PROF(C, "adj_misc", k_sum_partial<<<C->red_blocks, TB, 0, st>>>(G, A.pa, C->d_red));
-    k_gauge_adj<<<1, 1, 0, st>>>(C->d_red, C->red_blocks, A.pa, g.lin(1, 1, 1));
+    k_gauge_adj<<<1, TB, 0, st>>>(C->d_red, C->red_blocks, A.pa, g.lin(1, 1, 1));
     // UpdateContravariantBCs, UpdateCartesianBCs, contravariantToCartesian
     for (int d = 2; d >= 0; d--) {
         int na = d == 0 ? g.my : g.mx, nb = d == 2 ? g.my : g.mz;
@@ -1246,7 +1266,7 @@ static int adjoint_reverse_body(tg_ctx *C, bool capture)
     copy3(C, A.usa, A.ua);
     TG_PROF(C, "adj_set_rhs", k_adj_set_rhs<<<gfc(g), block3(), 0, st>>>(g, A.lam, A.usa, dt));
     adj_periodic(C, A.usa, 1);
-    k_adj_no_penetration<<<gfc(g), block3(), 0, st>>>(g, A.usa, C->prm);
+    k_adj_no_penetration<false><<<gfc(g), block3(), 0, st>>>(g, A.usa, C->prm, A.usa);
     // stages
     copy3(C, A.uoa, A.usa);
     zero3(C, A.dpa);
@@ -1277,12 +1297,10 @@ static int adjoint_reverse_body(tg_ctx *C, bool capture)
                                                            C->prm, A.f1a, A.f2a, A.f3a, A.uta, A.cta, A.na, twa));
         // stage Ucat: periodic copies, interior from contravariantToCartesian, other ghosts from the state Ucat
         adj_periodic(C, A.cta, 0);
-        adj_contra(C, A.cta, A.uta);
-        TG_PROF(C, "adj_misc", k_axpy3<<<nblk1(G), TB, 0, st>>>(G, A.ca, 1.0, A.cta));
+        adj_contra(C, A.cta, A.uta, &A.ca);
         // stage Ucont = Pf(Pnp(pre))
         adj_periodic(C, A.uta, 1);
-        k_adj_no_penetration<<<gfc(g), block3(), 0, st>>>(g, A.uta, C->prm);
-        TG_PROF(C, "adj_misc", k_axpy3<<<nblk1(G), TB, 0, st>>>(G, A.uoa, 1.0, A.uta));
+        TG_PROF(C, "adj_misc", k_adj_no_penetration<true><<<gall(g), block3(), 0, st>>>(g, A.uta, C->prm, A.uoa));
     }
     // GradP
     TG_PROF(C, "adj_grad_p", k_adj_grad_p<<<gint(g), block3(), 0, st>>>(g, C->m, A.dpa, A.pa));
@@ -1298,10 +1316,10 @@ static int adjoint_reverse_body(tg_ctx *C, bool capture)
         const V3f<double> upa{A.upa[0], A.upa[1], A.upa[2]};
         dim3 grid((g.mx - 2 + 31) / 32, (g.mz - 2 + 7) / 8);
         TG_PROF(C, "adj_wall", k_adj_wall_fwd<<<WNB, 256, 0, st>>>(g, C->m, T.ucat_n, A.wpart));
-        k_adj_wall_fwd_final<<<1, 1, 0, st>>>(g, C->prm, A.wpart, A.wsc);
+        k_adj_wall_fwd_final<<<1, 256, 0, st>>>(g, C->prm, A.wpart, A.wsc);
         TG_PROF(C, "adj_wall", k_adj_wall_local<<<WNB, 256, 0, st>>>(g, C->m, C->prm, T.ucat_n, T.wum, T.wfx, T.wfy, T.meta,
                                                                       twa, A.wxa, A.wya, A.wma, upa, A.upa[3], A.wsc, A.wpart));
-        k_adj_wall_mean<<<1, 1, 0, st>>>(g, C->prm, A.wpart, A.wsc);
+        k_adj_wall_mean<<<1, 256, 0, st>>>(g, C->prm, A.wpart, A.wsc);
         TG_PROF(C, "adj_wall", k_adj_wall_scatter<<<grid, b2, 0, st>>>(g, C->m, T.ucat_n, upa, A.upa[3], A.wsc, A.ca));
     }
     // turbines: C_T' gradient and the adjoint of the Ucat they sampled
