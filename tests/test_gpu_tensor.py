@@ -126,3 +126,50 @@ def test_metric_write_rebuilds_the_step():
     assert rel_l2(a.get("UCAT"), b.get("UCAT")) <= 1e-12
     assert not a.graph_info()[1] and a.graph_info()[0] > 2
     a.close(); b.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(13, 11, 9), (33, 8, 5)])
+def test_metric_write_reaches_the_metric_products(nx, ny, nz):
+    """The curvilinear kernels read products of the face metrics that are formed
+    once: doubling a face Jacobian doubles its component of GradP, exactly."""
+    cfg, nodes, u, p, T = cases.hill_case(nx=nx, ny=ny, nz=nz, ddt=api.DDT_RK4, teqn=True, t_amp=0.05, seed=3)
+    s = tosca_b200.gpu_solver(cfg)
+    cases.setup(s, nodes, u, p, T)
+    s.step(2)
+    s.GradP()
+    d = s.get("DP")
+    assert np.abs(d).max(axis=(0, 1, 2)).min() > 0.0
+    for f, q in (("IAJ", 0), ("JAJ", 1), ("KAJ", 2)):
+        s.set(f, 2.0 * s.get(f))
+        s.GradP()
+        d[..., q] *= 2.0
+        assert np.array_equal(s.get("DP"), d)
+    s.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz,kind,over", [
+    (7, 7, 7, "abl", {}), (6, 9, 8, "abl", {}), (9, 38, 11, "abl", dict(stretched=True)), (12, 36, 8, "abl", dict(les=0, nu=0.5)),
+    (13, 13, 13, "tgv", {}), (10, 37, 9, "box", {}), (9, 12, 10, "abl", dict(ddt=api.DDT_FE, dt=0.02))])
+def test_adjoint_against_general_kernels(nx, ny, nz, kind, over):
+    """The reverse step's kernels for meshes of planes, around their tile of
+    32 x 4 x 2 cells and the two cells to an end that the scatter keeps. Same
+    products in another order, as above; the transposed pressure solve stops at
+    the context's relative tolerance of 1e-13. The adjoint of P is bounded
+    against its seed: with one stage per step (forward Euler) the projection takes
+    out all that an old P puts in, and what is left is rounding."""
+    cfg, nodes, u, p, T = make(kind, nx, ny, nz, **over)
+    cfg.source = 1
+    rng = np.random.default_rng(nx + ny)
+    a, b = pair(cfg, nodes, u, p, T)
+    seeds = {f: rng.standard_normal(a.field_shape(f)) for f in ("UCAT_ADJ", "UCONT_ADJ", "P_ADJ")}
+    for s in (a, b):
+        s.step(2)
+        for f, v in seeds.items():
+            w = np.zeros_like(v)
+            w[1:-1, 1:-1, 1:-1] = v[1:-1, 1:-1, 1:-1]
+            s.set(f, w)
+        s.adjoint_step()
+    for f in ("UCONT_ADJ", "UCAT_ADJ", "SOURCE_ADJ"):
+        assert rel_l2(a.get(f), b.get(f)) <= 1e-11, f
+    assert np.linalg.norm(a.get("P_ADJ") - b.get("P_ADJ")) <= 1e-9 * np.linalg.norm(seeds["P_ADJ"])
+    a.close(); b.close()

@@ -495,13 +495,43 @@ __global__ void k_adj_rhs_faces(Grid g, Metrics m, V3f<double> ra, double scale,
     if (!g.pk && k == mz - 2) acc = acc + tz(c) * ld3(m.zet, c + pl);
     st3(fpa, c, acc);
 }
+// The face points 0 .. m-2 of which an index is within two of an end, the ones
+// whose fluxes reach a cell outside adj_core: SHELL kernels take them as a list
+// (planes of k, then of j, then of i), n per direction > 6
+__host__ __device__ inline int64_t shell_faces(const Grid &g)
+{
+    const int64_t nx = g.mx - 1, ny = g.my - 1, nz = g.mz - 1;
+    return 5 * (ny * nx + (nz - 5) * nx + (nz - 5) * (ny - 5));
+}
+__device__ __forceinline__ bool shell_face(const Grid &g, int64_t t, int &k, int &j, int &i)
+{
+    const int nx = g.mx - 1, ny = g.my - 1, nz = g.mz - 1;
+    auto end = [](int q, int n) { return q < 3 ? q : n - 5 + q; };
+    int q = (int)t, row = ny * nx;
+    if (t >= shell_faces(g)) return false;
+    if (q < 5 * row) { k = end(q / row, nz); q %= row; j = q / nx; i = q % nx; return true; }
+    q -= 5 * row; row = (nz - 5) * nx;
+    if (q < 5 * row) { j = end(q / row, ny); q %= row; k = 3 + q / nx; i = q % nx; return true; }
+    q -= 5 * row;
+    i = end(q % 5, nx); q /= 5;
+    j = 3 + q % (ny - 5); k = 3 + q / (ny - 5);
+    return true;
+}
+// the cells that receive from regular faces only
+__device__ __forceinline__ bool adj_core(const Grid &g, int k, int j, int i)
+{
+    return i >= 2 && i <= g.mx - 3 && j >= 2 && j <= g.my - 3 && k >= 2 && k <= g.mz - 3;
+}
+
 // pass 2 transpose (gather per face): flux_adj(f) = fp_adj(left cell) -
 // fp_adj(right cell), with the periodic face-0 read of cell 1 remapped to
 // face m-2
+template <bool SHELL>
 __global__ void k_adj_cell_fp(Grid g, V3f<double> fpa, V3f<double> f1a, V3f<double> f2a, V3f<double> f3a)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
+    if (SHELL) { if (!shell_face(g, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, k, j, i)) return; }
+    else if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
     const int mx = g.mx, my = g.my, mz = g.mz, pl = mx * my;
     int f = g.lin(k, j, i);
     R3<double> z{0, 0, 0};
@@ -567,8 +597,9 @@ __device__ __forceinline__ void visc_adj_ax(double cs, double et, double ze, int
 // pass 1 transpose: per face, scatter to Ucat (atomics), Ucont (own face) and
 // nut. AX: the mesh is axis-aligned and the forward step formed the
 // axis-aligned viscous flux, whose exact transpose reads 3 of the 9 face
-// metric components
-template <bool AX>
+// metric components. SHELL: only the faces that reach a cell outside adj_core,
+// and only those cells; k_adj_face_core does the others
+template <bool AX, bool SHELL>
 __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double> uc, const double *nut, Params p,
                                   V3f<double> f1a, V3f<double> f2a, V3f<double> f3a,
                                   V3f<double> uta, V3f<double> cta, double *na, V3f<double> twa)
@@ -580,11 +611,11 @@ __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double>
     // tile are read from global memory.
     constexpr int ATX = BX + 3, ATY = BY + 3, ATZ = BZ + 3, ATN = ATX * ATY * ATZ;
     static_assert(BX == 32 && (BX * BY * BZ) % 32 == 0 && 3 * ATY * ATZ <= BX * BY * BZ, "tile staging layout");
-    __shared__ double su[3][ATN];
-    __shared__ double sn[ATN];
+    __shared__ double su[3][SHELL ? 1 : ATN];
+    __shared__ double sn[SHELL ? 1 : ATN];
     const int mx = g.mx, my = g.my, mz = g.mz;
     const int i0 = blockIdx.x * BX, j0 = blockIdx.y * BY, k0 = blockIdx.z * BZ;
-    {
+    if (!SHELL) {
         auto stage = [&](int tx, int ty, int tz, int gi) {
             const int gj = g.wj(j0 - 1 + ty), gk = g.wk(k0 - 1 + tz), q = (tz * ATY + ty) * ATX + tx;
             double ux = 0.0, uy = 0.0, uz = 0.0, nt = 0.0;
@@ -604,25 +635,29 @@ __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double>
             stage(tx, r % ATY, r / ATY, g.wi(i0 - 1 + tx));
         }
     }
-    __syncthreads();
-    const int i = i0 + threadIdx.x, j = j0 + threadIdx.y, k = k0 + threadIdx.z;
-    if (i > mx - 2 || j > my - 2 || k > mz - 2) return;
+    if (!SHELL) __syncthreads();
+    int i = i0 + threadIdx.x, j = j0 + threadIdx.y, k = k0 + threadIdx.z;
+    if (SHELL) { if (!shell_face(g, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, k, j, i)) return; }
+    else if (i > mx - 2 || j > my - 2 || k > mz - 2) return;
     const bool npi = !g.pi, npj = !g.pj, npk = !g.pk;
-    const bool quickDiv = p.div_scheme == TG_DIV_QUICK;
+    const bool quickDiv = !SHELL && p.div_scheme == TG_DIV_QUICK;
     const double nu = p.nu;
     int f = g.lin(k, j, i);
+    const bool own = !SHELL || !adj_core(g, k, j, i);
     // tile index of (kk, jj, ii), or -1 outside the tile
     auto tq = [&](int kk, int jj, int ii) {
         const int tx = ii - i0 + 1, ty = jj - j0 + 1, tz = kk - k0 + 1;
-        return ((unsigned)tx < (unsigned)ATX && (unsigned)ty < (unsigned)ATY && (unsigned)tz < (unsigned)ATZ) ? (tz * ATY + ty) * ATX + tx : -1;
+        return !SHELL && ((unsigned)tx < (unsigned)ATX && (unsigned)ty < (unsigned)ATY && (unsigned)tz < (unsigned)ATZ) ? (tz * ATY + ty) * ATX + tx : -1;
     };
     auto U = [&](int kk, int jj, int ii) {
         const int q = tq(kk, jj, ii);
         return q >= 0 ? R3<double>{su[0][q], su[1][q], su[2][q]} : ld3(uc, g.id(kk, jj, ii));
     };
-    auto UA = [&](int kk, int jj, int ii, double w, R3<double> v) { aadd3(cta, g.id(kk, jj, ii), w, v); };
+    auto UA = [&](int kk, int jj, int ii, double w, R3<double> v) {
+        if (!SHELL || !adj_core(g, kk, jj, ii)) aadd3(cta, g.id(kk, jj, ii), w, v);
+    };
     auto NUT = [&](int kk, int jj, int ii) { const int q = tq(kk, jj, ii); return q >= 0 ? sn[q] : nut[g.id(kk, jj, ii)]; };
-    auto NA = [&](int kk, int jj, int ii, double v) { aadd(na + g.id(kk, jj, ii), v); };
+    auto NA = [&](int kk, int jj, int ii, double v) { if (!SHELL || !adj_core(g, kk, jj, ii)) aadd(na + g.id(kk, jj, ii), v); };
     auto quickW = [](double w, double q[4]) {
         if (w > 0) { q[0] = -0.125; q[1] = 0.75; q[2] = 0.375; q[3] = 0.0; }
         else       { q[0] = 0.0; q[1] = 0.375; q[2] = 0.75; q[3] = -0.125; }
@@ -648,7 +683,7 @@ __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double>
             uface = 0.5 * (U(k, j, i) + U(k, j, i + 1));
             UA(k, j, i, 0.5, ga); UA(k, j, i + 1, 0.5, ga);
         }
-        uta.x[f] += -dot3(gv, uface);
+        if (own) uta.x[f] += -dot3(gv, uface);
         double nuEff; bool vnut = false;
         if (p.les) {
             if ((p.bc[TG_ILEFT] == TG_BC_SLIP && i == 0) || (p.bc[TG_IRIGHT] == TG_BC_SLIP && i == mx - 2)) nuEff = 0.0;
@@ -702,7 +737,7 @@ __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double>
             uface = 0.5 * (U(k, j, i) + U(k, j + 1, i));
             UA(k, j, i, 0.5, ga); UA(k, j + 1, i, 0.5, ga);
         }
-        uta.y[f] += -dot3(gv, uface);
+        if (own) uta.y[f] += -dot3(gv, uface);
         double nuEff; bool vnut = false;
         if (p.les) {
             if ((p.bc[TG_JLEFT] == TG_BC_WALL_SHUMANN && j == 0) || (p.bc[TG_JRIGHT] == TG_BC_WALL_SHUMANN && j == my - 2)) {
@@ -759,7 +794,7 @@ __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double>
             uface = 0.5 * (U(k, j, i) + U(k + 1, j, i));
             UA(k, j, i, 0.5, ga); UA(k + 1, j, i, 0.5, ga);
         }
-        uta.z[f] += -dot3(gv, uface);
+        if (own) uta.z[f] += -dot3(gv, uface);
         double nuEff; bool vnut = false;
         if (p.les) {
             if ((p.bc[TG_KLEFT] == TG_BC_SLIP && k == 0) || (p.bc[TG_KRIGHT] == TG_BC_SLIP && k == mz - 2)) nuEff = 0.0;
@@ -791,6 +826,85 @@ __global__ void k_adj_face_fluxes(Grid g, Metrics m, V3f<double> ut, V3f<double>
         else if (jo == 2) { UA(k + 1, j + 1, i, 0.5, dd[1]); UA(k, j + 1, i, 0.5, dd[1]); UA(k + 1, j, i, -0.5, dd[1]); UA(k, j, i, -0.5, dd[1]); }
         else              { UA(k + 1, j + 1, i, 0.25, dd[1]); UA(k, j + 1, i, 0.25, dd[1]); UA(k + 1, j - 1, i, -0.25, dd[1]); UA(k, j - 1, i, -0.25, dd[1]); }
     }
+}
+
+// The cells of adj_core on a mesh of planes with central convection, where every
+// face that reaches a cell has the regular stencil: a gather. A thread forms
+// the six faces of its cell, and the one component that each of the 24 faces
+// along its edges sends through a cross derivative, from a tile of fp_adj, Ucat and nut
+// (one cell of halo); the metrics are products of spacings (ts), and the flux
+// adjoints are differences of fp_adj. No atomics, of which the scatter above issues
+// 114 per cell. 128 x 64 x 64, per stage: 147 us by the scatter alone, 60 us here
+// plus 31 for the scatter's shell (floor 11 us: 136 bytes per cell; it is bound by
+// the latency of its chains at three blocks of 256 threads per SM; unrolled, the two
+// sides took 128 registers and the same time).
+constexpr int GTX = 32, GTY = 4, GTZ = 2, GHX = GTX + 2, GHY = GTY + 2, GHZ = GTZ + 2, GHN = GHX * GHY * GHZ;
+template <bool LES>
+__global__ void __launch_bounds__(GTX * GTY * GTZ, 3) k_adj_face_core(Grid g, Tensor t, V3f<double> ut, V3f<double> uc, const double *nut, double nu,
+                                                                      V3f<double> fpa, V3f<double> uta, V3f<double> cta, double *na)
+{
+    __shared__ double sf[3][GHN], su[3][GHN], sn[LES ? GHN : 1];
+    const int i0 = 2 + blockIdx.x * GTX, j0 = 2 + blockIdx.y * GTY, k0 = 2 + blockIdx.z * GTZ;
+    for (int q = (threadIdx.z * GTY + threadIdx.y) * GTX + threadIdx.x; q < GHN; q += GTX * GTY * GTZ) {
+        const int i = i0 - 1 + q % GHX, j = j0 - 1 + q / GHX % GHY, k = k0 - 1 + q / (GHX * GHY);
+        const bool in = i <= g.mx - 2 && j <= g.my - 2 && k <= g.mz - 2;
+        const int c = in ? g.lin(k, j, i) : 0;
+        sf[0][q] = in ? fpa.x[c] : 0.0; sf[1][q] = in ? fpa.y[c] : 0.0; sf[2][q] = in ? fpa.z[c] : 0.0;
+        su[0][q] = in ? uc.x[c] : 0.0; su[1][q] = in ? uc.y[c] : 0.0; su[2][q] = in ? uc.z[c] : 0.0;
+        if (LES) sn[q] = in ? nut[c] : 0.0;
+    }
+    __syncthreads();
+    const int i = i0 + threadIdx.x, j = j0 + threadIdx.y, k = k0 + threadIdx.z;
+    if (!adj_core(g, k, j, i)) return;
+    const int c = g.lin(k, j, i), o = ((threadIdx.z + 1) * GHY + threadIdx.y + 1) * GHX + threadIdx.x + 1;
+    const double dx = t.dx[k], dy = t.dy[i], dz = t.dz[j];
+    R3<double> acc{0, 0, 0};
+    double nacc = 0.0;
+    auto F = [&](int d, int a, int b) { return sf[d][a] - sf[d][b]; };        // flux adjoint of the face a|b
+    auto nuF = [&](int a, int b) { return LES ? nu + 0.5 * (sn[a] + sn[b]) : nu; };
+    // one of the cell's six faces: stride st of its direction n, on the + (e = 0) or
+    // the - side (e = -1); w: spacings of the normal derivative, uf: its Ucont.
+    // r: the component the cross derivatives carry; along st1 (weight w1) it comes
+    // from component r1 of the flux adjoint, along st2 (w2) from r2
+    auto face = [&](int st, int e, int n, double w, double uf, int r, int st1, double w1, int r1, int st2, double w2, int r2) {
+        const int a = o + e * st, b = a + st;
+        const double gv[3] = {F(0, a, b), F(1, a, b), F(2, a, b)};
+        const double nuE = nuF(a, b);
+        double dd[3] = {w * gv[0], w * gv[1], w * gv[2]};
+        dd[r] += dd[r];
+        const double sg = e == 0 ? -nuE : nuE, h = -0.5 * uf;
+        acc.x += h * gv[0] + sg * dd[0]; acc.y += h * gv[1] + sg * dd[1]; acc.z += h * gv[2] + sg * dd[2];
+        if (LES) {
+            double ne = 0.0;
+            #pragma unroll
+            for (int d = 0; d < 3; d++) ne += dd[d] * (su[d][b] - su[d][a]);
+            ne += w1 * gv[r1] * (0.25 * (su[r][b + st1] + su[r][a + st1] - su[r][b - st1] - su[r][a - st1]));
+            ne += w2 * gv[r2] * (0.25 * (su[r][b + st2] + su[r][a + st2] - su[r][b - st2] - su[r][a - st2]));
+            nacc += 0.5 * ne;
+        }
+        // the cross derivatives of the four faces beside this one
+        double v = w1 * (nuF(a - st1, b - st1) * F(r1, a - st1, b - st1) - nuF(a + st1, b + st1) * F(r1, a + st1, b + st1))
+                 + w2 * (nuF(a - st2, b - st2) * F(r2, a - st2, b - st2) - nuF(a + st2, b + st2) * F(r2, a + st2, b + st2));
+        v *= 0.25;
+        if (r == 0) acc.x += v; else if (r == 1) acc.y += v; else acc.z += v;
+        if (e == 0) {
+            double u = 0.0;
+            #pragma unroll
+            for (int d = 0; d < 3; d++) u += gv[d] * (0.5 * (su[d][a] + su[d][b]));
+            double *const q = n == 0 ? uta.x : n == 1 ? uta.y : uta.z;
+            q[c] -= u;
+        }
+    };
+    constexpr int sI = 1, sJ = GHX, sK = GHX * GHY;
+    const int pl = g.mx * g.my;
+    #pragma unroll 1
+    for (int e = 0; e >= -1; e--) {
+        face(sI, e, 0, dx * dz * t.rdyf[i + e], ut.x[c + e], 1, sJ, dx, 2, sK, dz, 0);
+        face(sJ, e, 1, dx * dy * t.rdzf[j + e], ut.y[c + e * g.mx], 2, sI, dx, 1, sK, dy, 0);
+        face(sK, e, 2, dy * dz * t.rdxf[k + e], ut.z[c + e * pl], 0, sI, dz, 1, sJ, dy, 2);
+    }
+    cta.x[c] += acc.x; cta.y[c] += acc.y; cta.z[c] += acc.z;
+    if (LES) na[c] += nacc;
 }
 
 // ------------------------------------------------------------------- GradP
@@ -1286,15 +1400,28 @@ static int adjoint_reverse_body(tg_ctx *C, bool capture)
         if (C->prm.farm) farm_adj_stage(C, A.ra);
         // FormU transposed
         TG_PROF(C, "adj_rhs_faces", k_adj_rhs_faces<<<gint(g), block3(), 0, st>>>(g, C->m, A.ra, 1.0, A.fpa));
-        TG_PROF(C, "adj_cell_fp", k_adj_cell_fp<<<gfc(g), block3(), 0, st>>>(g, A.fpa, A.f1a, A.f2a, A.f3a));
+        // gather where every stencil is regular, scatter with atomics elsewhere
+        // (k_adj_face_core's figures); below nine points in a direction the shell is
+        // all there is, and its list would name points twice
+        const bool core = C->axis_aligned && C->prm.div_scheme != TG_DIV_QUICK && std::min({g.mx, g.my, g.mz}) >= 9;
+        const int nsh = (int)((shell_faces(g) + 127) / 128);
+        if (core) TG_PROF(C, "adj_cell_fp", k_adj_cell_fp<true><<<nsh, 128, 0, st>>>(g, A.fpa, A.f1a, A.f2a, A.f3a));
+        else TG_PROF(C, "adj_cell_fp", k_adj_cell_fp<false><<<gfc(g), block3(), 0, st>>>(g, A.fpa, A.f1a, A.f2a, A.f3a));
         zero3(C, A.uta);
         zero3(C, A.cta);
-        if (C->axis_aligned)
-            TG_PROF(C, "adj_face_fluxes", k_adj_face_fluxes<true><<<gfc(g), block3(), 0, st>>>(g, C->m, T.ut[s], T.uc[s], T.nut,
+        auto scatter = [&](auto kernel, dim3 grid, dim3 block) {
+            TG_PROF(C, "adj_face_fluxes", kernel<<<grid, block, 0, st>>>(g, C->m, T.ut[s], T.uc[s], T.nut,
                                                           C->prm, A.f1a, A.f2a, A.f3a, A.uta, A.cta, A.na, twa));
-        else
-            TG_PROF(C, "adj_face_fluxes", k_adj_face_fluxes<false><<<gfc(g), block3(), 0, st>>>(g, C->m, T.ut[s], T.uc[s], T.nut,
-                                                           C->prm, A.f1a, A.f2a, A.f3a, A.uta, A.cta, A.na, twa));
+        };
+        if (core) {
+            const dim3 gc((g.mx - 4 + GTX - 1) / GTX, (g.my - 4 + GTY - 1) / GTY, (g.mz - 4 + GTZ - 1) / GTZ), bc(GTX, GTY, GTZ);
+            auto gather = [&](auto kernel) {
+                TG_PROF(C, "adj_face_core", kernel<<<gc, bc, 0, st>>>(g, C->ts, T.ut[s], T.uc[s], T.nut, C->prm.nu, A.fpa, A.uta, A.cta, A.na));
+            };
+            if (C->prm.les) gather(k_adj_face_core<true>); else gather(k_adj_face_core<false>);
+            scatter(k_adj_face_fluxes<true, true>, dim3(nsh), dim3(128));
+        } else if (C->axis_aligned) scatter(k_adj_face_fluxes<true, false>, gfc(g), block3());
+        else scatter(k_adj_face_fluxes<false, false>, gfc(g), block3());
         // stage Ucat: periodic copies, interior from contravariantToCartesian, other ghosts from the state Ucat
         adj_periodic(C, A.cta, 0);
         adj_contra(C, A.cta, A.uta, &A.ca);
