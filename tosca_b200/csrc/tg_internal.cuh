@@ -329,6 +329,13 @@ __device__ __forceinline__ bool last_block(unsigned *count)
     if (last && threadIdx.x == 0) { __threadfence(); *count = 0u; }
     return last;
 }
+// copy of one double from global to shared memory, of the calling thread's current group
+__device__ __forceinline__ void cp_async8(double *sm, const double *gm)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(sm);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gm));
+}
+
 // sums of the NV partials per block at part[NV * block ..], in thread 0 of a
 // block of NT threads
 template <int NT, int NV>

@@ -252,11 +252,6 @@ __device__ void fp_boundary_block(const Grid &g, const Tensor &t, const State &s
 // and one cell around them are copied asynchronously into shared memory.
 constexpr int PX = 32, PY = 8, PTX = PX + 2, PTY = PY + 2;
 
-__device__ __forceinline__ void cp_async8(double *sm, const double *gm)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(sm);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gm));
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <int mode, bool LES, int KZ>

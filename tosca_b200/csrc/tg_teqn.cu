@@ -68,14 +68,21 @@ __device__ __forceinline__ void stencil4(int i, int m, int per, int &L, int &R)
 }
 
 // pass 1: the flux at the faces of the interior cells, convective plus diffusive
-// (mode 0), convective (1) or diffusive (2). One thread per interior cell
-// (k, j, i) forms the i, j and k faces on the cell's + side, and a cell next to
-// a non-periodic 0 boundary also the face on its - side (face 0; face 0 of a
-// periodic direction is read from face m-2 by the budget and is not formed). T
-// and nut are staged in a shared-memory tile of the block's cells with one cell
-// below and two above in every direction (the DMDA wrap of periodic directions
-// applied once, at staging), so every stencil read is a fixed tile offset; the
-// WENO points of the boundary faces, which may lie outside the tile (periodic
+// (mode 0), convective (1) or diffusive (2). A block takes 32 x 8 columns of
+// interior cells and marches along k; a thread forms the i, j and k faces on its
+// cell's + side, and a cell next to a non-periodic 0 boundary also the face on
+// its - side (face 0; face 0 of a periodic direction is read from face m-2 by
+// the budget and is not formed). T and nut are read from a ring of six planes in
+// shared memory with one cell below and two above in i and j; plane k + 4 is
+// copied while plane k is worked on, one barrier per plane. Bound by instruction
+// issue (525 of 725 per cell were integer and select work) and by the
+// latency of the divisions: blocks of 32 x 4 x 2 cells that staged 35 x 7 x 5 points
+// each took 3.52 ms of a step at 192 x 96 x 96 (curvilinear) and 0.890 ms at
+// 128 x 128 x 64, this one 3.43 and 0.875 (3.44 and 0.884 with the ends of each
+// direction tested per derivative instead of once per face; 3.47 and 0.900 with
+// 80 registers and three blocks per SM). The floor, at 64 to 160 bytes per cell, is
+// a fifth to a third of its time.
+// The WENO points of the boundary faces, which may lie outside the tile (periodic
 // i = mx + 2 and i = -3), are read from global memory.
 //
 // AX: a mesh of planes: the metric tensor of a face is its normal component
@@ -86,189 +93,204 @@ __device__ __forceinline__ void stencil4(int i, int m, int per, int &L, int &R)
 // Jacobian are SetCoeffMatrix's arrays (9 values per cell, the face metrics 30).
 // rd2: 1/delta^2 of the i, j and k faces (k_t_width), on a
 // mesh of planes a product of factors as well.
-constexpr int TBX = 32, TBY = 4, TBZ = 2, TBN = TBX * TBY * TBZ;
-constexpr int TTX = TBX + 3, TTY = TBY + 3, TTZ = TBZ + 3, TTN = TTX * TTY * TTZ;
+constexpr int TBX = 32, TBY = 8, TBN = TBX * TBY;
+constexpr int TTX = TBX + 3, TTY = TBY + 3, TTN = TTX * TTY, TRING = 6;
 
 template <bool AX, int mode>
-__global__ void __launch_bounds__(TBN) k_t_face_fluxes(Grid g, Metrics m, Tensor t, State s, Params p, V3f<double> rd2, V3f<double> fl)
+__global__ void __launch_bounds__(TBN, 4) k_t_face_fluxes(const __grid_constant__ Grid g, const __grid_constant__ Metrics m, const __grid_constant__ Tensor t,
+                                                          const __grid_constant__ State s, const __grid_constant__ Params p, V3f<double> rd2, V3f<double> fl,
+                                                          int nbi, int nbj, int kc)
 {
-    __shared__ double st[TTN];
-    __shared__ double sn[TTN];
-    const int mx = g.mx, my = g.my, mz = g.mz;
-    const int i0 = 1 + blockIdx.x * TBX, j0 = 1 + blockIdx.y * TBY, k0 = 1 + blockIdx.z * TBZ;
-    // staging: tile point (tx, ty, tz) <- DMDA (i0-1+tx, j0-1+ty, k0-1+tz),
-    // wrapped; 0 outside a non-periodic extent
-    auto stage = [&](int tx, int ty, int tz, int gi) {
-        const int gj = g.wj(j0 - 1 + ty), gk = g.wk(k0 - 1 + tz), q = (tz * TTY + ty) * TTX + tx;
-        double tv = 0.0, nv = 0.0;
-        if (gi >= 0 && gi < mx && gj >= 0 && gj < my && gk >= 0 && gk < mz) {
-            const int c = (gk * my + gj) * mx + gi;
-            tv = s.tmprt[c];
-            if (p.les) nv = s.nut[c];
-        }
-        st[q] = tv; sn[q] = nv;
-    };
-    {
-        // each warp stages whole tile rows (lane = tx, warp-uniform row), then
-        // every thread at most one point of the last three columns
-        static_assert(TBX == 32 && TBN % 32 == 0 && 3 * TTY * TTZ <= TBN, "one warp per tile row, one pass for the last columns");
-        const int lane = threadIdx.x, wid = threadIdx.z * TBY + threadIdx.y;
-        const int gi = g.wi(i0 - 1 + lane);
-        for (int r = wid; r < TTY * TTZ; r += TBN / 32) stage(lane, r % TTY, r / TTY, gi);
-        const int q = wid * 32 + lane;
-        if (q < 3 * TTY * TTZ) {
-            const int r = q / 3, tx = TBX + (q - 3 * r);
-            stage(tx, r % TTY, r / TTY, g.wi(i0 - 1 + tx));
-        }
+    __shared__ double ring[TRING * 2 * TTN];         // per plane T, then nut
+    const int mx = g.mx, my = g.my, mz = g.mz, pl = mx * my;
+    const int br = blockIdx.x / nbi;
+    const int i0 = 1 + (blockIdx.x % nbi) * TBX, j0 = 1 + (br % nbj) * TBY, k0 = 1 + (br / nbj) * kc, k1 = min(k0 + kc - 1, mz - 2);
+    // what this thread copies of every plane: elements tid and tid + TBN of the
+    // tile (DMDA i0 - 1 + x, j0 - 1 + y; points outside the domain are never used
+    // and read the plane's first element)
+    const int tid = threadIdx.y * TBX + threadIdx.x;
+    static_assert(TTN <= 2 * TBN, "two elements per thread");
+    int off[2];
+    #pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int e = tid + q * TBN, ti = i0 - 1 + e % TTX, tj = j0 - 1 + e / TTX;
+        off[q] = ti < mx && tj < my ? tj * mx + ti : 0;
     }
-    __syncthreads();
-    const int i = i0 + threadIdx.x, j = j0 + threadIdx.y, k = k0 + threadIdx.z;
-    if (i > mx - 2 || j > my - 2 || k > mz - 2) return;
+    const bool les = p.les, two = tid < TTN - TBN;
+    // plane q into a slot of the ring
+    auto load = [&](int q, double *d) {
+        if (q <= mz - 1) {
+            const int o = q * pl;
+            d += tid;
+            cp_async8(d, s.tmprt + o + off[0]);
+            if (mode != 1 && les) cp_async8(d + TTN, s.nut + o + off[0]);
+            if (two) {
+                cp_async8(d + TBN, s.tmprt + o + off[1]);
+                if (mode != 1 && les) cp_async8(d + TBN + TTN, s.nut + o + off[1]);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    #pragma unroll
+    for (int q = 0; q < 5; q++) load(k0 - 1 + q, ring + q * 2 * TTN);
+    const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+    const bool on = i <= mx - 2 && j <= my - 2;
+    const int t0 = (threadIdx.y + 1) * TTX + threadIdx.x + 1;
+    int slot = 0;                                    // of plane k - 1
     const bool npi = !g.pi, npj = !g.pj, npk = !g.pk;
-    const int t0 = ((threadIdx.z + 1) * TTY + threadIdx.y + 1) * TTX + threadIdx.x + 1;
-    auto T = [&](int dk, int dj, int di) { return st[t0 + (dk * TTY + dj) * TTX + di]; };
-    auto NUT = [&](int dk, int dj, int di) { return sn[t0 + (dk * TTY + dj) * TTX + di]; };
+    const int ni = (i == 1 && npi) ? 2 : 1, nj = (j == 1 && npj) ? 2 : 1;
     auto TG = [&](int kk, int jj, int ii) { return s.tmprt[g.id(kk, jj, ii)]; };
     const double sqt = sqrt(p.t_ref);
+    // the column's factors of 1/delta^2 (q) and of the diffusion (w) at the faces E, N, T
+    const bool ax = AX && on;
+    const double qE = ax && les ? t.rqyf[i] * t.rqz[j] : 0.0, qN = ax && les ? t.rqy[i] * t.rqzf[j] : 0.0, qT = ax && les ? t.rqy[i] * t.rqz[j] : 0.0;
+    const double wE = ax ? t.dz[j] * t.rdyf[i] : 0.0, wN = ax ? t.dy[i] * t.rdzf[j] : 0.0, wT = ax ? t.dy[i] * t.dz[j] : 0.0;
+    // plane k + 2 is there when all but the newest copy have arrived
+    for (int k = k0; k <= k1; k++, slot = slot == TRING - 1 ? 0 : slot + 1) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        auto plane = [&](int d) { const int q = slot + d; return ring + (q >= TRING ? q - TRING : q) * (2 * TTN); };
+        load(k + 4, plane(5));
+        if (!on) continue;
+        const double *const Pm = plane(0) + t0, *const P0 = plane(1) + t0, *const P1 = plane(2) + t0, *const P2 = plane(3) + t0;
+        auto T = [&](int dk, int dj, int di) { return (dk < 0 ? Pm : dk == 0 ? P0 : P1)[dj * TTX + di]; };
+        auto NUT = [&](int dj, int di) { return P0[TTN + dj * TTX + di]; };
+        const double rqx = AX && les ? t.rqx[k] : 0.0, dx = AX ? t.dx[k] : 0.0;
+        // A derivative along a face is central except, on a face of the boundary, at
+        // the two ends of its direction when either is not periodic.
 
-    // ---- i face fi = i + e (Compute_dscalar_i, inline.h:3210-3247)
-    auto iface = [&](int fi, int e) {
-        const int f = g.lin(k, j, fi);
-        const bool edge = (fi == 0 || fi == mx - 2);
-        const double dtdc = T(0, 0, e + 1) - T(0, 0, e);
-        double dtde, dtdz = 0.0;
-        if (j == my - 2 && edge && (npj || npi))      dtde = (T(0, 0, e + 1) + T(0, 0, e) - T(0, -1, e + 1) - T(0, -1, e)) * 0.5;
-        else if (j == 1 && edge && (npj || npi))      dtde = (T(0, 1, e + 1) + T(0, 1, e) - T(0, 0, e + 1) - T(0, 0, e)) * 0.5;
-        else                                          dtde = (T(0, 1, e + 1) + T(0, 1, e) - T(0, -1, e + 1) - T(0, -1, e)) * 0.25;
-        if (!AX) {
-            if (k == mz - 2 && edge && (npk || npi))  dtdz = (T(0, 0, e + 1) + T(0, 0, e) - T(-1, 0, e + 1) - T(-1, 0, e)) * 0.5;
-            else if (k == 1 && edge && (npk || npi))  dtdz = (T(1, 0, e + 1) + T(1, 0, e) - T(0, 0, e + 1) - T(0, 0, e)) * 0.5;
-            else                                      dtdz = (T(1, 0, e + 1) + T(1, 0, e) - T(-1, 0, e + 1) - T(-1, 0, e)) * 0.25;
-        }
-        double o = 0.0;
-        if (mode != 2) {
-            const double uc = s.ucont.x[f];
-            double w;
-            if (edge) {
-                int iL, iR;
-                stencil4(fi, mx, g.pi, iL, iR);
-                w = weno3(TG(k, j, iL), T(0, 0, e), T(0, 0, e + 1), TG(k, j, iR), uc);
-            } else w = weno3(T(0, 0, e - 1), T(0, 0, e), T(0, 0, e + 1), T(0, 0, e + 2), uc);
-            o = -uc * w;
-        }
-        if (mode == 1) { fl.x[f] = o; return; }
-        const double wd = !p.les ? 0.0 : AX ? t.rqx[k] * t.rqyf[fi] * t.rqz[j] : rd2.x[f];
-        const double ke = kappa_eff(p, p.les ? 0.5 * (NUT(0, 0, e) + NUT(0, 0, e + 1)) : 0.0, dtde, wd, sqt);
-        if (AX) {
-            fl.x[f] = o + (t.dx[k] * t.dz[j] * t.rdyf[fi] * dtdc) * ke;
-        } else {
-            double a = 0.0, b = 0.0, c = 0.0;
-            if (e == 0) { a = m.g11[f]; b = m.g12[f]; c = m.g13[f]; }
-            else {                       // face 0 has its own metrics
-                const R3<double> n = ld3(m.icsi, f);
-                const double w = m.iaj[f];
-                a = dot3(ld3(m.icsi, f), n) * w; b = dot3(ld3(m.ieta, f), n) * w; c = dot3(ld3(m.izet, f), n) * w;
+        // ---- i face fi = i + e (Compute_dscalar_i, inline.h:3210-3247)
+        auto iface = [&](int fi, int e) {
+            const int f = g.lin(k, j, fi);
+            const double dtdc = T(0, 0, e + 1) - T(0, 0, e);
+            double dtde = (T(0, 1, e + 1) + T(0, 1, e) - T(0, -1, e + 1) - T(0, -1, e)) * 0.25, dtdz = 0.0, o = 0.0;
+            if (!AX) dtdz = (T(1, 0, e + 1) + T(1, 0, e) - T(-1, 0, e + 1) - T(-1, 0, e)) * 0.25;
+            const double uc = mode != 2 ? s.ucont.x[f] : 0.0;
+            if (fi == 0 || fi == mx - 2) {
+                if (npj || npi) {
+                    if (j == my - 2)   dtde = (T(0, 0, e + 1) + T(0, 0, e) - T(0, -1, e + 1) - T(0, -1, e)) * 0.5;
+                    else if (j == 1)   dtde = (T(0, 1, e + 1) + T(0, 1, e) - T(0, 0, e + 1) - T(0, 0, e)) * 0.5;
+                }
+                if (!AX && (npk || npi)) {
+                    if (k == mz - 2)   dtdz = (T(0, 0, e + 1) + T(0, 0, e) - T(-1, 0, e + 1) - T(-1, 0, e)) * 0.5;
+                    else if (k == 1)   dtdz = (T(1, 0, e + 1) + T(1, 0, e) - T(0, 0, e + 1) - T(0, 0, e)) * 0.5;
+                }
+                if (mode != 2) {
+                    int iL, iR;
+                    stencil4(fi, mx, g.pi, iL, iR);
+                    o = -uc * weno3(TG(k, j, iL), T(0, 0, e), T(0, 0, e + 1), TG(k, j, iR), uc);
+                }
+            } else if (mode != 2) o = -uc * weno3(T(0, 0, e - 1), T(0, 0, e), T(0, 0, e + 1), T(0, 0, e + 2), uc);
+            if (mode == 1) { fl.x[f] = o; return; }
+            const double wd = !les ? 0.0 : AX ? rqx * (e == 0 ? qE : t.rqyf[0] * t.rqz[j]) : rd2.x[f];
+            const double ke = kappa_eff(p, les ? 0.5 * (NUT(0, e) + NUT(0, e + 1)) : 0.0, dtde, wd, sqt);
+            if (AX) {
+                fl.x[f] = o + (dx * (e == 0 ? wE : t.dz[j] * t.rdyf[0]) * dtdc) * ke;
+            } else {
+                double a = 0.0, b = 0.0, c = 0.0;
+                if (e == 0) { a = m.g11[f]; b = m.g12[f]; c = m.g13[f]; }
+                else {                       // face 0 has its own metrics
+                    const R3<double> n = ld3(m.icsi, f);
+                    const double w = m.iaj[f];
+                    a = dot3(ld3(m.icsi, f), n) * w; b = dot3(ld3(m.ieta, f), n) * w; c = dot3(ld3(m.izet, f), n) * w;
+                }
+                fl.x[f] = o + (a * dtdc + b * dtde + c * dtdz) * ke;
             }
-            fl.x[f] = o + (a * dtdc + b * dtde + c * dtdz) * ke;
-        }
-    };
-    // ---- j face fj = j + e (Compute_dscalar_j, inline.h:3252-3289)
-    auto jface = [&](int fj, int e) {
-        const int f = g.lin(k, fj, i);
-        const bool edge = (fj == 0 || fj == my - 2);
-        const double dtde = T(0, e + 1, 0) - T(0, e, 0);
-        double dtdc = 0.0, dtdz = 0.0;
-        if (!AX) {
-            if (i == mx - 2 && edge && (npi || npj))  dtdc = (T(0, e + 1, 0) + T(0, e, 0) - T(0, e + 1, -1) - T(0, e, -1)) * 0.5;
-            else if (i == 1 && edge && (npi || npj))  dtdc = (T(0, e + 1, 1) + T(0, e, 1) - T(0, e + 1, 0) - T(0, e, 0)) * 0.5;
-            else                                      dtdc = (T(0, e + 1, 1) + T(0, e, 1) - T(0, e + 1, -1) - T(0, e, -1)) * 0.25;
-            if (k == mz - 2 && edge && (npk || npj))  dtdz = (T(0, e + 1, 0) + T(0, e, 0) - T(-1, e + 1, 0) - T(-1, e, 0)) * 0.5;
-            else if (k == 1 && edge && (npk || npj))  dtdz = (T(1, e + 1, 0) + T(1, e, 0) - T(0, e + 1, 0) - T(0, e, 0)) * 0.5;
-            else                                      dtdz = (T(1, e + 1, 0) + T(1, e, 0) - T(-1, e + 1, 0) - T(-1, e, 0)) * 0.25;
-        }
-        double o = 0.0;
-        if (mode != 2) {
-            const double uc = s.ucont.y[f];
-            double w;
-            if (edge) {
-                int jL, jR;
-                stencil4(fj, my, g.pj, jL, jR);
-                w = weno3(TG(k, jL, i), T(0, e, 0), T(0, e + 1, 0), TG(k, jR, i), uc);
-            } else w = weno3(T(0, e - 1, 0), T(0, e, 0), T(0, e + 1, 0), T(0, e + 2, 0), uc);
-            o = -uc * w;
-        }
-        if (mode == 1) { fl.y[f] = o; return; }
-        const double wd = !p.les ? 0.0 : AX ? t.rqx[k] * t.rqy[i] * t.rqzf[fj] : rd2.y[f];
-        double ke = kappa_eff(p, p.les ? 0.5 * (NUT(0, e, 0) + NUT(0, e + 1, 0)) : 0.0, dtde, wd, sqt);
-        double v0 = 0.0;
-        if (p.t_wall && fj == 0) {
-            // thetaWallFunction (teqn_solvers.c:337-352): the modelled flux
-            // -qWall . jEta, qWall = (0, 0, q), replaces the diffusive one
-            const R3<double> et = ld3(m.jeta, f);
-            v0 = -1.0 * (0.0 * et.x + 0.0 * et.y + s.qwall[k * mx + i] * et.z);
-            ke = 0.0;
-        }
-        if (AX) {
-            fl.y[f] = o + (v0 + (t.dx[k] * t.dy[i] * t.rdzf[fj] * dtde) * ke);
-        } else {
-            double a = 0.0, b = 0.0, c = 0.0;
-            if (e == 0) { a = m.g21[f]; b = m.g22[f]; c = m.g23[f]; }
-            else {                       // face 0 has its own metrics
-                const R3<double> n = ld3(m.jeta, f);
-                const double w = m.jaj[f];
-                a = dot3(ld3(m.jcsi, f), n) * w; b = dot3(ld3(m.jeta, f), n) * w; c = dot3(ld3(m.jzet, f), n) * w;
+        };
+        // ---- j face fj = j + e (Compute_dscalar_j, inline.h:3252-3289)
+        auto jface = [&](int fj, int e) {
+            const int f = g.lin(k, fj, i);
+            const double dtde = T(0, e + 1, 0) - T(0, e, 0);
+            double dtdc = 0.0, dtdz = 0.0, o = 0.0;
+            if (!AX) {
+                dtdc = (T(0, e + 1, 1) + T(0, e, 1) - T(0, e + 1, -1) - T(0, e, -1)) * 0.25;
+                dtdz = (T(1, e + 1, 0) + T(1, e, 0) - T(-1, e + 1, 0) - T(-1, e, 0)) * 0.25;
             }
-            fl.y[f] = o + (v0 + (a * dtdc + b * dtde + c * dtdz) * ke);
-        }
-    };
-    // ---- k face fk = k + e (Compute_dscalar_k, inline.h:3294-3331)
-    auto kface = [&](int fk, int e) {
-        const int f = g.lin(fk, j, i);
-        const bool edge = (fk == 0 || fk == mz - 2);
-        double dtdc = 0.0, dtde;
-        if (!AX) {
-            if (i == mx - 2 && edge && (npi || npk))  dtdc = (T(e + 1, 0, 0) + T(e, 0, 0) - T(e + 1, 0, -1) - T(e, 0, -1)) * 0.5;
-            else if (i == 1 && edge && (npi || npk))  dtdc = (T(e + 1, 0, 1) + T(e, 0, 1) - T(e + 1, 0, 0) - T(e, 0, 0)) * 0.5;
-            else                                      dtdc = (T(e + 1, 0, 1) + T(e, 0, 1) - T(e + 1, 0, -1) - T(e, 0, -1)) * 0.25;
-        }
-        if (j == my - 2 && edge && (npj || npk))      dtde = (T(e + 1, 0, 0) + T(e, 0, 0) - T(e + 1, -1, 0) - T(e, -1, 0)) * 0.5;
-        else if (j == 1 && edge && (npj || npk))      dtde = (T(e + 1, 1, 0) + T(e, 1, 0) - T(e + 1, 0, 0) - T(e, 0, 0)) * 0.5;
-        else                                          dtde = (T(e + 1, 1, 0) + T(e, 1, 0) - T(e + 1, -1, 0) - T(e, -1, 0)) * 0.25;
-        const double dtdz = T(e + 1, 0, 0) - T(e, 0, 0);
-        double o = 0.0;
-        if (mode != 2) {
-            const double uc = s.ucont.z[f];
-            double w;
-            if (edge) {
-                int kL, kR;
-                stencil4(fk, mz, g.pk, kL, kR);
-                w = weno3(TG(kL, j, i), T(e, 0, 0), T(e + 1, 0, 0), TG(kR, j, i), uc);
-            } else w = weno3(T(e - 1, 0, 0), T(e, 0, 0), T(e + 1, 0, 0), T(e + 2, 0, 0), uc);
-            o = -uc * w;
-        }
-        if (mode == 1) { fl.z[f] = o; return; }
-        const double wd = !p.les ? 0.0 : AX ? t.rqxf[fk] * t.rqy[i] * t.rqz[j] : rd2.z[f];
-        const double ke = kappa_eff(p, p.les ? 0.5 * (NUT(e, 0, 0) + NUT(e + 1, 0, 0)) : 0.0, dtde, wd, sqt);
-        if (AX) {
-            fl.z[f] = o + (t.dy[i] * t.dz[j] * t.rdxf[fk] * dtdz) * ke;
-        } else {
-            double a = 0.0, b = 0.0, c = 0.0;
-            if (e == 0) { a = m.g31[f]; b = m.g32[f]; c = m.g33[f]; }
-            else {                       // face 0 has its own metrics
-                const R3<double> n = ld3(m.kzet, f);
-                const double w = m.kaj[f];
-                a = dot3(ld3(m.kcsi, f), n) * w; b = dot3(ld3(m.keta, f), n) * w; c = dot3(ld3(m.kzet, f), n) * w;
+            const double uc = mode != 2 ? s.ucont.y[f] : 0.0;
+            if (fj == 0 || fj == my - 2) {
+                if (!AX && (npi || npj)) {
+                    if (i == mx - 2)   dtdc = (T(0, e + 1, 0) + T(0, e, 0) - T(0, e + 1, -1) - T(0, e, -1)) * 0.5;
+                    else if (i == 1)   dtdc = (T(0, e + 1, 1) + T(0, e, 1) - T(0, e + 1, 0) - T(0, e, 0)) * 0.5;
+                }
+                if (!AX && (npk || npj)) {
+                    if (k == mz - 2)   dtdz = (T(0, e + 1, 0) + T(0, e, 0) - T(-1, e + 1, 0) - T(-1, e, 0)) * 0.5;
+                    else if (k == 1)   dtdz = (T(1, e + 1, 0) + T(1, e, 0) - T(0, e + 1, 0) - T(0, e, 0)) * 0.5;
+                }
+                if (mode != 2) {
+                    int jL, jR;
+                    stencil4(fj, my, g.pj, jL, jR);
+                    o = -uc * weno3(TG(k, jL, i), T(0, e, 0), T(0, e + 1, 0), TG(k, jR, i), uc);
+                }
+            } else if (mode != 2) o = -uc * weno3(T(0, e - 1, 0), T(0, e, 0), T(0, e + 1, 0), T(0, e + 2, 0), uc);
+            if (mode == 1) { fl.y[f] = o; return; }
+            const double wd = !les ? 0.0 : AX ? rqx * (e == 0 ? qN : t.rqy[i] * t.rqzf[0]) : rd2.y[f];
+            double ke = kappa_eff(p, les ? 0.5 * (NUT(e, 0) + NUT(e + 1, 0)) : 0.0, dtde, wd, sqt);
+            double v0 = 0.0;
+            if (p.t_wall && fj == 0) {
+                // thetaWallFunction (teqn_solvers.c:337-352): the modelled flux
+                // -qWall . jEta, qWall = (0, 0, q), replaces the diffusive one
+                const R3<double> et = ld3(m.jeta, f);
+                v0 = -1.0 * (0.0 * et.x + 0.0 * et.y + s.qwall[k * mx + i] * et.z);
+                ke = 0.0;
             }
-            fl.z[f] = o + (a * dtdc + b * dtde + c * dtdz) * ke;
-        }
-    };
-    const int ni = (i == 1 && npi) ? 2 : 1, nj = (j == 1 && npj) ? 2 : 1, nk = (k == 1 && npk) ? 2 : 1;
+            if (AX) {
+                fl.y[f] = o + (v0 + (dx * (e == 0 ? wN : t.dy[i] * t.rdzf[0]) * dtde) * ke);
+            } else {
+                double a = 0.0, b = 0.0, c = 0.0;
+                if (e == 0) { a = m.g21[f]; b = m.g22[f]; c = m.g23[f]; }
+                else {                       // face 0 has its own metrics
+                    const R3<double> n = ld3(m.jeta, f);
+                    const double w = m.jaj[f];
+                    a = dot3(ld3(m.jcsi, f), n) * w; b = dot3(ld3(m.jeta, f), n) * w; c = dot3(ld3(m.jzet, f), n) * w;
+                }
+                fl.y[f] = o + (v0 + (a * dtdc + b * dtde + c * dtdz) * ke);
+            }
+        };
+        // ---- k face fk = k + e (Compute_dscalar_k, inline.h:3294-3331). A and B: the
+        // planes of its two cells, Z and C: those before and after
+        auto kface = [&](int fk, int e, const double *Z, const double *A, const double *B, const double *C) {
+            const int f = g.lin(fk, j, i);
+            double dtdc = 0.0, dtde = (B[TTX] + A[TTX] - B[-TTX] - A[-TTX]) * 0.25, o = 0.0;
+            if (!AX) dtdc = (B[1] + A[1] - B[-1] - A[-1]) * 0.25;
+            const double dtdz = B[0] - A[0], uc = mode != 2 ? s.ucont.z[f] : 0.0;
+            if (fk == 0 || fk == mz - 2) {
+                if (!AX && (npi || npk)) {
+                    if (i == mx - 2)   dtdc = (B[0] + A[0] - B[-1] - A[-1]) * 0.5;
+                    else if (i == 1)   dtdc = (B[1] + A[1] - B[0] - A[0]) * 0.5;
+                }
+                if (npj || npk) {
+                    if (j == my - 2)   dtde = (B[0] + A[0] - B[-TTX] - A[-TTX]) * 0.5;
+                    else if (j == 1)   dtde = (B[TTX] + A[TTX] - B[0] - A[0]) * 0.5;
+                }
+                if (mode != 2) {
+                    int kL, kR;
+                    stencil4(fk, mz, g.pk, kL, kR);
+                    o = -uc * weno3(TG(kL, j, i), A[0], B[0], TG(kR, j, i), uc);
+                }
+            } else if (mode != 2) o = -uc * weno3(Z[0], A[0], B[0], C[0], uc);
+            if (mode == 1) { fl.z[f] = o; return; }
+            const double wd = !les ? 0.0 : AX ? t.rqxf[fk] * qT : rd2.z[f];
+            const double ke = kappa_eff(p, les ? 0.5 * (A[TTN] + B[TTN]) : 0.0, dtde, wd, sqt);
+            if (AX) {
+                fl.z[f] = o + (wT * t.rdxf[fk] * dtdz) * ke;
+            } else {
+                double a = 0.0, b = 0.0, c = 0.0;
+                if (e == 0) { a = m.g31[f]; b = m.g32[f]; c = m.g33[f]; }
+                else {                       // face 0 has its own metrics
+                    const R3<double> n = ld3(m.kzet, f);
+                    const double w = m.kaj[f];
+                    a = dot3(ld3(m.kcsi, f), n) * w; b = dot3(ld3(m.keta, f), n) * w; c = dot3(ld3(m.kzet, f), n) * w;
+                }
+                fl.z[f] = o + (a * dtdc + b * dtde + c * dtdz) * ke;
+            }
+        };
 #pragma unroll 1
-    for (int e = 0; e > -ni; e--) iface(i + e, e);
+        for (int e = 0; e > -ni; e--) iface(i + e, e);
 #pragma unroll 1
-    for (int e = 0; e > -nj; e--) jface(j + e, e);
-#pragma unroll 1
-    for (int e = 0; e > -nk; e--) kface(k + e, e);
+        for (int e = 0; e > -nj; e--) jface(j + e, e);
+        kface(k, 0, Pm, P0, P1, P2);
+        if (k == 1 && npk) kface(0, -1, Pm, Pm, P0, P1);      // its outer points are not in the ring
+    }
 }
 
 // FormT pass 1 on the context's stream
@@ -276,12 +298,22 @@ template <int mode>
 void t_face_fluxes(tg_ctx *C)
 {
     const Grid g = C->g;
-    const dim3 gr((g.mx - 2 + TBX - 1) / TBX, (g.my - 2 + TBY - 1) / TBY, (g.mz - 2 + TBZ - 1) / TBZ), bl(TBX, TBY, TBZ);
+    const int nbi = (g.mx - 2 + TBX - 1) / TBX, nbj = (g.my - 2 + TBY - 1) / TBY, nk = g.mz - 2;
+    // planes per block: every chunk costs about three planes of start-up, every
+    // started wave of four blocks per SM a chunk
+    int kc = nk;
+    int64_t best = INT64_MAX;
+    for (int ch = 1; ch <= std::max(1, nk / 2); ch++) {
+        const int c = (nk + ch - 1) / ch;
+        const int64_t waves = ((int64_t)nbi * nbj * ((nk + c - 1) / c) + 4 * 148 - 1) / (4 * 148), cost = waves * (c + 3);
+        if (cost < best) { best = cost; kc = c; }
+    }
+    const dim3 gr(nbi * nbj * ((nk + kc - 1) / kc)), bl(TBX, TBY);
     State &s = C->s;
     if (C->axis_aligned)
-        TG_PROF(C, "teqn_face_fluxes", (k_t_face_fluxes<true, mode><<<gr, bl, 0, C->stream>>>(g, C->m, C->ts, s, C->prm, s.trd2, s.tflux)));
+        TG_PROF(C, "teqn_face_fluxes", (k_t_face_fluxes<true, mode><<<gr, bl, 0, C->stream>>>(g, C->m, C->ts, s, C->prm, s.trd2, s.tflux, nbi, nbj, kc)));
     else
-        TG_PROF(C, "teqn_face_fluxes", (k_t_face_fluxes<false, mode><<<gr, bl, 0, C->stream>>>(g, C->m, C->ts, s, C->prm, s.trd2, s.tflux)));
+        TG_PROF(C, "teqn_face_fluxes", (k_t_face_fluxes<false, mode><<<gr, bl, 0, C->stream>>>(g, C->m, C->ts, s, C->prm, s.trd2, s.tflux, nbi, nbj, kc)));
 }
 
 // pass 2 (teqn_solvers.c:520-566): the flux budget of interior cell c times aj,
