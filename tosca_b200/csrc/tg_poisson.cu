@@ -381,12 +381,11 @@ __global__ void k_cg_dir(int64_t n, const double *sc, const double *z, double *p
 // residual to near rounding at once, so directions need no conjugation: each
 // pass takes z = M r and the step length that CG's first iteration takes,
 // alpha = (r, z) / (z, L z), and reads z where CG reads its direction p. The
-// vector work of a solve is four kernels instead of 14 launches (256 x 256 x 128:
-// 0.61 ms before, 0.44 ms now, of 0.39 ms for their bytes), each with its dot
-// products finished by the last block to arrive. The row loops are unrolled by
-// four: on small grids a row is a handful of loads whose latency nothing else
-// hides (a step of 75 x 75 x 25 0.241 -> 0.238 ms, of 32^3 0.119 -> 0.118 ms). Threads take rows of the compact grid (a
-// warp per row, lanes along i), so that 3-D indices cost one division per row.
+// vector work of a solve is four kernels instead of 14 launches, each with its dot
+// products finished by the last block to arrive (256 x 256 x 128: 0.61 ms before,
+// 0.37 ms now, of 0.30 ms for their bytes). In k_direct_begin a warp takes a row of
+// the compact grid, lanes along i, so that 3-D indices cost one division per row;
+// the two that apply the operator march along k (op7_march).
 struct Rows {
     int nx, ny, nrow, lane, row, step;
     __device__ __forceinline__ Rows(const PoissonCtx &P)
@@ -476,70 +475,74 @@ __global__ void __launch_bounds__(RB) k_direct_begin(Grid g, State s, PoissonCtx
     }
 }
 
-// (L x)_c of k_apply7 at column i of a row; FAC: coefficients from their factors
-template <bool FAC>
-struct Op7 {
-    const PoissonCtx &P;
-    const double *x;
-    int c0, oN, oS, oT, oB;
-    bool hN, hS, hT, hB;
-    double e, nN, nS, tT, tB;         // row factors
-    __device__ __forceinline__ Op7(const PoissonCtx &P_, const double *x_, int row) : P(P_), x(x_)
-    {
-        const int jc = row % P.ny, kc = row / P.ny, nx = P.nx, pl = nx * P.ny;
-        c0 = row * nx;
-        oN = jc < P.ny - 1 ? nx : nx - pl; oS = jc > 0 ? -nx : pl - nx;
-        oT = kc < P.nz - 1 ? pl : pl - pl * P.nz; oB = kc > 0 ? -pl : pl * P.nz - pl;
-        hN = jc < P.ny - 1 || P.pj; hS = jc > 0 || P.pj; hT = kc < P.nz - 1 || P.pk; hB = kc > 0 || P.pk;
+// f(c, x_c, (L x)_c) of k_apply7 for every cell; FAC: coefficients from their
+// factors. A block takes 32 x 8 columns (a warp per j) of kc cells along k and
+// holds the column's cell, the one below and the one above in registers.
+// Latency-bound: with rows of i per warp, whose loads waited for the stores of the
+// cells before them (no read-only loads) and which fetched each x three times
+// from L2, r = b - L x took 137 us at 256 x 256 x 128 and the dot products 89 us; now
+// 77 and 69, of 41 and 31 us for their bytes. A step of 256 x 256 x 128 went 3.07 -> 3.00 ms, of
+// 192 x 192 x 96 1.461 -> 1.430 ms, and those of 75 x 75 x 25 and 32^3 stayed. Read-only
+// loads in the rows alone gave nothing; three blocks per SM (80 registers, unrolled
+// by four) 3.09 ms, five 3.015 ms.
+template <bool FAC, class F>
+__device__ __forceinline__ void op7_march(const PoissonCtx &P, const double *x, int kc, F f)
+{
+    const int nx = P.nx, ny = P.ny, nz = P.nz, pl = nx * ny, nbi = (nx + 31) / 32, nbj = (ny + RB / 32 - 1) / (RB / 32), nt = nbi * nbj * ((nz + kc - 1) / kc);
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int i = t % nbi * 32 + (threadIdx.x & 31), j = t / nbi % nbj * (RB / 32) + (threadIdx.x >> 5), k0 = t / (nbi * nbj) * kc, k1 = min(k0 + kc, nz);
+        if (i >= nx || j >= ny) continue;
+        // a face without a flux has a zero coefficient; its offset wraps inside the grid
+        const int oE = i < nx - 1 ? 1 : 1 - nx, oW = i > 0 ? -1 : nx - 1, oN = j < ny - 1 ? nx : nx - pl, oS = j > 0 ? -nx : pl - nx;
+        const bool hE = i < nx - 1 || P.pi, hW = i > 0 || P.pi, hN = j < ny - 1 || P.pj, hS = j > 0 || P.pj;
+        double m = 0.0, my = 0.0, kE = 0.0, kW = 0.0, kN = 0.0, kS = 0.0;
         if (FAC) {
-            const double my = P.op.my[jc], mz = P.op.mz[kc];
-            e = my * mz;
-            nN = hN ? P.op.ky[jc] * mz : 0.0; nS = hS ? P.op.ky[jc > 0 ? jc - 1 : P.ny - 1] * mz : 0.0;
-            tT = hT ? P.op.kz[kc] * my : 0.0; tB = hB ? P.op.kz[kc > 0 ? kc - 1 : P.nz - 1] * my : 0.0;
+            m = P.op.mx[i]; my = P.op.my[j];
+            kE = hE ? P.op.kx[i] : 0.0; kW = hW ? P.op.kx[i > 0 ? i - 1 : nx - 1] : 0.0;
+            kN = hN ? P.op.ky[j] : 0.0; kS = hS ? P.op.ky[j > 0 ? j - 1 : ny - 1] : 0.0;
+        }
+        int c = (k0 * ny + j) * nx + i;
+        double xb = __ldg(x + c + (k0 > 0 ? -pl : pl * nz - pl)), xc = __ldg(x + c);
+        double gb = k0 > 0 || P.pk ? (FAC ? P.op.kz[k0 > 0 ? k0 - 1 : nz - 1] * my : __ldg(P.gT3 + c + (k0 > 0 ? -pl : pl * nz - pl))) : 0.0;
+        #pragma unroll 2
+        for (int k = k0; k < k1; k++, c += pl) {
+            const bool top = k < nz - 1;
+            const double xt = __ldg(x + (top ? c + pl : c + pl - pl * nz)), xe = __ldg(x + c + oE), xw = __ldg(x + c + oW), xn = __ldg(x + c + oN), xs = __ldg(x + c + oS);
+            double acc = 0.0, gt = 0.0;
+            if (FAC) {
+                const double mz = __ldg(P.op.mz + k), e = my * mz;
+                if (top || P.pk) gt = __ldg(P.op.kz + k) * my;
+                acc += (kE * e) * (xc - xe);
+                acc += (kW * e) * (xc - xw);
+                acc += (m * (kN * mz)) * (xc - xn);
+                acc += (m * (kS * mz)) * (xc - xs);
+                acc += (m * gt) * (xc - xt);
+                acc += (m * gb) * (xc - xb);
+            } else {
+                if (top || P.pk) gt = __ldg(P.gT3 + c);
+                acc += (hE ? __ldg(P.gE1 + c) : 0.0) * (xc - xe);
+                acc += (hW ? __ldg(P.gE1 + c + oW) : 0.0) * (xc - xw);
+                acc += (hN ? __ldg(P.gN2 + c) : 0.0) * (xc - xn);
+                acc += (hS ? __ldg(P.gN2 + c + oS) : 0.0) * (xc - xs);
+                acc += gt * (xc - xt);
+                acc += gb * (xc - xb);
+            }
+            f(c, xc, acc);
+            xb = xc; xc = xt; gb = gt;
         }
     }
-    __device__ __forceinline__ double at(int i) const
-    {
-        const int nx = P.nx, c = c0 + i, ce = i < nx - 1 ? c + 1 : c + 1 - nx, cw = i > 0 ? c - 1 : c - 1 + nx;
-        const bool hE = i < nx - 1 || P.pi, hW = i > 0 || P.pi;
-        const double xc = x[c];
-        double acc = 0.0;
-        if (FAC) {
-            const double m = P.op.mx[i];
-            if (hE) acc += (P.op.kx[i] * e) * (xc - x[ce]);
-            if (hW) acc += (P.op.kx[i > 0 ? i - 1 : nx - 1] * e) * (xc - x[cw]);
-            if (hN) acc += (m * nN) * (xc - x[c + oN]);
-            if (hS) acc += (m * nS) * (xc - x[c + oS]);
-            if (hT) acc += (m * tT) * (xc - x[c + oT]);
-            if (hB) acc += (m * tB) * (xc - x[c + oB]);
-        } else {
-            if (hE) acc += P.gE1[c] * (xc - x[ce]);
-            if (hW) acc += P.gE1[cw] * (xc - x[cw]);
-            if (hN) acc += P.gN2[c] * (xc - x[c + oN]);
-            if (hS) acc += P.gN2[c + oS] * (xc - x[c + oS]);
-            if (hT) acc += P.gT3[c] * (xc - x[c + oT]);
-            if (hB) acc += P.gT3[c + oB] * (xc - x[c + oB]);
-        }
-        return acc;
-    }
-};
+}
 
 // r = b - L x with |r|^2, sum r and max |r aj| (sc[3..5]), and the loop's start
 template <bool FAC, bool CAP>
-__global__ void __launch_bounds__(RB) k_direct_resid(const __grid_constant__ PoissonCtx P, const double *w, double *sc, Loop L, cudaGraphConditionalHandle h)
+__global__ void __launch_bounds__(RB, 4) k_direct_resid(const __grid_constant__ PoissonCtx P, const double *w, int kc, double *sc, Loop L, cudaGraphConditionalHandle h)
 {
-    const Rows R(P);
     double v[3] = {0.0, 0.0, 0.0};
-    for (int row = R.row; row < R.nrow; row += R.step) {
-        const Op7<FAC> op(P, P.x, row);
-        #pragma unroll 4
-        for (int i = R.lane; i < R.nx; i += 32) {
-            const int c = op.c0 + i;
-            const double r = c == P.pin ? P.b[c] - P.x[c] : P.b[c] - op.at(i);
-            P.r[c] = r;
-            dot_acc(r, r, w ? w[c] : 0.0, v);
-        }
-    }
+    op7_march<FAC>(P, P.x, kc, [&](int c, double x, double Lx) {
+        const double r = __ldg(P.b + c) - (c == P.pin ? x : Lx);
+        P.r[c] = r;
+        dot_acc(r, r, w ? __ldg(w + c) : 0.0, v);
+    });
     dot_store(v, P.part);
     if (last_block(P.count)) {
         total<3, true>(P.part, v);
@@ -552,22 +555,16 @@ __global__ void __launch_bounds__(RB) k_direct_resid(const __grid_constant__ Poi
 
 // q = L z (zero at the pin) with (r, z - z_0) and (z - z_0, q) (sc[6], sc[9])
 template <bool FAC>
-__global__ void __launch_bounds__(RB) k_direct_dots(const __grid_constant__ PoissonCtx P, double *sc)
+__global__ void __launch_bounds__(RB, 4) k_direct_dots(const __grid_constant__ PoissonCtx P, int kc, double *sc)
 {
-    const Rows R(P);
     const double z0 = P.z[0];
     double v[3] = {0.0, 0.0, 0.0};
-    for (int row = R.row; row < R.nrow; row += R.step) {
-        const Op7<FAC> op(P, P.z, row);
-        #pragma unroll 4
-        for (int i = R.lane; i < R.nx; i += 32) {
-            const int c = op.c0 + i;
-            const double q = c == P.pin ? 0.0 : op.at(i), z = P.z[c] - z0;
-            P.q[c] = q;
-            v[0] += P.r[c] * z;
-            v[1] += z * q;
-        }
-    }
+    op7_march<FAC>(P, P.z, kc, [&](int c, double zc, double Lz) {
+        const double q = c == P.pin ? 0.0 : Lz, z = zc - z0;
+        P.q[c] = q;
+        v[0] += __ldg(P.r + c) * z;
+        v[1] += z * q;
+    });
     block_reduce<RB>(v, RedSum{}, RedSum{}, RedMax{});
     if (threadIdx.x == 0) { P.part[2 * blockIdx.x] = v[0]; P.part[2 * blockIdx.x + 1] = v[1]; }
     if (last_block(P.count)) {
@@ -710,6 +707,23 @@ static void read_scal(tg_ctx *C, int off, int cnt)
 
 static Loop loop_of(tg_ctx *C, double rtol, double divtol, int maxit, int base) { return Loop{rtol, divtol, C->prm.dt, maxit, base}; }
 
+// blocks and cells along k per block of op7_march: every chunk costs about two
+// cells of start-up, every started wave of four blocks per SM a chunk
+struct March {
+    int kc, nb;
+    explicit March(const PoissonCtx &P) : kc(P.nz)
+    {
+        const int64_t cols = (int64_t)((P.nx + 31) / 32) * ((P.ny + RB / 32 - 1) / (RB / 32));
+        int64_t best = INT64_MAX;
+        for (int ch = 1; ch <= P.nz; ch++) {
+            const int c = (P.nz + ch - 1) / ch;
+            const int64_t waves = (cols * ((P.nz + c - 1) / c) + 4 * 148 - 1) / (4 * 148), cost = waves * (c + 2);
+            if (cost < best) { best = cost; kc = c; }
+        }
+        nb = (int)std::min<int64_t>(cols * ((P.nz + kc - 1) / kc), P.nblocks);
+    }
+};
+
 // one pass of the direct solver's iteration; CAP: inside the captured loop
 template <bool CAP>
 static void direct_pass(tg_ctx *C, const Loop &L, cudaGraphConditionalHandle h)
@@ -717,9 +731,10 @@ static void direct_pass(tg_ctx *C, const Loop &L, cudaGraphConditionalHandle h)
     PoissonCtx &P = *C->pois;
     cudaStream_t s = C->stream;
     double *sc = C->d_scal;
+    const March march(P);
     fdm_apply(C, P.fdm, P.r, sc + 4, P.z);
-    if (P.op_exact) TG_PROF(C, "pois_dots", k_direct_dots<true><<<P.nblocks, RB, 0, s>>>(P, sc));
-    else TG_PROF(C, "pois_dots", k_direct_dots<false><<<P.nblocks, RB, 0, s>>>(P, sc));
+    if (P.op_exact) TG_PROF(C, "pois_dots", k_direct_dots<true><<<march.nb, RB, 0, s>>>(P, march.kc, sc));
+    else TG_PROF(C, "pois_dots", k_direct_dots<false><<<march.nb, RB, 0, s>>>(P, march.kc, sc));
     TG_PROF(C, "pois_update", (k_direct_update<CAP><<<P.nblocks, RB, 0, s>>>(P, L.divtol > 0 ? P.aj : nullptr, sc, L, h)));
 }
 template <bool CAP>
@@ -727,8 +742,9 @@ static void direct_resid(tg_ctx *C, const Loop &L, cudaGraphConditionalHandle h)
 {
     PoissonCtx &P = *C->pois;
     const double *w = L.divtol > 0 ? P.aj : nullptr;
-    if (P.op_exact) TG_PROF(C, "pois_resid", (k_direct_resid<true, CAP><<<P.nblocks, RB, 0, C->stream>>>(P, w, C->d_scal, L, h)));
-    else TG_PROF(C, "pois_resid", (k_direct_resid<false, CAP><<<P.nblocks, RB, 0, C->stream>>>(P, w, C->d_scal, L, h)));
+    const March march(P);
+    if (P.op_exact) TG_PROF(C, "pois_resid", (k_direct_resid<true, CAP><<<march.nb, RB, 0, C->stream>>>(P, w, march.kc, C->d_scal, L, h)));
+    else TG_PROF(C, "pois_resid", (k_direct_resid<false, CAP><<<march.nb, RB, 0, C->stream>>>(P, w, march.kc, C->d_scal, L, h)));
 }
 
 // direct solve of L x = b from the current P.x (P.b and |b|^2 in sc[0] set by the caller)
