@@ -37,32 +37,37 @@ DIV_TOL = 5e-9
 # algorithmic bytes per interior cell of one launch, by storage precision of
 # the arrays the kernel reads (each array counted once per read and once per
 # write; metrics re-read every launch). The mixed mode reads FP32 copies of the
-# metrics (4 B) and keeps the state, fluxes and Krylov vectors in FP64. On an
-# axis-aligned mesh (tg_mesh_info) the stencil kernels read one component of
-# each metric vector.
+# metrics (4 B) and keeps the state, fluxes and Krylov vectors in FP64. On a
+# mesh of planes (tg_mesh_info's axis-aligned) the stencil kernels take the
+# metrics from six spacing arrays and read none of them, in either mode.
 def bytes_per_cell(kernel, precision, axis=False):
     m = 4 if precision == "mixed" else 8      # metric storage
     g = 4 if precision == "mixed" else 8      # multigrid storage
     if axis:
         table = {
-            # ucat 3, ucont 3, nut 1; per face the normal metric component of
-            # csi, eta, zet and aj (12) -> fluxes 9
+            # ucont 3, nut 1 -> fp 3 (explicit stages: Ucat is formed on the way)
+            "formu_stage_fp": 7 * 8,
+            # ucat 3, ucont 3, nut 1 -> fp 3
+            "formu_cell_fp": 10 * 8,
+            # ucat 3, ucont 3, nut 1; csi.y, eta.z, zet.x and aj of the three faces
+            # -> fluxes 9 (QUICK, which keeps the face-flux kernel)
             "formu_face_fluxes": 7 * 8 + 12 * m + 9 * 8,
-            # fp 3, dP 3, and the RK4 update applied in place (U_o, Utmp -> Utmp,
-            # U: 9, 12, 12, 6 values over the four stages); csi.y, eta.z, zet.x,
-            # face aj 3, icsi.y, jeta.z, kzet.x
-            "formu_rhs_faces": (6 + 39 / 4) * 8 + 9 * m,
-            # ucont 3 -> ucat 3; csi.y, eta.z, zet.x
-            "contra_to_cart": 6 * 8 + 3 * m,
-            # ucat 3 -> nut 1; csi.y, eta.z, zet.x, aj
-            "smagorinsky": 4 * 8 + 4 * m,
-            # p 1 -> dP 3; icsi.y, jeta.z, kzet.x and the face aj 3
-            "grad_p": 4 * 8 + 6 * m,
-            # phi 1, ucont 3 -> ucont 3; icsi.y, jeta.z, kzet.x and the face aj 3
-            "project": 7 * 8 + 6 * m,
-            # T 1, nut 1, ucont 3; icsi.y, jeta.z, kzet.x and the face aj 3 (FP64
-            # in every mode) -> convective and diffusive fluxes 6
-            "teqn_face_fluxes": (5 + 6 + 6) * 8,
+            # fp 3, p 1, and the RK4 update applied in place (U_o, Utmp -> Utmp,
+            # U: 9, 12, 12, 6 values over the four stages)
+            "formu_rhs_faces": (4 + 39 / 4) * 8,
+            # ucont 3 -> ucat 3
+            "contra_to_cart": 6 * 8,
+            "contra_div_final": 6 * 8,
+            # ucat 3 -> nut 1
+            "smagorinsky": 4 * 8,
+            # p 1 -> dP 3
+            "grad_p": 4 * 8,
+            # solution 1, p 1, ucont 3 -> phi 1, p 1, ucont 3
+            "pressure_project": 10 * 8,
+            # phi 1, ucont 3 -> ucont 3
+            "project": 7 * 8,
+            # T 1, nut 1, ucont 3 -> fluxes 3
+            "teqn_face_fluxes": 8 * 8,
         }
         if kernel in table:
             return table[kernel]
@@ -78,10 +83,10 @@ def bytes_per_cell(kernel, precision, axis=False):
         "contra_to_cart": 6 * 8 + 9 * m,
         # ucat 3 -> nut 1 (FP64); csi/eta/zet 9, aj 1
         "smagorinsky": 4 * 8 + 10 * m,
-        # p 1 -> dP 3 (FP64); face metrics 27 + 3
-        "grad_p": 4 * 8 + 30 * m,
-        # phi 1, ucont 3 -> ucont 3 (FP64); face metrics 27 + 3
-        "project": 7 * 8 + 30 * m,
+        # p 1 -> dP 3; the nine metric products of SetCoeffMatrix (FP64)
+        "grad_p": 4 * 8 + 9 * 8,
+        # phi 1, ucont 3 -> ucont 3; the nine metric products
+        "project": 7 * 8 + 9 * 8,
         # one zebra colour (half the cells): r, minv, aN, c', aE, aT, x of the
         # other colour -> x: 8 values per cell of the colour
         "mg_smooth_line_L0": 8 * g / 2,
@@ -94,8 +99,15 @@ def bytes_per_cell(kernel, precision, axis=False):
         "pois_cg_update": 48,          # x, r read/write; p, q read
         "pois_cg_dir": 24,             # z, p read; p write
         "pois_dot": 16,                # two vectors
-        # T 1, nut 1, ucont 3; face metrics 27 + 3 (FP64) -> fluxes 6
-        "teqn_face_fluxes": (5 + 30 + 6) * 8,
+        # the direct solver's iteration: ucont 3, x and its history 3 -> b, x, history 4;
+        # x, b, aj -> r; z, r -> q; x, z, r, q, aj -> x, r; a transform of one direction
+        "pois_begin": 10 * 8,
+        "pois_resid": 4 * 8,
+        "pois_dots": 3 * 8,
+        "pois_update": 7 * 8,
+        "fdm_x_fwd": 16, "fdm_x_inv": 16, "fdm_z_fwd": 16, "fdm_z_inv": 16,
+        # T 1, nut 1, ucont 3, filter width 3, the nine metric products -> fluxes 3
+        "teqn_face_fluxes": (5 + 3 + 9 + 3) * 8,
     }
     return table.get(kernel)
 

@@ -350,8 +350,9 @@ tg_status tg_momentum_info(tg_ctx *ctx, int32_t *outer, int32_t *inner, double *
 /* How the kernels classified the mesh set by tg_set_mesh_nodes: orthogonal
  * (every cross term of the face metric tensor is zero: 7-point pressure
  * operator, conjugate gradients) and axis-aligned (csi || y, eta || z,
- * zet || x up to round-off: the stencil kernels read one component of each
- * metric vector). */
+ * zet || x up to round-off, and every metric a product of 1-D spacings: a mesh
+ * of planes, whose kernels read the spacings and whose pressure solve is direct
+ * where its rules allow). Writing a metric field withdraws the latter. */
 tg_status tg_mesh_info(tg_ctx *ctx, int32_t *orthogonal, int32_t *axis_aligned);
 
 /* --------------------------------------------------------------- wind farm -- */
