@@ -349,10 +349,11 @@ tg_status tg_graph_info(tg_ctx *ctx, int64_t *replays, int32_t *capture_failed);
 tg_status tg_momentum_info(tg_ctx *ctx, int32_t *outer, int32_t *inner, double *residual);
 /* How the kernels classified the mesh set by tg_set_mesh_nodes: orthogonal
  * (every cross term of the face metric tensor is zero: 7-point pressure
- * operator, conjugate gradients) and axis-aligned (csi || y, eta || z,
- * zet || x up to round-off, and every metric a product of 1-D spacings: a mesh
- * of planes, whose kernels read the spacings and whose pressure solve is direct
- * where its rules allow). Writing a metric field withdraws the latter. */
+ * operator, conjugate gradients) and axis-aligned: a mesh of planes (x the same
+ * over each k plane, y over each i plane, z over each j plane, up to four units of
+ * rounding of the largest coordinate), whose kernels read 1-D spacings and whose
+ * pressure solve is direct where its rules allow. Writing a metric field withdraws
+ * the latter. */
 tg_status tg_mesh_info(tg_ctx *ctx, int32_t *orthogonal, int32_t *axis_aligned);
 
 /* --------------------------------------------------------------- wind farm -- */

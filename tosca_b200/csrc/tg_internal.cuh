@@ -194,10 +194,9 @@ struct tg_ctx {
     int red_blocks = 0;
     bool has_mesh = false;
     bool orthogonal = true;              // all cross metric-tensor terms vanish
-    // csi || y, eta || z, zet || x at every point of every cell and face
-    // metric up to round-off (the reference's i -> y, j -> z, k -> x axes on
-    // a mesh of planes), and every metric a product of the spacings in ts: the
-    // stage kernels of tg_tensor.cu run
+    // a mesh of planes along the reference's axes (i -> y, j -> z, k -> x), up to
+    // the rounding of its coordinates: the stage kernels of tg_tensor.cu run, on
+    // the spacings in ts
     bool axis_aligned = false;
     tg::Tensor ts{};
     double *ts_mem = nullptr;            // storage of ts
@@ -388,7 +387,7 @@ inline dim3 block3() { return dim3(BX, BY, BZ); }
 
 // stage kernels on a mesh of planes (tg_tensor.cu)
 struct RkArgs;
-bool tensor_setup(tg_ctx *C);
+bool tensor_setup(tg_ctx *C, const double *nodes, bool cross);   // nodes: the host array
 void contra_to_cart_tensor(tg_ctx *C, const char *name);
 void smagorinsky_tensor(tg_ctx *C);
 void grad_p_tensor(tg_ctx *C);

@@ -65,7 +65,11 @@ struct Cg {   // compact grid indexing with periodic wrap
 };
 
 // ------------------------------------------------------------ setup kernels
-__global__ void k_gather_g(Grid g, Metrics m, PoissonCtx P)
+// planes: the normal coefficients from the spacings that the projection reads
+// (k_pressure_project). The metrics give the same up to the rounding of the
+// coordinates, but a projection that differs from the operator it was solved with
+// leaves that much divergence.
+__global__ void k_gather_g(Grid g, Metrics m, Tensor t, bool planes, PoissonCtx P)
 {
     int ic = blockIdx.x * blockDim.x + threadIdx.x, jc = blockIdx.y * blockDim.y + threadIdx.y, kc = blockIdx.z * blockDim.z + threadIdx.z;
     if (ic >= P.nx || jc >= P.ny || kc >= P.nz) return;
@@ -75,6 +79,10 @@ __global__ void k_gather_g(Grid g, Metrics m, PoissonCtx P)
     P.gN1[c] = m.g21[d]; P.gN2[c] = m.g22[d]; P.gN3[c] = m.g23[d];
     P.gT1[c] = m.g31[d]; P.gT2[c] = m.g32[d]; P.gT3[c] = m.g33[d];
     P.aj[c] = m.aj[d];
+    if (planes) {
+        const double dx = t.dx[kc + 1], dy = t.dy[ic + 1], dz = t.dz[jc + 1];
+        P.gE1[c] = dx * dz * t.rdyf[ic + 1]; P.gN2[c] = dx * dy * t.rdzf[jc + 1]; P.gT3[c] = dy * dz * t.rdxf[kc + 1];
+    }
 }
 
 // --------------------------------------------------------- fine operators
@@ -681,7 +689,7 @@ void poisson_setup(tg_ctx *C)
     P->nblocks = vblocks(n);
     P->part = dallocd(C, 3 * (size_t)P->nblocks);
     P->count = (unsigned *)dalloc(C, sizeof(unsigned));
-    k_gather_g<<<cgrid(P->nx, P->ny, P->nz), block3(), 0, C->stream>>>(g, C->m, *P);
+    k_gather_g<<<cgrid(P->nx, P->ny, P->nz), block3(), 0, C->stream>>>(g, C->m, C->ts, C->axis_aligned, *P);
 
     P->fdm = P->ortho ? fdm_create(C, P->gE1, P->gN2, P->gT3, P->nx, P->ny, P->nz, P->pi, P->pj, P->pk) : nullptr;
     P->op_exact = P->fdm && fdm_factors(P->fdm, &P->op);

@@ -917,24 +917,44 @@ void set_fp_attrs()
 
 }  // namespace
 
-// The spacings of an axis-aligned mesh from its metrics, into C->ts; true if
-// every metric equals its product of spacings to 1e-13 (a mesh of planes
-// leaves the rounding of the products, some 1e-15).
-bool tensor_setup(tg_ctx *C)
+// Is the mesh one of planes (x depends on k alone, y on i, z on j), and if so its
+// spacings into C->ts. The question is put to the nodes and not to the metrics:
+// those form the same size by sums of different nodes and differ from each other by
+// some units of rounding of the coordinates over the spacing (2e-13 at 1300 cells
+// of 7.3 m, 1.4e-11 at map coordinates of 500 km), which says nothing about the
+// planes. A node may be off its plane by four units of rounding of the largest
+// coordinate. cross: the cross components of the metrics vanish to 1e-12; then nodes
+// further off count as well, as long as every metric is its product to 1e-12.
+bool tensor_setup(tg_ctx *C, const double *nodes, bool cross)
 {
     const Grid g = C->g;
     cudaStream_t st = C->stream;
-    auto line = [&](const double *a, int64_t first, int64_t stride, int n) {
-        std::vector<double> h(n);
-        TG_CUDA(cudaMemcpy2DAsync(h.data(), sizeof(double), a + first, stride * sizeof(double), sizeof(double), n, cudaMemcpyDeviceToHost, st));
-        TG_CUDA(cudaStreamSynchronize(st));
-        return h;
-    };
-    const int64_t pl = (int64_t)g.mx * g.my, o = g.lin(1, 1, 1);
-    const FaceMet<double> &m = C->fm64;
+    constexpr double EPS = 2.220446049250313e-16;
     const int n[3] = {g.mz, g.mx, g.my};                       // x, y, z
-    const int64_t first[3] = {o - pl, o - 1, o - g.mx}, stride[3] = {pl, 1, g.mx};
-    const double *area[3] = {m.zet.x, m.csi.y, m.eta.z}, *farea[3] = {m.kzet.x, m.icsi.y, m.jeta.z}, *fj[3] = {m.kaj, m.iaj, m.jaj};
+    const int64_t stride[3] = {(int64_t)g.mx * g.my, 1, g.mx};
+    const int per[3] = {g.pk, g.pi, g.pj};
+    std::vector<double> X[3];                                  // planes 0 .. n-2
+    double big[3], hmin[3], round = 0.0;
+    for (int q = 0; q < 3; q++) {
+        X[q].resize(n[q] - 1);
+        big[q] = 0.0; hmin[q] = HUGE_VAL;
+        for (int l = 0; l < n[q] - 1; l++) {
+            X[q][l] = nodes[3 * stride[q] * l + q];
+            big[q] = std::max(big[q], std::fabs(X[q][l]));
+            if (l > 0) hmin[q] = std::min(hmin[q], std::fabs(X[q][l] - X[q][l - 1]));
+        }
+        round += EPS * big[q] / hmin[q];
+    }
+    if (!std::isfinite(round)) return false;                   // coinciding planes, or no numbers
+    const double off[3] = {4 * EPS * big[0], 4 * EPS * big[1], 4 * EPS * big[2]};
+    bool planes = true;
+    for (int k = 0; k < g.mz - 1 && planes; k++)
+        for (int j = 0; j < g.my - 1 && planes; j++) {
+            const double *x = nodes + 3 * (int64_t)g.lin(k, j, 0);
+            for (int i = 0; i < g.mx - 1; i++, x += 3)
+                planes &= std::fabs(x[0] - X[0][k]) <= off[0] && std::fabs(x[1] - X[1][i]) <= off[1] && std::fabs(x[2] - X[2][j]) <= off[2];
+        }
+    if (!planes && !cross) return false;
     constexpr int NA = 7;        // arrays per direction
     if (!C->ts_mem) C->ts_mem = dallocd(C, NA * ((size_t)g.mx + g.my + g.mz));
     double *mem = C->ts_mem;
@@ -943,31 +963,39 @@ bool tensor_setup(tg_ctx *C)
                                {&t.dy, &t.rdy, &t.dyf, &t.rdyf, &t.qy, &t.rqy, &t.rqyf},
                                {&t.dz, &t.rdz, &t.dzf, &t.rdzf, &t.qz, &t.rqz, &t.rqzf}};
     for (int q = 0; q < 3; q++) {
-        // size = volume / area at the cells of the line through (1, 1, 1), with
-        // its ghosts, and across the faces 0 .. m-2
-        const std::vector<double> aj = line(m.aj, first[q], stride[q], n[q]), a = line(area[q], first[q], stride[q], n[q]),
-                                  fa = line(farea[q], first[q], stride[q], n[q]), fv = line(fj[q], first[q], stride[q], n[q]);
-        std::vector<double> h(NA * (size_t)n[q], 0.0);
-        for (int l = 0; l < n[q]; l++) {
-            const double r = aj[l] * a[l], rf = fv[l] * fa[l];
-            h[l] = 1.0 / r; h[n[q] + l] = r;
-            if (l < n[q] - 1) { h[2 * n[q] + l] = 1.0 / rf; h[3 * n[q] + l] = rf; }
+        // cell sizes with those of the ghosts (mirrored, or the opposite cell's), and the
+        // distances across the faces 0 .. m-2 as the face metrics take them
+        // (mesh.c:1354-1930): half the distance of the planes on either side, one-sided at
+        // an end, averaged over the seam at face m-2 of a periodic direction
+        const int m = n[q];
+        std::vector<double> h(NA * (size_t)m, 0.0);
+        auto size = [&](int l) { return X[q][l] - X[q][l - 1]; };
+        for (int l = 0; l < m; l++) {
+            const double s = size(l == 0 ? (per[q] ? m - 2 : 1) : l == m - 1 ? (per[q] ? 1 : m - 2) : l);
+            const double f = l == 0 ? size(1) : l < m - 2 ? 0.5 * (X[q][l + 1] - X[q][l - 1]) : per[q] ? 0.5 * (size(1) + size(m - 2)) : size(m - 2);
+            h[l] = s; h[m + l] = 1.0 / s;
+            if (l < m - 1) { h[2 * m + l] = f; h[3 * m + l] = 1.0 / f; }
             auto sq = [](double x) { return std::cbrt(x) * std::cbrt(x); };
-            h[4 * n[q] + l] = sq(h[l]);                         // (dx dy dz)^(2/3) by factors
-            h[5 * n[q] + l] = sq(r);
-            if (l < n[q] - 1) h[6 * n[q] + l] = sq(rf);
+            h[4 * m + l] = sq(h[l]);                            // (dx dy dz)^(2/3) by factors
+            h[5 * m + l] = sq(h[m + l]);
+            if (l < m - 1) h[6 * m + l] = sq(h[3 * m + l]);
         }
         TG_CUDA(cudaMemcpyAsync(mem, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, st));
         TG_CUDA(cudaStreamSynchronize(st));
-        for (int e = 0; e < NA; e++) *d[q][e] = mem + (size_t)e * n[q];
+        for (int e = 0; e < NA; e++) *d[q][e] = mem + (size_t)e * m;
         mem += h.size();
     }
-    k_tensor_check<<<C->red_blocks, 256, 0, st>>>(g, m, C->ts, C->d_red);
+    // The metrics against their products. On planes this is a guard: a size by a sum of
+    // eight nodes is off by up to 3.5 units of rounding over the spacing, by 8 more
+    // if the nodes are off their planes by four on either side, and a product has the
+    // directions' sum.
+    k_tensor_check<<<C->red_blocks, 256, 0, st>>>(g, C->fm64, C->ts, C->d_red);
     std::vector<double> part(C->red_blocks);
     TG_CUDA(cudaMemcpyAsync(part.data(), C->d_red, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
+    const double tol = planes ? std::max(1e-12, 12 * round) : 1e-12;
     bool ok = true;
-    for (double v : part) ok = ok && v <= 1e-13;
+    for (double v : part) ok = ok && v <= tol;
     if (ok) {
         set_fp_attrs<0>(); set_fp_attrs<1>(); set_fp_attrs<2>();
         TG_CUDA(cudaFuncSetAttribute((const void *)k_stage_fp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGE_SMEM));
