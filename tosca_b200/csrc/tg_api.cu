@@ -1,6 +1,7 @@
 // C-ABI of include/tosca_gpu.h: context lifetime, host<->device transfers in
 // TOSCA's AoS DMDA layout, and the stage entry points. Every entry point
 // returns a tg_status and never exits or traps.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -23,6 +24,15 @@ void *dalloc(tg_ctx *C, size_t bytes)
     e = cudaMemsetAsync(p, 0, bytes, C->stream);
     if (e != cudaSuccess) throw CudaError{e, "cudaMemsetAsync"};
     return p;
+}
+
+void dfree(tg_ctx *C, void *p)
+{
+    auto q = std::find(C->allocs.rbegin(), C->allocs.rend(), p);
+    if (!p || q == C->allocs.rend()) return;
+    C->allocs.erase(std::next(q).base());
+    TG_CUDA(cudaStreamSynchronize(C->stream));
+    TG_CUDA(cudaFree(p));
 }
 
 V3f<double> dalloc3(tg_ctx *C, size_t n)
@@ -364,6 +374,7 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
         if (!nodes) return fail(C, TG_ERR_BAD_ARG, "null nodes");
         const Grid g = C->g;
         const size_t G = (size_t)g.size();
+        C->has_mesh = false;       // until the new one is complete
         double *dn = (double *)dalloc(C, 3 * G * sizeof(double));
         TG_CUDA(cudaMemcpyAsync(dn, nodes, 3 * G * sizeof(double), cudaMemcpyHostToDevice, C->stream));
         k_zero_last_nodes<<<grid3(g.mx, g.my, g.mz), block3(), 0, C->stream>>>(g, dn);
@@ -414,6 +425,7 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
         graph_destroy(C);          // the captured step refers to the old solver buffers
         C->graph_failed = false;
         farm_destroy(C);           // turbine stencils refer to the old cell centres
+        dfree(C, dn);
         poisson_setup(C);
         C->has_mesh = true;
         return TG_OK;

@@ -629,7 +629,7 @@ Fdm *fdm_create(tg_ctx *C, const double *aE, const double *aN, const double *aT,
 
 bool fdm_factors(const Fdm *F, FdmOp *op) { *op = F->op; return F->dev <= 1e-13; }
 
-void fdm_destroy(Fdm *F) { delete F; }   // device buffers are owned by the context allocation list
+void fdm_destroy(Fdm *F) { delete F; }   // the device buffers go with the solver's
 
 void fdm_apply(tg_ctx *C, Fdm *F, const double *r, const double *d_sum, double *z)
 {

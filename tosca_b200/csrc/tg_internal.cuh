@@ -178,7 +178,8 @@ struct tg_ctx {
     tg::State s{};
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    std::vector<void *> allocs;          // every device allocation of this context
+    std::vector<void *> allocs;          // the device allocations of this context, but for
+    std::vector<void *> pois_allocs;     // those of its pressure solver, which go with it
     double *d_red = nullptr;             // reduction scratch (partials)
     double *d_scal = nullptr;            // device scalars
     unsigned *d_count = nullptr;         // arrival counters of last_block: 0 wall model, 1 thermal wall model
@@ -267,6 +268,7 @@ struct CudaError {
     } while (0)
 
 void *dalloc(tg_ctx *C, size_t bytes);        // zeroed device allocation owned by C
+void dfree(tg_ctx *C, void *p);               // gives one back
 inline double *dallocd(tg_ctx *C, size_t n) { return (double *)dalloc(C, n * sizeof(double)); }
 V3f<double> dalloc3(tg_ctx *C, size_t n);
 

@@ -227,7 +227,7 @@ void metrics_from_nodes(tg_ctx *C, const double *d_nodes)
     k_face_metrics<<<grid3(g.mx, g.my, g.mz), block3(), 0, st>>>(X, C->m);
     k_gtensor<<<grid3(g.mx, g.my, g.mz), block3(), 0, st>>>(g, C->m);
     TG_CUDA(cudaGetLastError());
-    TG_CUDA(cudaStreamSynchronize(st));
+    for (const V3f<double> &v : {csit, etat, zett}) dfree(C, v.x);
 }
 
 }  // namespace tg

@@ -673,6 +673,7 @@ __global__ void k_phi_to_dmda(Grid g, State s, PoissonCtx P)
 void poisson_setup(tg_ctx *C)
 {
     if (C->pois) poisson_destroy(C);
+    const size_t mark = C->allocs.size();
     PoissonCtx *P = new PoissonCtx();
     C->pois = P;
     const Grid g = C->g;
@@ -696,14 +697,20 @@ void poisson_setup(tg_ctx *C)
     P->mg = P->fdm ? nullptr : mg_create(C, C->cfg.precision == TG_PREC_MIXED, P->gE1, P->gN2, P->gT3,
                                          P->nx, P->ny, P->nz, P->pi, P->pj, P->pk);
     TG_CUDA(cudaGetLastError());
+    C->pois_allocs.assign(C->allocs.begin() + mark, C->allocs.end());
+    C->allocs.resize(mark);
 }
 
 void poisson_destroy(tg_ctx *C)
 {
     if (C->pois && C->pois->mg) mg_destroy(C->pois->mg);
     if (C->pois && C->pois->fdm) fdm_destroy(C->pois->fdm);
-    delete C->pois;   // device buffers are owned by the context allocation list
+    delete C->pois;
     C->pois = nullptr;
+    if (C->pois_allocs.empty()) return;
+    cudaStreamSynchronize(C->stream);
+    for (void *p : C->pois_allocs) cudaFree(p);
+    C->pois_allocs.clear();
 }
 
 // host read of device scalars [off, off+cnt)
