@@ -263,7 +263,10 @@ tg_status tg_set_mesh_nodes(tg_ctx *ctx, const double *nodes);
 
 /* Generic field transfer (global extent if halo = 0, local ghosted if halo > 0).
  * Vectors are AoS triples. Used to hand over TOSCA's own metrics and state
- * (DMDAVecGetArray pointers) and to read results back. */
+ * (DMDAVecGetArray pointers) and to read results back. What is derived from the
+ * metrics follows a write of them: filter widths and metric products at once, the
+ * pressure operator and its solver once before the next step, pressure solve,
+ * adjoint call or tg_mesh_info, whatever the number of writes. */
 tg_status tg_set_field(tg_ctx *ctx, int32_t which, const double *host, int32_t halo);
 tg_status tg_get_field(tg_ctx *ctx, int32_t which, double *host, int32_t halo);
 /* A field in TOSCA's field-file format (readFields / writeFields, io.c:247-420,

@@ -1677,6 +1677,7 @@ tg_status adj_guard(tg_ctx *C, F &&f)
 tg_status check_adjoint(tg_ctx *C)
 {
     if (!C->has_mesh) { C->err = "mesh not set"; return TG_ERR_STATE; }
+    refresh_solver(C);
     std::string why;
     if (!adjoint_supported(C, why)) { C->err = why; return TG_ERR_BAD_ARG; }
     return TG_OK;

@@ -35,6 +35,31 @@ void dfree(tg_ctx *C, void *p)
     TG_CUDA(cudaFree(p));
 }
 
+// every cross term of the face metric tensor vanishes
+static bool metrics_orthogonal(tg_ctx *C)
+{
+    std::vector<double> h((size_t)C->g.size());
+    double mx = 0.0;
+    TG_CUDA(cudaStreamSynchronize(C->stream));
+    for (double *a : {C->m.g12, C->m.g13, C->m.g21, C->m.g23, C->m.g31, C->m.g32}) {
+        TG_CUDA(cudaMemcpy(h.data(), a, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
+        for (double v : h) mx = std::max(mx, std::fabs(v));
+    }
+    return mx == 0.0;
+}
+
+// the pressure operator and its solver from the metrics as they are, once after
+// any number of metric writes
+void refresh_solver(tg_ctx *C)
+{
+    if (!C->solver_stale) return;
+    C->orthogonal = metrics_orthogonal(C);
+    graph_destroy(C);              // the captured steps refer to the old solver buffers
+    C->graph_failed = false;
+    poisson_setup(C);
+    C->solver_stale = false;
+}
+
 V3f<double> dalloc3(tg_ctx *C, size_t n)
 {
     double *b = (double *)dalloc(C, 3 * n * sizeof(double));
@@ -393,18 +418,12 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
                                       cudaMemcpyDeviceToDevice, C->stream));
         }
         C->met32_stale = true;
-        // orthogonality: every cross term of the face metric tensor vanishes
-        std::vector<double> h(G);
-        double mx = 0.0;
-        for (double *a : {C->m.g12, C->m.g13, C->m.g21, C->m.g23, C->m.g31, C->m.g32}) {
-            TG_CUDA(cudaMemcpy(h.data(), a, G * sizeof(double), cudaMemcpyDeviceToHost));
-            for (double v : h) mx = std::max(mx, std::fabs(v));
-        }
-        C->orthogonal = (mx == 0.0);
+        C->orthogonal = metrics_orthogonal(C);
         // axis alignment: a mesh of planes by its nodes (tensor_setup), or one whose
         // cell-face (csi, eta, zet) and face (icsi .. kzet) metrics have only csi.y,
         // eta.z, zet.x above 1e-12 of the array's largest component
         const Metrics &M = C->m;
+        std::vector<double> h(G);
         auto amax = [&](const double *a) {
             TG_CUDA(cudaMemcpy(h.data(), a, G * sizeof(double), cudaMemcpyDeviceToHost));
             double r = 0.0;
@@ -427,6 +446,7 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
         farm_destroy(C);           // turbine stencils refer to the old cell centres
         dfree(C, dn);
         poisson_setup(C);
+        C->solver_stale = false;
         C->has_mesh = true;
         return TG_OK;
     });
@@ -470,11 +490,9 @@ tg_status tg_set_field(tg_ctx *C, int32_t w, const double *host, int32_t halo)
         if ((w >= TG_F_CSI && w <= TG_F_KZET) || (w >= TG_F_AJ && w <= TG_F_KAJ)) {
             C->met32_stale = true;
             refresh_gtensor(C);
-            if (w >= TG_F_AJ) refresh_teqn_mesh(C);
-            if (C->axis_aligned) {         // the caller's metrics need not be those of a mesh of planes
-                C->axis_aligned = false;
-                graph_destroy(C);
-            }
+            if (w >= TG_F_AJ) { refresh_filter(C); refresh_teqn_mesh(C); }
+            C->axis_aligned = false;       // the caller's metrics need not be those of a mesh of planes
+            C->solver_stale = C->has_mesh;
         }
         return TG_OK;
     });
@@ -682,6 +700,7 @@ tg_status tg_solve_p(tg_ctx *C, tg_stats *st)
 {
     return guarded(C, [&]() -> tg_status {
         if (!C->has_mesh) return fail(C, TG_ERR_STATE, "mesh not set");
+        refresh_solver(C);
         tg_stats local{};
         int rc = solve_p(C, st ? st : &local);
         TG_CUDA(cudaStreamSynchronize(C->stream));
@@ -706,6 +725,7 @@ tg_status tg_step(tg_ctx *C, int32_t nsteps, tg_stats *st)
         if (!C->has_mesh) return fail(C, TG_ERR_STATE, "mesh not set");
         if (nsteps < 0) return fail(C, TG_ERR_BAD_ARG, "negative step count");
         if (const char *why = theta_wall_missing(C)) return fail(C, TG_ERR_STATE, why);
+        refresh_solver(C);
         tg_stats local{};
         tg_stats *s = st ? st : &local;
         *s = tg_stats{};
@@ -759,6 +779,7 @@ tg_status tg_mesh_info(tg_ctx *C, int32_t *orthogonal, int32_t *axis_aligned)
     return guarded(C, [&]() -> tg_status {
         if (!orthogonal || !axis_aligned) return fail(C, TG_ERR_BAD_ARG, "null output");
         if (!C->has_mesh) return fail(C, TG_ERR_STATE, "mesh not set");
+        refresh_solver(C);
         *orthogonal = C->orthogonal ? 1 : 0;
         *axis_aligned = C->axis_aligned ? 1 : 0;
         return TG_OK;
@@ -782,6 +803,7 @@ tg_status tg_step_host(tg_ctx *C, double *ucont, double *ucat, double *p, double
         if (!ucont || !ucat || !p || halo < 0) return fail(C, TG_ERR_BAD_ARG, "null state");
         if (!C->has_mesh) return fail(C, TG_ERR_STATE, "mesh not set");
         if (const char *why = theta_wall_missing(C)) return fail(C, TG_ERR_STATE, why);
+        refresh_solver(C);
         upload(C, ucont, halo, C->s.ucont.x, C->s.ucont.y, C->s.ucont.z);
         upload(C, ucat, halo, C->s.ucat.x, C->s.ucat.y, C->s.ucat.z);
         upload(C, p, halo, C->s.p, nullptr, nullptr);

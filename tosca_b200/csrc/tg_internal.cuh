@@ -194,6 +194,7 @@ struct tg_ctx {
     size_t stage_nut_bytes = 0;
     int red_blocks = 0;
     bool has_mesh = false;
+    bool solver_stale = false;           // metrics written since the pressure solver was set up
     bool orthogonal = true;              // all cross metric-tensor terms vanish
     // a mesh of planes along the reference's axes (i -> y, j -> z, k -> x), up to
     // the rounding of its coordinates: the stage kernels of tg_tensor.cu run, on
@@ -403,6 +404,7 @@ void contra_div_tensor(tg_ctx *C);             // final Ucat and the partial div
 
 // stage entry points (tg_step.cu)
 void metrics_from_nodes(tg_ctx *C, const double *d_nodes);
+void refresh_solver(tg_ctx *C);               // before a pressure solve: the solver of the metrics as they are
 void refresh_gtensor(tg_ctx *C);              // g11 .. g33 from the face metrics
 void alloc_precision_work(tg_ctx *C);         // FP64 views, FP32 copies (mixed mode)
 void refresh_met32(tg_ctx *C);
