@@ -57,6 +57,15 @@ def test_periodic_channel_sizes(nx, ny, nz):
     compare(cfg, nodes, u, p)
 
 
+@pytest.mark.parametrize("nz", [32, 33, 61, 64, 65, 113, 255, 256, 257, 300])
+def test_line_lengths(nz):
+    """The solver of the j lines has four forms: chunks of 4, 8 and 16 cells per
+    warp (up to 32, 64 and 256 cells) and one thread per line, each with its
+    remainders. A line solve that is off shows in the bound on the iterations."""
+    cfg, nodes, u, p = cases.abl_case(nx=5, ny=5, nz=nz, Lx=50.0, Ly=50.0, H=8.0 * nz, ddt=api.DDT_RK4, dt=0.1)
+    compare(cfg, nodes, u, p)
+
+
 @pytest.mark.parametrize("nx,ny,nz,axis", [(12, 6, 5, None), (13, 8, 5, None), (9, 6, 5, 0), (16, 8, 6, 0), (42, 5, 4, 0)])
 def test_open_channel_sizes(nx, ny, nz, axis):
     cfg, nodes, u, p = cases.channel_case(nx=nx, ny=ny, nz=nz, Lx=10.0 * nx, Ly=10.0 * ny, H=8.0 * nz, ddt=api.DDT_RK4, dt=0.1)

@@ -116,6 +116,27 @@ def test_against_oracle(kind, nx, ny, nz, over):
     g.close(); o.close()
 
 
+# 79 x 65 x 64 cells away from the boundary give 480 tiles of 32 x 8 x 4 cells,
+# above the three per SM from which the tile kernel takes four cells along k; 79
+# and 65 leave remainders
+@pytest.mark.parametrize("over", [{}, dict(les=0, nu=0.5), dict(ddt=api.DDT_ABCN, snes_atol=1e-12)])
+def test_deep_tiles(over):
+    case = make("abl", 80, 66, 66, **over)
+    a, b = pair(*case)
+    o = oracle.solver(case[0])
+    cases.setup(o, *case[1:])
+    for s in (a, b, o):
+        s.FormU(1.0, True)
+    assert rel_l2(a.get("RHS"), o.get("RHS")) <= 1e-12
+    assert rel_l2(a.get("RHS"), b.get("RHS")) <= 1e-12
+    if case[0].ddt_scheme == api.DDT_ABCN:                 # the convective and the viscous part by themselves
+        for s in (a, b):
+            s.step(1)
+        assert rel_l2(a.get("UCAT"), b.get("UCAT")) <= 1e-9
+    for s in (a, b, o):
+        s.close()
+
+
 def test_metric_write_rebuilds_the_step():
     """A metric written between replayed steps takes effect on the next one."""
     a, b = pair(*make("abl", 12, 16, 9))
