@@ -419,11 +419,12 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
         }
         C->met32_stale = true;
         C->orthogonal = metrics_orthogonal(C);
-        // axis alignment: a mesh of planes by its nodes (tensor_setup), or one whose
-        // cell-face (csi, eta, zet) and face (icsi .. kzet) metrics have only csi.y,
-        // eta.z, zet.x above 1e-12 of the array's largest component
+        // axis alignment: a mesh of planes by its nodes, or one whose cell-face (csi,
+        // eta, zet) and face (icsi .. kzet) metrics have only csi.y, eta.z, zet.x above
+        // 1e-12 of the array's largest component
+        const bool planes = planes_of_nodes(g, nodes);
         const Metrics &M = C->m;
-        std::vector<double> h(G);
+        std::vector<double> h(planes ? 0 : G);
         auto amax = [&](const double *a) {
             TG_CUDA(cudaMemcpy(h.data(), a, G * sizeof(double), cudaMemcpyDeviceToHost));
             double r = 0.0;
@@ -437,10 +438,12 @@ tg_status tg_set_mesh_nodes(tg_ctx *C, const double *nodes)
             for (int q = 0; q < 3 && ax; q++)
                 if (q != keep && !(amax(c[q]) <= 1e-12 * d)) ax = false;
         };
-        for (const V3f<double> &v : {M.csi, M.icsi, M.jcsi, M.kcsi}) along(v, 1);
-        for (const V3f<double> &v : {M.eta, M.ieta, M.jeta, M.keta}) along(v, 2);
-        for (const V3f<double> &v : {M.zet, M.izet, M.jzet, M.kzet}) along(v, 0);
-        C->axis_aligned = tensor_setup(C, nodes, ax);
+        if (!planes) {
+            for (const V3f<double> &v : {M.csi, M.icsi, M.jcsi, M.kcsi}) along(v, 1);
+            for (const V3f<double> &v : {M.eta, M.ieta, M.jeta, M.keta}) along(v, 2);
+            for (const V3f<double> &v : {M.zet, M.izet, M.jzet, M.kzet}) along(v, 0);
+        }
+        C->axis_aligned = ax && tensor_setup(C, nodes, planes);
         graph_destroy(C);          // the captured step refers to the old solver buffers
         C->graph_failed = false;
         farm_destroy(C);           // turbine stencils refer to the old cell centres

@@ -585,31 +585,41 @@ void set_attrs()
 
 }  // namespace
 
-Fdm *fdm_create(tg_ctx *C, const double *aE, const double *aN, const double *aT,
+Fdm *fdm_create(tg_ctx *C, const Tensor *t, const double *aE, const double *aN, const double *aT,
                 int nx, int ny, int nz, int pi, int pj, int pk)
 {
     cudaStream_t st = C->stream;
     const size_t pl = (size_t)nx * ny;
-    // a line of coefficients through cell (0, 0, 0)
     auto line = [&](const double *a, size_t stride, int n) {
         std::vector<double> h(n);
         TG_CUDA(cudaMemcpy2DAsync(h.data(), sizeof(double), a, stride * sizeof(double), sizeof(double), n, cudaMemcpyDeviceToHost, st));
         TG_CUDA(cudaStreamSynchronize(st));
         return h;
     };
-    // normalised to mx_0 = my_0 = mz_0 = 1
-    std::vector<double> kx = line(aE, 1, nx), mx = line(aN, 1, nx), ky = line(aN, nx, ny), mz = line(aN, pl, nz),
-                        my = line(aT, nx, ny), kz = line(aT, pl, nz);
-    const double n0 = ky[0], t0 = kz[0];
+    std::vector<double> kx, mx, ky, my, kz, mz;
+    if (t) {
+        // cells 1 .. of the DMDA; the masses are the sizes, and a factor has one
+        // rounding where one read off the coefficients has three
+        kx = line(t->rdyf + 1, 1, nx); mx = line(t->dy + 1, 1, nx);
+        ky = line(t->rdzf + 1, 1, ny); my = line(t->dz + 1, 1, ny);
+        kz = line(t->rdxf + 1, 1, nz); mz = line(t->dx + 1, 1, nz);
+        // two axes may run downwards; the coefficients' sign is checked below
+        for (auto *v : {&kx, &mx, &ky, &my, &kz, &mz})
+            for (double &q : *v) q = std::fabs(q);
+    } else {
+        // lines of coefficients through cell (0, 0, 0), normalised to mx_0 = my_0 = mz_0 = 1
+        kx = line(aE, 1, nx); mx = line(aN, 1, nx); ky = line(aN, nx, ny); mz = line(aN, pl, nz); my = line(aT, nx, ny); kz = line(aT, pl, nz);
+        const double n0 = ky[0], t0 = kz[0];
+        for (double &v : mx) v /= n0;
+        for (double &v : mz) v /= n0;
+        for (double &v : my) v /= t0;
+    }
     auto positive = [](const std::vector<double> &v, int cnt) {
         for (int q = 0; q < cnt; q++) if (!(v[q] > 0.0) || !std::isfinite(v[q])) return false;
         return true;
     };
     if (!positive(kx, pi ? nx : nx - 1) || !positive(mx, nx) || !positive(ky, pj ? ny : ny - 1) || !positive(mz, nz) ||
         !positive(my, ny) || !positive(kz, pk ? nz : nz - 1)) return nullptr;
-    for (double &v : mx) v /= n0;
-    for (double &v : mz) v /= n0;
-    for (double &v : my) v /= t0;
     FdmDir dx, dy, dz;
     if (!plan_dir(dx, nx, pi, kx, mx) || !plan_dir(dz, nz, pk, kz, mz) || (pj && !plan_dir(dy, ny, true, ky, my)) ||
         dx.gs + dz.gs > FDM_MAX_ROWS) return nullptr;

@@ -15,10 +15,11 @@ struct FdmOp { const double *kx, *mx, *ky, *my, *kz, *mz; };
 // the operator may be evaluated from them
 bool fdm_factors(const Fdm *F, FdmOp *op);
 
-// face coefficients as for mg_create (tg_mg.cuh). nullptr when the operator
-// does not separate or a direction is outside the solver's range; the caller
-// then uses the multigrid.
-Fdm *fdm_create(tg_ctx *C, const double *aE, const double *aN, const double *aT,
+// face coefficients as for mg_create (tg_mg.cuh); on a mesh of planes t, whose
+// spacings are the factors, else null. nullptr when the operator does not separate
+// or a direction is outside the solver's range; the caller then uses the
+// multigrid.
+Fdm *fdm_create(tg_ctx *C, const Tensor *t, const double *aE, const double *aN, const double *aT,
                 int nx, int ny, int nz, int pi, int pj, int pk);
 void fdm_destroy(Fdm *F);
 

@@ -390,7 +390,8 @@ inline dim3 block3() { return dim3(BX, BY, BZ); }
 
 // stage kernels on a mesh of planes (tg_tensor.cu)
 struct RkArgs;
-bool tensor_setup(tg_ctx *C, const double *nodes, bool cross);   // nodes: the host array
+bool planes_of_nodes(const Grid &g, const double *nodes);        // nodes: the host array
+bool tensor_setup(tg_ctx *C, const double *nodes, bool planes);
 void contra_to_cart_tensor(tg_ctx *C, const char *name);
 void smagorinsky_tensor(tg_ctx *C);
 void grad_p_tensor(tg_ctx *C);

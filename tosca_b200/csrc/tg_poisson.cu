@@ -484,15 +484,12 @@ __global__ void __launch_bounds__(RB) k_direct_begin(Grid g, State s, PoissonCtx
 }
 
 // f(c, x_c, (L x)_c) of k_apply7 for every cell; FAC: coefficients from their
-// factors. A block takes 32 x 8 columns (a warp per j) of kc cells along k and
+// factors, associated as the projection's (k_pressure_project): (area) / distance,
+// so that the two are the same numbers. A block takes 32 x 8 columns (a warp per j) of kc cells along k and
 // holds the column's cell, the one below and the one above in registers.
-// Latency-bound: with rows of i per warp, whose loads waited for the stores of the
-// cells before them (no read-only loads) and which fetched each x three times
-// from L2, r = b - L x took 137 us at 256 x 256 x 128 and the dot products 89 us; now
-// 77 and 69, of 41 and 31 us for their bytes. A step of 256 x 256 x 128 went 3.07 -> 3.00 ms, of
-// 192 x 192 x 96 1.461 -> 1.430 ms, and those of 75 x 75 x 25 and 32^3 stayed. Read-only
-// loads in the rows alone gave nothing; three blocks per SM (80 registers, unrolled
-// by four) 3.09 ms, five 3.015 ms.
+// Latency-bound: r = b - L x takes 77 us at 256 x 256 x 128 and the dot products 69, of
+// 41 and 31 us for their bytes; rows of i per warp, whose loads wait for the stores
+// of the cells before them and which fetch each x three times from L2, 137 and 89.
 template <bool FAC, class F>
 __device__ __forceinline__ void op7_march(const PoissonCtx &P, const double *x, int kc, F f)
 {
@@ -509,9 +506,10 @@ __device__ __forceinline__ void op7_march(const PoissonCtx &P, const double *x, 
             kE = hE ? P.op.kx[i] : 0.0; kW = hW ? P.op.kx[i > 0 ? i - 1 : nx - 1] : 0.0;
             kN = hN ? P.op.ky[j] : 0.0; kS = hS ? P.op.ky[j > 0 ? j - 1 : ny - 1] : 0.0;
         }
+        const double mmy = m * my;
         int c = (k0 * ny + j) * nx + i;
         double xb = __ldg(x + c + (k0 > 0 ? -pl : pl * nz - pl)), xc = __ldg(x + c);
-        double gb = k0 > 0 || P.pk ? (FAC ? P.op.kz[k0 > 0 ? k0 - 1 : nz - 1] * my : __ldg(P.gT3 + c + (k0 > 0 ? -pl : pl * nz - pl))) : 0.0;
+        double gb = k0 > 0 || P.pk ? (FAC ? P.op.kz[k0 > 0 ? k0 - 1 : nz - 1] * mmy : __ldg(P.gT3 + c + (k0 > 0 ? -pl : pl * nz - pl))) : 0.0;
         #pragma unroll 2
         for (int k = k0; k < k1; k++, c += pl) {
             const bool top = k < nz - 1;
@@ -519,13 +517,14 @@ __device__ __forceinline__ void op7_march(const PoissonCtx &P, const double *x, 
             double acc = 0.0, gt = 0.0;
             if (FAC) {
                 const double mz = __ldg(P.op.mz + k), e = my * mz;
-                if (top || P.pk) gt = __ldg(P.op.kz + k) * my;
+                const double mmz = m * mz;
+                if (top || P.pk) gt = __ldg(P.op.kz + k) * mmy;
                 acc += (kE * e) * (xc - xe);
                 acc += (kW * e) * (xc - xw);
-                acc += (m * (kN * mz)) * (xc - xn);
-                acc += (m * (kS * mz)) * (xc - xs);
-                acc += (m * gt) * (xc - xt);
-                acc += (m * gb) * (xc - xb);
+                acc += (kN * mmz) * (xc - xn);
+                acc += (kS * mmz) * (xc - xs);
+                acc += gt * (xc - xt);
+                acc += gb * (xc - xb);
             } else {
                 if (top || P.pk) gt = __ldg(P.gT3 + c);
                 acc += (hE ? __ldg(P.gE1 + c) : 0.0) * (xc - xe);
@@ -692,7 +691,7 @@ void poisson_setup(tg_ctx *C)
     P->count = (unsigned *)dalloc(C, sizeof(unsigned));
     k_gather_g<<<cgrid(P->nx, P->ny, P->nz), block3(), 0, C->stream>>>(g, C->m, C->ts, C->axis_aligned, *P);
 
-    P->fdm = P->ortho ? fdm_create(C, P->gE1, P->gN2, P->gT3, P->nx, P->ny, P->nz, P->pi, P->pj, P->pk) : nullptr;
+    P->fdm = P->ortho ? fdm_create(C, C->axis_aligned ? &C->ts : nullptr, P->gE1, P->gN2, P->gT3, P->nx, P->ny, P->nz, P->pi, P->pj, P->pk) : nullptr;
     P->op_exact = P->fdm && fdm_factors(P->fdm, &P->op);
     P->mg = P->fdm ? nullptr : mg_create(C, C->cfg.precision == TG_PREC_MIXED, P->gE1, P->gN2, P->gT3,
                                          P->nx, P->ny, P->nz, P->pi, P->pj, P->pk);

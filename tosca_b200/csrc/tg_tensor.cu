@@ -917,44 +917,65 @@ void set_fp_attrs()
 
 }  // namespace
 
-// Is the mesh one of planes (x depends on k alone, y on i, z on j), and if so its
-// spacings into C->ts. The question is put to the nodes and not to the metrics:
-// those form the same size by sums of different nodes and differ from each other by
-// some units of rounding of the coordinates over the spacing (2e-13 at 1300 cells
-// of 7.3 m, 1.4e-11 at map coordinates of 500 km), which says nothing about the
-// planes. A node may be off its plane by four units of rounding of the largest
-// coordinate. cross: the cross components of the metrics vanish to 1e-12; then nodes
-// further off count as well, as long as every metric is its product to 1e-12.
-bool tensor_setup(tg_ctx *C, const double *nodes, bool cross)
+namespace {
+constexpr double EPS = 2.220446049250313e-16;
+// coordinates of the planes 0 .. m-2 of direction q (x, y, z) through the first node
+std::vector<double> plane_line(const Grid &g, const double *nodes, int q)
+{
+    const int n = (q == 0 ? g.mz : q == 1 ? g.mx : g.my) - 1;
+    const int64_t st = q == 0 ? (int64_t)g.mx * g.my : q == 1 ? 1 : g.mx;
+    std::vector<double> X(n);
+    for (int l = 0; l < n; l++) X[l] = nodes[3 * st * l + q];
+    return X;
+}
+double largest(const std::vector<double> &X)
+{
+    double r = 0.0;
+    for (double x : X) r = std::max(r, std::fabs(x));
+    return r;
+}
+}  // namespace
+
+// Is the mesh one of planes (x depends on k alone, y on i, z on j)? The question is
+// put to the nodes and not to the metrics: those form the same size by sums of
+// different nodes and differ from each other by some units of rounding of the
+// coordinates over the spacing (2e-13 at 1300 cells of 7.3 m, 1.4e-11 at map
+// coordinates of 500 km), which says nothing about the planes. A node may be off
+// its plane by four units of rounding of the largest coordinate.
+bool planes_of_nodes(const Grid &g, const double *nodes)
+{
+    const std::vector<double> X = plane_line(g, nodes, 0), Y = plane_line(g, nodes, 1), Z = plane_line(g, nodes, 2);
+    const double ox = 4 * EPS * largest(X), oy = 4 * EPS * largest(Y), oz = 4 * EPS * largest(Z);
+    for (int k = 0; k < g.mz - 1; k++)
+        for (int j = 0; j < g.my - 1; j++) {
+            const double *x = nodes + 3 * (int64_t)g.lin(k, j, 0);
+            bool on = true;
+            for (int i = 0; i < g.mx - 1; i++, x += 3)
+                on = on && std::fabs(x[0] - X[k]) <= ox && std::fabs(x[1] - Y[i]) <= oy && std::fabs(x[2] - Z[j]) <= oz;
+            if (!on) return false;
+        }
+    return true;
+}
+
+// The spacings of a mesh of planes from its nodes, into C->ts. planes: as
+// planes_of_nodes; without it the caller found the cross components of the metrics
+// to vanish to 1e-12, and every metric has to be its product to 1e-12. false if
+// the metrics are not these products.
+bool tensor_setup(tg_ctx *C, const double *nodes, bool planes)
 {
     const Grid g = C->g;
     cudaStream_t st = C->stream;
-    constexpr double EPS = 2.220446049250313e-16;
     const int n[3] = {g.mz, g.mx, g.my};                       // x, y, z
-    const int64_t stride[3] = {(int64_t)g.mx * g.my, 1, g.mx};
     const int per[3] = {g.pk, g.pi, g.pj};
     std::vector<double> X[3];                                  // planes 0 .. n-2
-    double big[3], hmin[3], round = 0.0;
+    double round = 0.0;
     for (int q = 0; q < 3; q++) {
-        X[q].resize(n[q] - 1);
-        big[q] = 0.0; hmin[q] = HUGE_VAL;
-        for (int l = 0; l < n[q] - 1; l++) {
-            X[q][l] = nodes[3 * stride[q] * l + q];
-            big[q] = std::max(big[q], std::fabs(X[q][l]));
-            if (l > 0) hmin[q] = std::min(hmin[q], std::fabs(X[q][l] - X[q][l - 1]));
-        }
-        round += EPS * big[q] / hmin[q];
+        X[q] = plane_line(g, nodes, q);
+        double h = HUGE_VAL;
+        for (int l = 1; l < n[q] - 1; l++) h = std::min(h, std::fabs(X[q][l] - X[q][l - 1]));
+        round += EPS * largest(X[q]) / h;
     }
-    if (!std::isfinite(round)) return false;                   // coinciding planes, or no numbers
-    const double off[3] = {4 * EPS * big[0], 4 * EPS * big[1], 4 * EPS * big[2]};
-    bool planes = true;
-    for (int k = 0; k < g.mz - 1 && planes; k++)
-        for (int j = 0; j < g.my - 1 && planes; j++) {
-            const double *x = nodes + 3 * (int64_t)g.lin(k, j, 0);
-            for (int i = 0; i < g.mx - 1; i++, x += 3)
-                planes &= std::fabs(x[0] - X[0][k]) <= off[0] && std::fabs(x[1] - X[1][i]) <= off[1] && std::fabs(x[2] - X[2][j]) <= off[2];
-        }
-    if (!planes && !cross) return false;
+    if (!std::isfinite(round)) return false;                   // coinciding planes
     constexpr int NA = 7;        // arrays per direction
     if (!C->ts_mem) C->ts_mem = dallocd(C, NA * ((size_t)g.mx + g.my + g.mz));
     double *mem = C->ts_mem;
