@@ -277,11 +277,11 @@ int solve_u_cn(tg_ctx *C, tg_stats *st)
     // F is evaluated in FP64 in every precision mode: the differenced
     // Jacobian-vector products divide F's change over h ~ 1e-8 |U|, below
     // the rounding of an FP32 residual
-    const auto pol = C->pol;
-    C->pol = decltype(C->pol){};
+    const bool met32 = C->met32;
+    C->met32 = false;
     const int rc = jfnk_solve(C, W.j, [&](const double *U, double *F) { cn_eval(C, W, U, F, scale); }, C->cfg.snes_atol,
                               C->cfg.snes_rtol, maxit, newton, linear, fn);
-    C->pol = pol;
+    C->met32 = met32;
     // Ucont <- U (SNESFuncEval left the last evaluated point in the state)
     TG_CUDA(cudaMemcpyAsync(C->s.ucont.x, W.j.U, sizeof(double) * n, cudaMemcpyDeviceToDevice, C->stream));
     C->mom_outer = newton;

@@ -84,11 +84,9 @@ struct Tensor {
     const double *rqx, *rqy, *rqz, *rqxf, *rqyf, *rqzf;
 };
 
-// FormU work planes at storage precision T: face fluxes per direction and
-// their cell divergence
-template <class T>
+// FormU work planes: face fluxes per direction and their cell divergence
 struct FluxWork {
-    V3f<T> f1, f2, f3, fp;
+    V3f<double> f1, f2, f3, fp;
 };
 
 // physical state and work arrays
@@ -207,23 +205,14 @@ struct tg_ctx {
     double *series_t = nullptr, *series_v = nullptr;   // thetaWallFunction -4 surface temperature series
     int series_n = 0;
     int it = 0;
-    // mixed precision: FP32 copies of the stencil metrics (and FP32 FormU
-    // planes when the policy stores the face fluxes in FP32)
+    // mixed precision: FP32 copies of the stencil metrics, read by the kernels of
+    // curvilinear meshes and by QUICK's face fluxes (alloc_precision_work)
     bool mixed = false;
-    // which momentum stages read the FP32 metric copies (and compute in FP32)
-    struct {
-        bool contra_m32 = false;     // contravariantToCartesian: FP32 metrics
-        bool contra_a32 = false;     //   ... and FP32 arithmetic
-        bool visc32 = false;         // FormU viscous fluxes
-        bool flux32 = false;         // FormU face-flux planes stored in FP32
-        bool rhs32 = false;          // FormU face assembly metrics
-        bool smag32 = false;         // Smagorinsky eddy viscosity
-    } pol;
+    bool met32 = false;                  // they read them (not inside the Crank-Nicolson residual)
     bool met32_stale = true;             // metrics changed since the FP32 copies were made
     tg::FaceMet<double> fm64{};
     tg::FaceMet<float> fm32{};
-    tg::FluxWork<double> fw64{};
-    tg::FluxWork<float> fw32{};
+    tg::FluxWork fw{};
     // a caller wrote Rhs / dP through tg_set_field: the next evaluation clears
     // the points outside the ones it writes
     bool clear_rhs = false, clear_dp = false;
@@ -408,8 +397,8 @@ void metrics_from_nodes(tg_ctx *C, const double *d_nodes);
 void refresh_solver(tg_ctx *C);               // before a pressure solve: the solver of the metrics as they are
 void refresh_gtensor(tg_ctx *C);              // g11 .. g33 from the face metrics
 void alloc_precision_work(tg_ctx *C);         // FP64 views, FP32 copies (mixed mode)
-void refresh_met32(tg_ctx *C);
-void refresh_filter(tg_ctx *C);          // FP64 Smagorinsky filter widths after a mesh change                // FP32 metric copies from the FP64 fields
+void refresh_met32(tg_ctx *C);                // FP32 metric copies from the FP64 fields
+void refresh_filter(tg_ctx *C);               // FP64 Smagorinsky filter widths after a change of aj
 void contra_to_cart(tg_ctx *C);
 void reset_cell_periodic(tg_ctx *C, V3f<double> v);
 void reset_cell_periodic_s(tg_ctx *C, double *v);

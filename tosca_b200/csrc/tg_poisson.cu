@@ -59,9 +59,6 @@ struct Cg {   // compact grid indexing with periodic wrap
     __device__ __forceinline__ int wj(int j) const { if (j < 0) j += ny; else if (j >= ny) j -= ny; return j; }
     __device__ __forceinline__ int wk(int k) const { if (k < 0) k += nz; else if (k >= nz) k -= nz; return k; }
     __device__ __forceinline__ int id(int k, int j, int i) const { return (wk(k) * ny + wj(j)) * nx + wi(i); }
-    __device__ __forceinline__ bool in(int k, int j, int i) const {
-        return (pi || (i >= 0 && i < nx)) && (pj || (j >= 0 && j < ny)) && (pk || (k >= 0 && k < nz));
-    }
 };
 
 // ------------------------------------------------------------ setup kernels

@@ -4,7 +4,6 @@
 // (file:line at the kernel). All fields are SoA FP64 on the global DMDA extent.
 #include <algorithm>
 #include <cmath>
-#include <type_traits>
 
 #include "tg_internal.cuh"
 #include "tg_mo.cuh"
@@ -15,8 +14,7 @@ namespace {
 
 __device__ __forceinline__ bool is_wall(int t) { return t == TG_BC_NOSLIP || t == TG_BC_SLIP || t == TG_BC_WALL_SHUMANN; }
 
-// 2-D plane launch helper
-inline dim3 g2(int na, int nb) { return dim3((na + 31) / 32, (nb + 7) / 8); }
+// block of the 2-D plane launches
 const dim3 b2(32, 8);
 
 // element-type conversion of a vector triple
@@ -27,30 +25,29 @@ __device__ __forceinline__ R3<To> cvta(R3<From> a) { return R3<To>{(To)a.x, (To)
 // contravariantToCartesian (ueqn.c:528-635): average face fluxes to the
 // centre and solve [csi;eta;zet] u = q by Cramer's rule. Interior cells.
 // MS is the storage type of the metrics (FP32 copies in the mixed-precision
-// mode), A the arithmetic type; Ucont and Ucat stay FP64.
+// mode); the arithmetic is FP64.
 // ------------------------------------------------------------------------
-template <class A, class MS>
+template <class MS>
 __device__ __forceinline__ void contra_cell(const Grid &g, const FaceMet<MS> &m, const State &s, int c)
 {
-    using M = A;
-    R3<M> sc = cvta<M>(ld3(m.csi, c)), e = cvta<M>(ld3(m.eta, c)), z = cvta<M>(ld3(m.zet, c));
-    M m00 = sc.x, m01 = sc.y, m02 = sc.z, m10 = e.x, m11 = e.y, m12 = e.z, m20 = z.x, m21 = z.y, m22 = z.z;
-    M q0 = (M)(0.5 * (s.ucont.x[c - 1] + s.ucont.x[c]));
-    M q1 = (M)(0.5 * (s.ucont.y[c - g.mx] + s.ucont.y[c]));
-    M q2 = (M)(0.5 * (s.ucont.z[c - g.mx * g.my] + s.ucont.z[c]));
-    M det  =  m00 * (m11 * m22 - m12 * m21) - m01 * (m10 * m22 - m12 * m20) + m02 * (m10 * m21 - m11 * m20);
-    M det0 =  q0 * (m11 * m22 - m12 * m21) - q1 * (m01 * m22 - m02 * m21) + q2 * (m01 * m12 - m02 * m11);
-    M det1 = -q0 * (m10 * m22 - m12 * m20) + q1 * (m00 * m22 - m02 * m20) - q2 * (m00 * m12 - m02 * m10);
-    M det2 =  q0 * (m10 * m21 - m11 * m20) - q1 * (m00 * m21 - m01 * m20) + q2 * (m00 * m11 - m01 * m10);
-    s.ucat.x[c] = (double)(det0 / det); s.ucat.y[c] = (double)(det1 / det); s.ucat.z[c] = (double)(det2 / det);
+    R3<double> sc = cvta<double>(ld3(m.csi, c)), e = cvta<double>(ld3(m.eta, c)), z = cvta<double>(ld3(m.zet, c));
+    double m00 = sc.x, m01 = sc.y, m02 = sc.z, m10 = e.x, m11 = e.y, m12 = e.z, m20 = z.x, m21 = z.y, m22 = z.z;
+    double q0 = 0.5 * (s.ucont.x[c - 1] + s.ucont.x[c]);
+    double q1 = 0.5 * (s.ucont.y[c - g.mx] + s.ucont.y[c]);
+    double q2 = 0.5 * (s.ucont.z[c - g.mx * g.my] + s.ucont.z[c]);
+    double det  =  m00 * (m11 * m22 - m12 * m21) - m01 * (m10 * m22 - m12 * m20) + m02 * (m10 * m21 - m11 * m20);
+    double det0 =  q0 * (m11 * m22 - m12 * m21) - q1 * (m01 * m22 - m02 * m21) + q2 * (m01 * m12 - m02 * m11);
+    double det1 = -q0 * (m10 * m22 - m12 * m20) + q1 * (m00 * m22 - m02 * m20) - q2 * (m00 * m12 - m02 * m10);
+    double det2 =  q0 * (m10 * m21 - m11 * m20) - q1 * (m00 * m21 - m01 * m20) + q2 * (m00 * m11 - m01 * m10);
+    s.ucat.x[c] = det0 / det; s.ucat.y[c] = det1 / det; s.ucat.z[c] = det2 / det;
 }
 
-template <class A, class MS>
+template <class MS>
 __global__ void k_contra_to_cart(Grid g, FaceMet<MS> m, State s)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
-    contra_cell<A>(g, m, s, g.lin(k, j, i));
+    contra_cell(g, m, s, g.lin(k, j, i));
 }
 
 // the same on the interior cells next to the boundary only: the cells whose
@@ -67,7 +64,7 @@ __global__ void k_contra_to_cart_shell(Grid g, FaceMet<double> m, State s)
     if (dir == 0) { k = b; j = a; i = right ? g.mx - 2 : 1; }
     else if (dir == 1) { k = b; i = a; j = right ? g.my - 2 : 1; }
     else { j = b; i = a; k = right ? g.mz - 2 : 1; }
-    contra_cell<double>(g, m, s, g.lin(k, j, i));
+    contra_cell(g, m, s, g.lin(k, j, i));
 }
 
 // FP32 copies of the stencil metrics
@@ -574,8 +571,8 @@ __device__ __forceinline__ R3<M> visc_flux_ax(M cs, M et, M ze, int dir, R3<M> d
     return v;
 }
 
-// M: storage and arithmetic type of the metrics in the viscous flux; F: storage
-// type of the face fluxes. The convective flux is formed in FP64 from the FP64
+// M: storage and arithmetic type of the metrics in the viscous flux. The
+// convective flux is formed in FP64 from the FP64
 // Ucont and Ucat. mode is FormU's formMode (ueqn_solvers.c:17, 105-106):
 // 0 convection + viscosity, 1 convection only, 2 viscosity (with the wall
 // stress) only; the skipped part of each face flux is zero. AX: the mesh is
@@ -583,8 +580,8 @@ __device__ __forceinline__ R3<M> visc_flux_ax(M cs, M et, M ze, int dir, R3<M> d
 constexpr int FBX = 32, FBY = 4, FBZ = 2, FBN = FBX * FBY * FBZ, FMINB = 4;   // block of k_face_fluxes
 constexpr int FTX = FBX + 3, FTY = FBY + 3, FTZ = FBZ + 3, FTN = FTX * FTY * FTZ;
 
-template <class M, class F, int mode, bool AX>
-__global__ void __launch_bounds__(FBN, FMINB) k_face_fluxes(Grid g, FaceMet<M> m, State s, FluxWork<F> w, Params p)
+template <class M, int mode, bool AX>
+__global__ void __launch_bounds__(FBN, FMINB) k_face_fluxes(Grid g, FaceMet<M> m, State s, FluxWork w, Params p)
 {
     __shared__ double su[3][FTN];
     __shared__ double sn[FTN];
@@ -664,7 +661,7 @@ __global__ void __launch_bounds__(FBN, FMINB) k_face_fluxes(Grid g, FaceMet<M> m
             if (AX) vv = cvta<double>(visc_flux_ax<M>(m.icsi.y[f], m.ieta.z[f], m.izet.x[f], 0, cvta<M>(dc), cvta<M>(de), cvta<M>(dz), m.iaj[f], nuEff));
             else vv = cvta<double>(visc_flux<M>(ld3(m.icsi, f), ld3(m.ieta, f), ld3(m.izet, f), 0, cvta<M>(dc), cvta<M>(de), cvta<M>(dz), m.iaj[f], nuEff));
         }
-        st3(w.f1, f, cvta<F>(dv + vv));
+        st3(w.f1, f, dv + vv);
     };
     // ---- j face (k, fj, i), fj = j + e: ueqn_solvers.c:397-602 with Compute_du_j (inline.h:2809-2869)
     auto jface = [&](int fj, int e) {
@@ -708,7 +705,7 @@ __global__ void __launch_bounds__(FBN, FMINB) k_face_fluxes(Grid g, FaceMet<M> m
             if (AX) vv = base + cvta<double>(visc_flux_ax<M>(m.jcsi.y[f], m.jeta.z[f], m.jzet.x[f], 1, cvta<M>(dc), cvta<M>(de), cvta<M>(dz), m.jaj[f], nuEff));
             else vv = base + cvta<double>(visc_flux<M>(ld3(m.jcsi, f), ld3(m.jeta, f), ld3(m.jzet, f), 1, cvta<M>(dc), cvta<M>(de), cvta<M>(dz), m.jaj[f], nuEff));
         }
-        st3(w.f2, f, cvta<F>(dv + vv));
+        st3(w.f2, f, dv + vv);
     };
     // ---- k face (fk, j, i), fk = k + e: ueqn_solvers.c:604-778 with Compute_du_k (inline.h:2871-2931)
     auto kface = [&](int fk, int e) {
@@ -746,7 +743,7 @@ __global__ void __launch_bounds__(FBN, FMINB) k_face_fluxes(Grid g, FaceMet<M> m
             if (AX) vv = cvta<double>(visc_flux_ax<M>(m.kcsi.y[f], m.keta.z[f], m.kzet.x[f], 2, cvta<M>(dc), cvta<M>(de), cvta<M>(dz), m.kaj[f], nuEff));
             else vv = cvta<double>(visc_flux<M>(ld3(m.kcsi, f), ld3(m.keta, f), ld3(m.kzet, f), 2, cvta<M>(dc), cvta<M>(de), cvta<M>(dz), m.kaj[f], nuEff));
         }
-        st3(w.f3, f, cvta<F>(dv + vv));
+        st3(w.f3, f, dv + vv);
     };
     // one emitted body per direction: the second pass is the face on the -
     // side of a cell next to a non-periodic 0 boundary
@@ -762,22 +759,20 @@ __global__ void __launch_bounds__(FBN, FMINB) k_face_fluxes(Grid g, FaceMet<M> m
 // Pass 2 (ueqn_solvers.c:825-947): divergence of the face fluxes of interior
 // cell (k, j, i). A periodic direction reads its face 0 from face m-2
 // (resetFacePeriodicFluxesVector, inline.h:5357-5451, applied to the fluxes).
-template <class M>
-__device__ __forceinline__ R3<M> cell_fp(const Grid &g, const FluxWork<M> &w, int k, int j, int i)
+__device__ __forceinline__ R3<double> cell_fp(const Grid &g, const FluxWork &w, int k, int j, int i)
 {
     const int c = g.lin(k, j, i), pl = g.mx * g.my;
     const int iw = (i == 1 && g.pi) ? c + g.mx - 3 : c - 1;
     const int js = (j == 1 && g.pj) ? c + (g.my - 3) * g.mx : c - g.mx;
     const int kb = (k == 1 && g.pk) ? c + (g.mz - 3) * pl : c - pl;
-    R3<M> F;
+    R3<double> F;
     F.x = w.f1.x[c] - w.f1.x[iw] + w.f2.x[c] - w.f2.x[js] + w.f3.x[c] - w.f3.x[kb];
     F.y = w.f1.y[c] - w.f1.y[iw] + w.f2.y[c] - w.f2.y[js] + w.f3.y[c] - w.f3.y[kb];
     F.z = w.f1.z[c] - w.f1.z[iw] + w.f2.z[c] - w.f2.z[js] + w.f3.z[c] - w.f3.z[kb];
     return F;
 }
 
-template <class F>
-__global__ void k_cell_fp(Grid g, FluxWork<F> w)
+__global__ void k_cell_fp(Grid g, FluxWork w)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
     if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
@@ -794,12 +789,12 @@ __global__ void k_cell_fp(Grid g, FluxWork<F> w)
 // Rhs = -dP (+ AB2 buoyancy) (ueqn_solvers.c:1305-1338), += turbine body
 // force (ueqn_solvers.c:1340-1344), += FormU, += sourceU (body force), +=
 // meanGradPForcing (ueqn_sources.c:3735-3822). MR:
-// metric storage type; F: face-flux storage type. kind: 0 R += scale FormU;
+// metric storage type; the arithmetic is FP64. kind: 0 R += scale FormU;
 // 1 the ExplicitRhsU value is stored in R; 2 it is not stored but masked at
 // the non-resolved faces and applied at once by the explicit time update
 // (rk_point, one RK4 stage or the FE step).
-template <class MR, class F, int kind>
-__global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State s, FluxWork<F> w, V3f<double> R, double scale, Params p, int ab2, RkArgs rk)
+template <class MR, int kind>
+__global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State s, FluxWork w, V3f<double> R, double scale, Params p, int ab2, RkArgs rk)
 {
     constexpr bool fused = kind >= 1;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -834,26 +829,23 @@ __global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State 
     } else {
         base = ld3(R, c);
     }
-    // arithmetic in FP32 only when both the metrics and the fluxes are FP32
-    using M = typename std::conditional<std::is_same<MR, float>::value && std::is_same<F, float>::value, float, double>::type;
-    auto FP = [&](int kk, int jj, int ii) { return cvta<M>(ld3(w.fp, g.lin(kk, jj, ii))); };
-    auto MT = [&](const V3f<MR> &v, int q) { return cvta<M>(ld3(v, q)); };
-    const M sc = (M)scale, h = M(0.5);
-    M v1, v2;
+    auto FP = [&](int kk, int jj, int ii) { return ld3(w.fp, g.lin(kk, jj, ii)); };
+    auto MT = [&](const V3f<MR> &v, int q) { return cvta<double>(ld3(v, q)); };
+    double v1, v2;
     double ox, oy, oz;
-    const R3<M> fpc = FP(k, j, i);
-    { R3<M> fb = i < g.mx - 2 ? FP(k, j, i + 1) : (g.pi ? FP(k, j, 1) : fpc);
-      R3<M> a = MT(m.csi, c), b = MT(m.csi, c + 1);
+    const R3<double> fpc = FP(k, j, i);
+    { R3<double> fb = i < g.mx - 2 ? FP(k, j, i + 1) : (g.pi ? FP(k, j, 1) : fpc);
+      R3<double> a = MT(m.csi, c), b = MT(m.csi, c + 1);
       v1 = a.x * fpc.x + a.y * fpc.y + a.z * fpc.z; v2 = b.x * fb.x + b.y * fb.y + b.z * fb.z;
-      ox = base.x + (double)(sc * (M)m.iaj[c] * (h * (v1 + v2))); }
-    { R3<M> fb = j < g.my - 2 ? FP(k, j + 1, i) : (g.pj ? FP(k, 1, i) : fpc);
-      int n = c + g.mx; R3<M> a = MT(m.eta, c), b = MT(m.eta, n);
+      ox = base.x + scale * m.iaj[c] * (0.5 * (v1 + v2)); }
+    { R3<double> fb = j < g.my - 2 ? FP(k, j + 1, i) : (g.pj ? FP(k, 1, i) : fpc);
+      int n = c + g.mx; R3<double> a = MT(m.eta, c), b = MT(m.eta, n);
       v1 = a.x * fpc.x + a.y * fpc.y + a.z * fpc.z; v2 = b.x * fb.x + b.y * fb.y + b.z * fb.z;
-      oy = base.y + (double)(sc * (M)m.jaj[c] * (h * (v1 + v2))); }
-    { R3<M> fb = k < g.mz - 2 ? FP(k + 1, j, i) : (g.pk ? FP(1, j, i) : fpc);
-      int n = c + g.mx * g.my; R3<M> a = MT(m.zet, c), b = MT(m.zet, n);
+      oy = base.y + scale * m.jaj[c] * (0.5 * (v1 + v2)); }
+    { R3<double> fb = k < g.mz - 2 ? FP(k + 1, j, i) : (g.pk ? FP(1, j, i) : fpc);
+      int n = c + g.mx * g.my; R3<double> a = MT(m.zet, c), b = MT(m.zet, n);
       v1 = a.x * fpc.x + a.y * fpc.y + a.z * fpc.z; v2 = b.x * fb.x + b.y * fb.y + b.z * fb.z;
-      oz = base.z + (double)(sc * (M)m.kaj[c] * (h * (v1 + v2))); }
+      oz = base.z + scale * m.kaj[c] * (0.5 * (v1 + v2)); }
     if (fused && p.source) {
         // sourceU (ueqn_solvers.c:1369, ueqn_sources.c:2884-2980): central body force . face area, FP64
         const V3f<double> &f = s.source;
@@ -864,11 +856,11 @@ __global__ void __launch_bounds__(256) k_rhs_faces(Grid g, FaceMet<MR> m, State 
         oz += 1.0 * (0.5 * (f.x[c] + f.x[kt]) * d.x + 0.5 * (f.y[c] + f.y[kt]) * d.y + 0.5 * (f.z[c] + f.z[kt]) * d.z);
     }
     if (fused && p.mean_grad_p) {
-        R3<M> a = MT(m.icsi, c), b = MT(m.jeta, c), d = MT(m.kzet, c);
-        const M g0 = (M)p.mgp[0], g1 = (M)p.mgp[1], g2 = (M)p.mgp[2];
-        ox += (double)(g0 * a.x + g1 * a.y + g2 * a.z);
-        oy += (double)(g0 * b.x + g1 * b.y + g2 * b.z);
-        oz += (double)(g0 * d.x + g1 * d.y + g2 * d.z);
+        R3<double> a = MT(m.icsi, c), b = MT(m.jeta, c), d = MT(m.kzet, c);
+        const double g0 = p.mgp[0], g1 = p.mgp[1], g2 = p.mgp[2];
+        ox += g0 * a.x + g1 * a.y + g2 * a.z;
+        oy += g0 * b.x + g1 * b.y + g2 * b.z;
+        oz += g0 * d.x + g1 * d.y + g2 * d.z;
     }
     finish(ox, oy, oz);
 }
@@ -1131,7 +1123,7 @@ inline int nblk(int64_t n) { int64_t b = (n + 255) / 256; return (int)(b < 148 *
 void contra_to_cart(tg_ctx *C)
 {
     if (C->axis_aligned) { contra_to_cart_tensor(C, "contra_to_cart_final"); return; }
-    TG_PROF(C, "contra_to_cart_final", k_contra_to_cart<double, double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
+    TG_PROF(C, "contra_to_cart_final", k_contra_to_cart<double><<<gi(C->g), block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
 }
 
 // contravariantToCartesian inside the momentum stages, at the precision the
@@ -1140,32 +1132,8 @@ void contra_to_cart_stage(tg_ctx *C)
 {
     if (C->axis_aligned) { contra_to_cart_tensor(C, "contra_to_cart"); return; }
     const dim3 gr = gi(C->g);
-    if (C->pol.contra_a32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<float, float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
-    else if (C->pol.contra_m32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<double, float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
-    else TG_PROF(C, "contra_to_cart", k_contra_to_cart<double, double><<<gr, block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
-}
-
-// Precision of each momentum stage in the mixed mode. Every momentum stencil
-// reads the FP32 metric copies (half the metric bytes, which dominate the
-// stencils' traffic). Two things stay FP64 because the pressure field is set by
-// the divergence of the momentum right-hand side, in which the convective
-// fluxes nearly cancel: the arithmetic of contravariantToCartesian, FormU's
-// convective fluxes and the face assembly, and the storage of the face-flux
-// planes. The projection keeps FP64 metrics too: with FP32 metric copies its
-// correction is no longer the exact gradient whose divergence the FP64 Poisson
-// operator balanced, and the left-over divergence raised the relative L2 error
-// of p to 3.3e-6 in 5 steps (ABL 16x16x12). Measured against the FP64 oracle
-// (ABL 48x48x32, 20 steps) FP32
-// storage of the face fluxes alone raised the relative L2 error of p from
-// 1.3e-7 to 4.9e-6; FP32 Cramer arithmetic raised it to 6e-7 in 5 steps.
-static void set_policy(tg_ctx *C)
-{
-    C->pol.contra_m32 = C->mixed;
-    C->pol.contra_a32 = false;
-    C->pol.visc32 = C->mixed;
-    C->pol.flux32 = false;
-    C->pol.rhs32 = C->mixed;
-    C->pol.smag32 = C->mixed;
+    if (C->met32) TG_PROF(C, "contra_to_cart", k_contra_to_cart<float><<<gr, block3(), 0, C->stream>>>(C->g, C->fm32, C->s));
+    else TG_PROF(C, "contra_to_cart", k_contra_to_cart<double><<<gr, block3(), 0, C->stream>>>(C->g, C->fm64, C->s));
 }
 
 // Smagorinsky filter width squared of every cell from its Jacobian, in the
@@ -1185,14 +1153,27 @@ void refresh_filter(tg_ctx *C)
     k_filter2<double><<<nblk(G), 256, 0, C->stream>>>(G, C->fm64.aj, C->fm64.flt2);
 }
 
+// Precision of each momentum stage in the mixed mode. On a curvilinear mesh, and in
+// QUICK's face fluxes on any, the momentum stencils read the FP32 metric copies
+// (half the metric bytes, which dominate the stencils' traffic) but for GradP and the
+// projection, which read SetCoeffMatrix's products; the kernels for meshes of planes
+// read no metric, so both modes run the same FP64 kernels there. Viscous fluxes and
+// the eddy viscosity are FP32 arithmetic as well. Elsewhere the arithmetic and the
+// face-flux planes stay FP64, because the pressure field is set by the divergence
+// of the momentum right-hand side, in which the convective fluxes nearly cancel:
+// measured against the FP64 oracle (ABL 48x48x32, 20 steps, on the general kernels)
+// FP32 storage of the face fluxes alone raised the relative L2 error of p from
+// 1.3e-7 to 4.9e-6, FP32 Cramer arithmetic raised it to 6e-7 in 5 steps, and a
+// projection on FP32 metrics, no longer the exact gradient whose divergence the
+// Poisson operator balanced, to 3.3e-6 in 5 steps (ABL 16x16x12).
 void alloc_precision_work(tg_ctx *C)
 {
     const size_t G = (size_t)C->g.size();
     const Metrics &m = C->m;
     C->fm64 = FaceMet<double>{m.csi, m.eta, m.zet, m.icsi, m.ieta, m.izet, m.jcsi, m.jeta, m.jzet,
                               m.kcsi, m.keta, m.kzet, m.aj, m.iaj, m.jaj, m.kaj, dallocd(C, G)};
-    set_policy(C);
-    if (!C->pol.flux32) C->fw64 = FluxWork<double>{dalloc3(C, G), dalloc3(C, G), dalloc3(C, G), dalloc3(C, G)};
+    C->fw = FluxWork{dalloc3(C, G), dalloc3(C, G), dalloc3(C, G), dalloc3(C, G)};
+    C->met32 = C->mixed;
     if (!C->mixed) return;
     auto f3 = [&]() {
         float *a = (float *)dalloc(C, 3 * G * sizeof(float));
@@ -1203,7 +1184,6 @@ void alloc_precision_work(tg_ctx *C)
     for (auto *v : vv) *v = f3();
     float **ss[] = {&f.aj, &f.iaj, &f.jaj, &f.kaj, &f.flt2};
     for (auto **v : ss) *v = (float *)dalloc(C, G * sizeof(float));
-    if (C->pol.flux32) C->fw32 = FluxWork<float>{f3(), f3(), f3(), f3()};
     C->met32_stale = true;
 }
 
@@ -1283,7 +1263,7 @@ void update_nut(tg_ctx *C)
     TG_CUDA(cudaMemsetAsync(C->s.nut, 0, sizeof(double) * g.size(), C->stream));
     refresh_met32(C);
     if (C->axis_aligned) smagorinsky_tensor(C);
-    else if (C->pol.smag32) TG_PROF(C, "smagorinsky", k_smagorinsky<float><<<gi(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm));
+    else if (C->met32) TG_PROF(C, "smagorinsky", k_smagorinsky<float><<<gi(g), block3(), 0, C->stream>>>(g, C->fm32, C->s, C->prm));
     else TG_PROF(C, "smagorinsky", k_smagorinsky<double><<<gi(g), block3(), 0, C->stream>>>(g, C->fm64, C->s, C->prm));
     int na = std::max(g.mx, g.my) - 2, nb = std::max(g.my, g.mz) - 2;
     dim3 grid((na + 31) / 32, (nb + 7) / 8, 6);
@@ -1325,18 +1305,15 @@ void buoyancy(tg_ctx *C)
         k_buoyancy<<<ga(C->g), block3(), 0, C->stream>>>(C->g, C->m, C->s, C->prm);
 }
 
-// FormU pass 1 (face fluxes) at the precision of the context's policy.
-// Pass 2 (k_cell_fp) follows; the flux planes are only read at the points
-// pass 1 writes, fp only at interior cells.
+// FormU pass 1 (face fluxes) at the context's precision. Pass 2 (k_cell_fp) follows;
+// the flux planes are only read at the points pass 1 writes, fp only at interior cells.
 template <int mode, bool AX>
 static void face_fluxes(tg_ctx *C, dim3 gr)
 {
     const Grid g = C->g;
-    const auto &P = C->pol;
-    if (P.visc32 && P.flux32) TG_PROF(C, "formu_face_fluxes", (k_face_fluxes<float, float, mode, AX><<<gr, dim3(FBX, FBY, FBZ), 0, C->stream>>>(g, C->fm32, C->s, C->fw32, C->prm)));
-    else if (P.visc32) TG_PROF(C, "formu_face_fluxes", (k_face_fluxes<float, double, mode, AX><<<gr, dim3(FBX, FBY, FBZ), 0, C->stream>>>(g, C->fm32, C->s, C->fw64, C->prm)));
-    else if (P.flux32) TG_PROF(C, "formu_face_fluxes", (k_face_fluxes<double, float, mode, AX><<<gr, dim3(FBX, FBY, FBZ), 0, C->stream>>>(g, C->fm64, C->s, C->fw32, C->prm)));
-    else TG_PROF(C, "formu_face_fluxes", (k_face_fluxes<double, double, mode, AX><<<gr, dim3(FBX, FBY, FBZ), 0, C->stream>>>(g, C->fm64, C->s, C->fw64, C->prm)));
+    const dim3 bl(FBX, FBY, FBZ);
+    if (C->met32) TG_PROF(C, "formu_face_fluxes", (k_face_fluxes<float, mode, AX><<<gr, bl, 0, C->stream>>>(g, C->fm32, C->s, C->fw, C->prm)));
+    else TG_PROF(C, "formu_face_fluxes", (k_face_fluxes<double, mode, AX><<<gr, bl, 0, C->stream>>>(g, C->fm64, C->s, C->fw, C->prm)));
 }
 
 static void form_u_faces(tg_ctx *C, int mode)
@@ -1346,13 +1323,11 @@ static void form_u_faces(tg_ctx *C, int mode)
     refresh_met32(C);
     // one thread per interior cell (k_face_fluxes)
     const dim3 gr((g.mx - 2 + FBX - 1) / FBX, (g.my - 2 + FBY - 1) / FBY, (g.mz - 2 + FBZ - 1) / FBZ);
-    const auto &P = C->pol;
     const bool ax = C->axis_aligned;
     if (mode == 1) { if (ax) face_fluxes<1, true>(C, gr); else face_fluxes<1, false>(C, gr); }
     else if (mode == 2) { if (ax) face_fluxes<2, true>(C, gr); else face_fluxes<2, false>(C, gr); }
     else { if (ax) face_fluxes<0, true>(C, gr); else face_fluxes<0, false>(C, gr); }
-    if (P.flux32) TG_PROF(C, "formu_cell_fp", k_cell_fp<float><<<gi(g), block3(), 0, C->stream>>>(g, C->fw32));
-    else TG_PROF(C, "formu_cell_fp", k_cell_fp<double><<<gi(g), block3(), 0, C->stream>>>(g, C->fw64));
+    TG_PROF(C, "formu_cell_fp", k_cell_fp<<<gi(g), block3(), 0, C->stream>>>(g, C->fw));
 }
 
 template <int fused>
@@ -1361,11 +1336,8 @@ static void rhs_faces(tg_ctx *C, V3f<double> rhs, double scale, int ab2, RkArgs 
     if (C->axis_aligned) { rhs_faces_tensor(C, fused, rhs, scale, ab2, rk); return; }
     const Grid g = C->g;
     const dim3 gr = gi(g);
-    const auto &P = C->pol;
-    if (P.rhs32 && P.flux32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<float, float, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw32, rhs, scale, C->prm, ab2, rk));
-    else if (P.rhs32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<float, double, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw64, rhs, scale, C->prm, ab2, rk));
-    else if (P.flux32) TG_PROF(C, "formu_rhs_faces", k_rhs_faces<double, float, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw32, rhs, scale, C->prm, ab2, rk));
-    else TG_PROF(C, "formu_rhs_faces", k_rhs_faces<double, double, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw64, rhs, scale, C->prm, ab2, rk));
+    if (C->met32) TG_PROF(C, "formu_rhs_faces", (k_rhs_faces<float, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm32, C->s, C->fw, rhs, scale, C->prm, ab2, rk)));
+    else TG_PROF(C, "formu_rhs_faces", (k_rhs_faces<double, fused><<<gr, block3(), 0, C->stream>>>(g, C->fm64, C->s, C->fw, rhs, scale, C->prm, ab2, rk)));
 }
 
 void form_u(tg_ctx *C, V3f<double> rhs, double scale, int mode)
@@ -1404,7 +1376,6 @@ static void explicit_rhs_head(tg_ctx *C, int mode)
 
 void explicit_rhs(tg_ctx *C, int mode)
 {
-    const Grid g = C->g;
     explicit_rhs_head(C, mode);
     rhs_faces<1>(C, C->s.rhs, 1.0, C->it > C->cfg.it_start ? 1 : 0);
     mask_non_resolved(C, C->s.rhs);

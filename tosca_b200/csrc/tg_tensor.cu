@@ -867,9 +867,9 @@ template <int mode, bool LES, int KZ>
 void launch_fp(tg_ctx *C, const Box &b)
 {
     constexpr int bytes = PTX * PTY * (KZ + 2) * 8 * (LES && mode != 1 ? 4 : 3);
-    static_assert(bytes <= 75 * 1024, "three blocks per SM");
+    static_assert(bytes <= 110 * 1024, "two blocks per SM, as the registers allow");
     const int nbi = (b.i1 - b.i0 + PX) / PX, nbj = (b.j1 - b.j0 + PY) / PY, nbk = (b.k1 - b.k0 + KZ) / KZ, nbnd = boundary_blocks(C->g);
-    TG_PROF(C, "formu_cell_fp", (k_fp_tensor<mode, LES, KZ><<<nbnd + nbi * nbj * nbk, dim3(PX, PY), bytes, C->stream>>>(C->g, C->ts, C->s, C->fw64.fp, C->prm, b, nbnd, nbi, nbj)));
+    TG_PROF(C, "formu_cell_fp", (k_fp_tensor<mode, LES, KZ><<<nbnd + nbi * nbj * nbk, dim3(PX, PY), bytes, C->stream>>>(C->g, C->ts, C->s, C->fw.fp, C->prm, b, nbnd, nbi, nbj)));
 }
 
 template <int mode>
@@ -900,7 +900,7 @@ void launch_stage_fp(tg_ctx *C)
         if (cost < best) { best = cost; kc = c; }
     }
     const int nedge = (edge_threads(g) + PX * PY - 1) / (PX * PY), nb = nedge + nbi * nbj * ((nk + kc - 1) / kc);
-    TG_PROF(C, "formu_stage_fp", (k_stage_fp<LES><<<nb, dim3(PX, PY), STAGE_SMEM, C->stream>>>(g, C->ts, C->s, C->fw64.fp, C->prm, nedge, nbi, nbj, kc)));
+    TG_PROF(C, "formu_stage_fp", (k_stage_fp<LES><<<nb, dim3(PX, PY), STAGE_SMEM, C->stream>>>(g, C->ts, C->s, C->fw.fp, C->prm, nedge, nbi, nbj, kc)));
 }
 
 template <int mode, bool LES, int KZ>
@@ -1057,7 +1057,7 @@ void stage_tail_tensor(tg_ctx *C)
 void rhs_faces_tensor(tg_ctx *C, int kind, V3f<double> rhs, double scale, int ab2, const RkArgs &rk, bool from_p)
 {
     const Grid g = C->g;
-    const V3f<double> fp = C->fw64.fp;
+    const V3f<double> fp = C->fw.fp;
     auto go = [&](auto kernel) {
         TG_PROF(C, "formu_rhs_faces", kernel<<<gi(g), block3(), 0, C->stream>>>(g, C->ts, C->s, fp, rhs, scale, C->prm, ab2, rk));
     };
