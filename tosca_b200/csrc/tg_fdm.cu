@@ -22,8 +22,8 @@
 // n a multiple of 4 folds twice. Work per cell and pass is 2 n / G operations
 // for G groups. At 256 x 256 x 128 a pass takes 72 to 99 us against 21 us for its
 // bytes and 29 us for its products at the 37 TFLOP/s that register-only
-// m8n8k4 reaches (load, product and store phases of a block alternate; three
-// blocks per SM overlap them), the j lines 58 us against 31 us for their bytes:
+// m8n8k4 reaches (load, product and store phases of a block alternate; two or
+// three blocks per SM overlap them in part), the j lines 58 us against 31 us for their bytes:
 // 0.39 ms for the solve, against 1.06 ms for one multigrid V-cycle. Operands in
 // fragment order (one 512-byte load per step) took a pass from 110 to 77 us.
 #include <algorithm>
@@ -433,9 +433,13 @@ bool is_uniform(const std::vector<double> &v, int cnt)
 // work per cell grows with it, that of a multigrid cycle does not. Measured,
 // ms per step (mixed) of the direct solve against the multigrid: 1024 x 512 x 32
 // (384 rows) 12.2 against 16.4, 75 x 75 x 25 (76) 0.36 against 1.38; 2048 x 32 x 32
-// (520) 2.84 against 2.71, 2047 x 32 x 32 open in x (1032) 3.64 against 3.29. The
-// bound also keeps the panels in shared memory and the set-up of an unfolded
-// direction (n^3) below half a second.
+// (520) 2.84 against 2.71, 2047 x 32 x 32 open in x (1032) 3.64 against 3.29. A
+// periodic j has the bound for itself: its rows are not added to the two, because
+// the multigrid is slower there as well (point instead of line sweeps): 1.90 direct
+// and 2.42 multigrid at 32 x 32 x 2048 (16 + 512 rows), 5.16 and 8.52 at 64 x 64 x 2048
+// (32 + 512), 6.23 and 15.6 at 128 x 128 x 1024 (64 + 256). The bound also keeps the
+// panels in shared memory and the set-up of an unfolded direction (n^3) at a tenth
+// of a second.
 constexpr int FDM_MAX_ROWS = 512;
 
 template <class T>
@@ -537,8 +541,13 @@ void upload_dir(tg_ctx *C, FdmDir &D, const FdmVectors &E)
     D.lam = to_device(C, E.lam);
 }
 
-// columns per panel: the widest whose panel takes at most a third of the shared
-// memory, so that three blocks share an SM; the narrowest in any case
+// Columns per panel: the widest whose panel of the contiguous direction takes at
+// most a third of the shared memory, so that three blocks share an SM there; the
+// narrowest in any case. The strided directions take the same width: their panels
+// pad each row instead of each column and can be a little larger (82 KB at 288 and
+// at 512 rows, two blocks), but narrower ones gain 6 % at 512 and lose 25 % at 288.
+// Forward / inverse at 128 x 64 columns, us, width in brackets: 256 cells 26.5 / 29.0 (32), 24.9 / 35.1 (16);
+// 288 31.5 / 36.4 (32), 30.0 / 53.6 (16), 36.1 / 45.4 (8); 512 80.4 / 86.4 (16), 72.2 / 84.8 (8).
 int panel_cols(const FdmDir &D)
 {
     for (int nc : {32, 16}) if ((size_t)nc * x_stride(D.G * D.gp) * 8 <= 75 * 1024) return nc;

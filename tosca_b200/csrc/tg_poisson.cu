@@ -159,8 +159,7 @@ __device__ __forceinline__ void row19(const PoissonCtx &P, const Cg &q, int ic, 
 // at peqn.c:1410-1418), y = x on the pinned row
 // Bound by the latency of its 55 loads: those of x do not wait for the coefficient's
 // threshold, and 80 registers hold them at three blocks per SM. A step of
-// 192 x 96 x 96 takes 3.47 ms with loads under the threshold, 3.39 ms this way,
-// 3.44 ms at four blocks (64 registers), 3.51 ms at two (106).
+// 192 x 96 x 96 took 3.47 ms with loads under the threshold, 3.39 ms this way.
 __global__ void __launch_bounds__(256, 3) k_apply19(PoissonCtx P, const double *__restrict__ x, double *__restrict__ y)
 {
     int ic = blockIdx.x * blockDim.x + threadIdx.x, jc = blockIdx.y * blockDim.y + threadIdx.y, kc = blockIdx.z * blockDim.z + threadIdx.z;

@@ -75,13 +75,10 @@ __device__ __forceinline__ void stencil4(int i, int m, int per, int &L, int &R)
 // the budget and is not formed). T and nut are read from a ring of six planes in
 // shared memory with one cell below and two above in i and j; plane k + 4 is
 // copied while plane k is worked on, one barrier per plane. Bound by instruction
-// issue (525 of 725 per cell were integer and select work) and by the
-// latency of the divisions: blocks of 32 x 4 x 2 cells that staged 35 x 7 x 5 points
-// each took 3.52 ms of a step at 192 x 96 x 96 (curvilinear) and 0.890 ms at
-// 128 x 128 x 64, this one 3.43 and 0.875 (3.44 and 0.884 with the ends of each
-// direction tested per derivative instead of once per face; 3.47 and 0.900 with
-// 80 registers and three blocks per SM). The floor, at 64 to 160 bytes per cell, is
-// a fifth to a third of its time.
+// issue and by the latency of the divisions: a launch takes three to five times what
+// its 64 (planes) to 160 (curvilinear) bytes per cell do. A step of 192 x 96 x 96
+// (curvilinear) takes 3.43 ms and one of 128 x 128 x 64 0.875; with blocks of
+// 32 x 4 x 2 cells that stage 35 x 7 x 5 points each, 3.52 and 0.890.
 // The WENO points of the boundary faces, which may lie outside the tile (periodic
 // i = mx + 2 and i = -3), are read from global memory.
 //
